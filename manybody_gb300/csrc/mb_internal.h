@@ -284,7 +284,7 @@ __device__ __forceinline__ void prefetch_up_group(const void* x, const uint32_t*
   if (lo >= row_bytes) return;
   const char* xg = static_cast<const char*>(x) + lo;
   for (int k = lane / kLines; k < nu; k += kPer)
-    asm volatile("prefetch.global.L2 [%0];" ::"l"(xg + (uint64_t)s_up[k] * row_bytes));
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(xg + (uint64_t)(s_up[k] & 0x7FFFFFFFu) * row_bytes));
 }
 #endif
 struct SlicedTable {
@@ -293,6 +293,13 @@ struct SlicedTable {
   std::vector<uint8_t> nneg;  // [D] negative entries per state
 };
 SlicedTable sliced_table(const HopTable& t, int64_t D);
+// 1 + ceil(log2(terms)), at least 6: the bits an integer sum (mb_isum.h) of that
+// many terms keeps free above its largest term, sign included.
+inline int isum_base(int64_t terms) {
+  int b = 6;
+  while ((int64_t(1) << (b - 1)) < terms) ++b;
+  return b;
+}
 // The same table with 16-bit entries (index | negative << 15; D + kSlicedPads
 // must stay below 2^15), a lane's slots 8i..8i+7 in one 16-byte word.
 struct SlicedTable16 {
@@ -361,6 +368,9 @@ struct OpView {
   int table_stage;
   int dn_max_words;
   int max_up_list;
+  // headroom bits of the complex128 applies' integer hop sums (isum_base of the
+  // most hops one state can have)
+  int isum_base;
   // Operators made from a sparse matrix instead of a lattice (mb_op_create_csr):
   // CSR on the device, values complex128 (and complex64 copies for MB_PREC_F32).
   const int64_t* csr_row;

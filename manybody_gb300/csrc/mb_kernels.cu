@@ -7,7 +7,10 @@
 // mb_internal.h) and diag = U * popcount(up & down) (+ self-bond energies).
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 #include "mb_internal.h"
+#include "mb_isum.h"
 
 namespace mb {
 
@@ -125,16 +128,24 @@ static int max_smem_optin() {
 // ---------------------------------------------------------------------------
 // The matrix-free apply:  y = scale * (H - shift) x + beta * z
 // with optional fused dot products (dot_mode bit0: Re<x,y>, bit1: <y,y>,
-// bit2: <x,x>).  One CTA per SM (two for complex64) walks the rows r_up in
-// the row schedule's order; it stages the row X[r_up, :] (and eight zero elements) in shared
-// memory when it fits, so the down hops, which stay inside the row, gather
-// from shared memory through the sliced table (one coalesced 16-byte load
-// per lane for four slots: neighbour index | sign << 31, padding = one of the
-// zero elements past the row), while the up hops read the neighbour rows X[r_up', c] from
-// L2/HBM with coalesced 8/16-byte loads, the row's sign-sorted target list
-// in shared memory (added, then subtracted).  Warp w takes the 32-column
-// groups w, w + 32, ... (with up_prefetch set it asks L2 for the group's
-// up-hop lines before its down hops).
+// bit2: <x,x>).  The CTAs walk the rows r_up in the row schedule's order; one
+// stages the row X[r_up, :] (and eight zero elements) in shared memory when it
+// fits, so the down hops, which stay inside the row, gather from shared memory
+// through the sliced table (one coalesced 16-byte load per lane for four
+// slots: neighbour index | sign << 31, padding = one of the zero elements past
+// the row), while the up hops read the neighbour rows X[r_up', c] from L2/HBM
+// with coalesced 8/16-byte loads, the row's sign-sorted target list in shared
+// memory.  Warp w takes the 32-column groups w, w + nwarps, ... (with
+// up_prefetch set it asks L2 for the group's up-hop lines before its down hops).
+//
+// complex128: the hop sums run on the integer pipes (mb_isum.h), the FP64 pipe
+// converts them and does the diagonal, the affine part and the dots.  A staged
+// row is decoded once (each element is a down neighbour about 16 times), up
+// neighbours as they arrive; a row or a sum outside the integer sums' range
+// takes the FP64 adds.  4x4 6+6 (64.1M states) 10.08 -> 4.06 ms, 5+5 2.81 ->
+// 1.23, 1D L=16 8+8 15.98 -> 7.41, 3x4 6+6 137 -> 68 us.  By the counters (4x4
+// 5+5) the ALU pipe is now 65 % busy, the FP64 pipe 38 %, issue 64 %, and the
+// largest stall is waiting for L2 (3.8 of 10.7 warps a scheduler).
 // ---------------------------------------------------------------------------
 constexpr int kApplyThreads = 1024;
 // CTAs per SM: complex64 rows are half the size, and two CTAs per SM (32
@@ -158,11 +169,16 @@ __device__ __forceinline__ void apply_rows(
     double* __restrict__ partials) {
   using V2 = typename C2<T>::type;
   constexpr int kShift = sizeof(V2) == 16 ? 4 : 3;
+  constexpr bool kInt = sizeof(T) == 8;  // hop sums on the integer pipes (mb_isum.h)
   extern __shared__ __align__(16) unsigned char smem[];
   const int64_t Dd = v.Dd;
   const uint32_t row_bytes = (uint32_t)(sizeof(V2) * Dd);
   uint32_t* s_up =
       reinterpret_cast<uint32_t*>(smem + (STAGED ? row_bytes + sizeof(V2) * kSlicedPads : 0));
+  // a staged complex128 row is kept decoded; s_wide[row parity]: it holds a
+  // value that does not fit there
+  __shared__ int s_wide[2];
+  if (threadIdx.x < 2) s_wide[threadIdx.x] = 0;
   if (STAGED && threadIdx.x < kSlicedPads) {
     V2 zero;
     zero.x = T(0);
@@ -172,20 +188,37 @@ __device__ __forceinline__ void apply_rows(
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   const int64_t ngroups = (Dd + 31) >> 5;
   DotAcc<T> a_xy, a_yy, a_xx;
+  const ISumForm form(v.isum_base);
+  int parity = 0;
 
-  for (int64_t ri = blockIdx.x; ri < v.Du; ri += gridDim.x) {
+  for (int64_t ri = blockIdx.x; ri < v.Du; ri += gridDim.x, parity ^= 1) {
     const int64_t r = v.row_sched ? (int64_t)v.row_sched[ri] : ri;
     const V2* xrow = x + r * Dd;
     __syncthreads();
     const int u0 = __ldg(&v.up_loff[r]), nu = __ldg(&v.up_loff[r + 1]) - u0;
     const int npos = __ldg(&v.up_lpos[r]);
-    for (int j = threadIdx.x; j < nu; j += blockDim.x) s_up[j] = __ldg(&v.up_list[u0 + j]);
-    if (STAGED)
-      for (int64_t c = threadIdx.x; c < Dd; c += blockDim.x)
-        reinterpret_cast<V2*>(smem)[c] = xrow[c];
+    // complex128: the sign in bit 31
+    for (int j = threadIdx.x; j < nu; j += blockDim.x)
+      s_up[j] = __ldg(&v.up_list[u0 + j]) | (kInt && j >= npos ? 0x80000000u : 0u);
+    if (STAGED) {
+      if constexpr (kInt) {
+        bool wide = false;
+        for (int64_t c = threadIdx.x; c < Dd; c += blockDim.x) {
+          const V2 val = xrow[c];
+          reinterpret_cast<longlong2*>(smem)[c] =
+              make_longlong2(isum_pack(val.x, &wide), isum_pack(val.y, &wide));
+        }
+        if (wide) s_wide[parity] = 1;
+        if (threadIdx.x == 0) s_wide[parity ^ 1] = 0;  // read before the last barrier
+      } else {
+        for (int64_t c = threadIdx.x; c < Dd; c += blockDim.x)
+          reinterpret_cast<V2*>(smem)[c] = xrow[c];
+      }
+    }
     __syncthreads();
     const uint32_t um = v.up_mask[r];
     const T su = self_up ? self_up[r] : T(0);
+    const bool wide = kInt && STAGED && s_wide[parity];
     for (int64_t g = warp; g < ngroups; g += nwarps) {
       const int64_t c = (g << 5) + lane;
       const bool live = c < Dd;
@@ -193,45 +226,122 @@ __device__ __forceinline__ void apply_rows(
       if (v.up_prefetch) prefetch_up_group<(int)sizeof(V2)>(x, s_up, nu, g, lane, row_bytes);
       T ar = T(0), ai = T(0);
       const int2 gi = __ldg(reinterpret_cast<const int2*>(v.dn_sgrp) + g);
-      auto hop = [&](uint32_t e) {
-        const uint32_t off = e << kShift;  // the sign bit shifts out
-        V2 val;
-        if (STAGED) {
-          val = *reinterpret_cast<const V2*>(smem + off);
-        } else if (off < row_bytes) {
-          val = __ldg(reinterpret_cast<const V2*>(reinterpret_cast<const char*>(xrow) + off));
-        } else {
-          val.x = T(0);
-          val.y = T(0);
-        }
+      // four slots per 16-byte load; the last word's unused slots are padding
+      const uint4* ep = reinterpret_cast<const uint4*>(v.dn_sell + gi.x) + lane;
+      const char* xc = reinterpret_cast<const char*>(x + cl);
+      // an up neighbour by its list entry
+      auto up = [&](uint32_t e) -> V2 {
+        const uint64_t r2 = kInt ? e & 0x7FFFFFFFu : e;
+        return __ldg(reinterpret_cast<const V2*>(xc + r2 * row_bytes));
+      };
+      // a down neighbour by table entry, in place or from global memory (the
+      // sign bit shifts out)
+      auto dn_far = [&](uint32_t e) -> V2 {
+        const uint32_t off = e << kShift;
+        if (off < row_bytes)
+          return __ldg(reinterpret_cast<const V2*>(reinterpret_cast<const char*>(xrow) + off));
+        V2 zero;
+        zero.x = T(0);
+        zero.y = T(0);
+        return zero;
+      };
+      auto dn = [&](uint32_t e) -> V2 {
+        if (STAGED && !kInt) return *reinterpret_cast<const V2*>(smem + (uint32_t)(e << kShift));
+        return dn_far(e);
+      };
+      auto hop = [&](uint32_t e, const V2& val) {
         const T w = unit_sign(e, T(0));
         ar = fma(w, val.x, ar);
         ai = fma(w, val.y, ai);
       };
-      // four slots per 16-byte load; the last word's unused slots are padding
-      const uint4* ep = reinterpret_cast<const uint4*>(v.dn_sell + gi.x) + lane;
-      for (int j = 0; j < gi.y; j += 4) {
-        const uint4 e = __ldg(ep + 8 * j);
-        hop(e.x);
-        hop(e.y);
-        hop(e.z);
-        hop(e.w);
-      }
-      const char* xc = reinterpret_cast<const char*>(x + cl);
+      auto fp_hops = [&] {
+        for (int j = 0; j < gi.y; j += 4) {
+          const uint4 e = __ldg(ep + 8 * j);
+          hop(e.x, dn(e.x));
+          hop(e.y, dn(e.y));
+          hop(e.z, dn(e.z));
+          hop(e.w, dn(e.w));
+        }
 #pragma unroll 4
-      for (int j = 0; j < npos; ++j) {
-        const V2 val = __ldg(reinterpret_cast<const V2*>(xc + (uint64_t)s_up[j] * row_bytes));
-        ar += val.x;
-        ai += val.y;
-      }
+        for (int j = 0; j < npos; ++j) {
+          const V2 val = up(s_up[j]);
+          ar += val.x;
+          ai += val.y;
+        }
 #pragma unroll 4
-      for (int j = npos; j < nu; ++j) {
-        const V2 val = __ldg(reinterpret_cast<const V2*>(xc + (uint64_t)s_up[j] * row_bytes));
-        ar -= val.x;
-        ai -= val.y;
+        for (int j = npos; j < nu; ++j) {
+          const V2 val = up(s_up[j]);
+          ar -= val.x;
+          ai -= val.y;
+        }
+      };
+      if constexpr (kInt) {
+        ISum2 sum;
+        auto dn_add = [&](auto n, const uint4& e) {
+          constexpr int N = decltype(n)::value;
+          const uint32_t all[4] = {e.x, e.y, e.z, e.w};
+          uint32_t neg[N];
+          if constexpr (STAGED) {
+            longlong2 val[N];
+#pragma unroll
+            for (int k = 0; k < N; ++k) {
+              neg[k] = all[k];
+              val[k] = *reinterpret_cast<const longlong2*>(smem + (uint32_t)(all[k] << kShift));
+            }
+            sum.add_packed<N>(form, val, neg);
+          } else {
+            V2 val[N];
+#pragma unroll
+            for (int k = 0; k < N; ++k) {
+              neg[k] = all[k];
+              val[k] = dn_far(all[k]);
+            }
+            sum.add<N>(form, val, neg);
+          }
+        };
+        auto up_add = [&](auto n, const uint4& e) {
+          constexpr int N = decltype(n)::value;
+          const uint32_t all[4] = {e.x, e.y, e.z, e.w};
+          uint32_t neg[N];
+          V2 val[N];
+#pragma unroll
+          for (int k = 0; k < N; ++k) {
+            neg[k] = all[k];
+            val[k] = up(all[k]);
+          }
+          sum.add<N>(form, val, neg);
+        };
+        using std::integral_constant;
+        if (!wide) {
+          int j = 0;
+          for (; j + 4 <= gi.y; j += 4) dn_add(integral_constant<int, 4>{}, __ldg(ep + 8 * j));
+          if (j < gi.y) {
+            const uint4 e = __ldg(ep + 8 * j);
+            if (j + 1 == gi.y) dn_add(integral_constant<int, 1>{}, e);
+            else if (j + 2 == gi.y) dn_add(integral_constant<int, 2>{}, e);
+            else dn_add(integral_constant<int, 3>{}, e);
+          }
+          const uint4* up4 = reinterpret_cast<const uint4*>(s_up);
+          for (j = 0; j + 4 <= nu; j += 4) up_add(integral_constant<int, 4>{}, up4[j >> 2]);
+          if (j < nu) {
+            const uint4 e = up4[j >> 2];
+            if (j + 1 == nu) up_add(integral_constant<int, 1>{}, e);
+            else if (j + 2 == nu) up_add(integral_constant<int, 2>{}, e);
+            else up_add(integral_constant<int, 3>{}, e);
+          }
+          const double2 hops = sum.value(form);
+          ar = hops.x;
+          ai = hops.y;
+        }
+        if (wide || sum.odd()) {
+          ar = ai = T(0);
+          fp_hops();
+        }
+      } else {
+        fp_hops();
       }
       if (!live) continue;
-      const V2 xv = STAGED ? reinterpret_cast<const V2*>(smem)[c] : xrow[c];
+      const V2 xv = STAGED && !kInt ? reinterpret_cast<const V2*>(smem)[c] : xrow[c];
       T dv = ufold[__popc(um & v.dn_mask[c])] + su;
       if (self_dn) dv += self_dn[c];
       const T ds = dscale * (dv - shift);
@@ -339,8 +449,8 @@ static void apply_t(const OpView& v, const void* x, void* y, double scale, doubl
   const T* uf = sizeof(T) == 8 ? (const T*)v.u_fold : (const T*)v.u_fold_f;
   const T* su = sizeof(T) == 8 ? (const T*)v.self_up : (const T*)v.self_up_f;
   const T* sd = sizeof(T) == 8 ? (const T*)v.self_dn : (const T*)v.self_dn_f;
-  const int grid = apply_grid(v, sizeof(T) == 4 ? MB_PREC_F32 : MB_PREC_F64);
-  kern<<<grid, kApplyThreads, smem, st>>>(v, (const V2*)x, (V2*)y, (T)(-v.t * scale), (T)scale,
+  const int precision = sizeof(T) == 4 ? MB_PREC_F32 : MB_PREC_F64;
+  kern<<<apply_grid(v, precision), kApplyThreads, smem, st>>>(v, (const V2*)x, (V2*)y, (T)(-v.t * scale), (T)scale,
                                           (T)shift, (T)beta, (const V2*)z, uf, su, sd, partials);
   MB_CUDA(cudaGetLastError());
 }
