@@ -143,7 +143,7 @@ static int max_smem_optin() {
 // row is decoded once (each element is a down neighbour about 16 times), up
 // neighbours as they arrive; a row or a sum outside the integer sums' range
 // takes the FP64 adds.  4x4 6+6 (64.1M states) 10.08 -> 4.06 ms, 5+5 2.81 ->
-// 1.23, 1D L=16 8+8 15.98 -> 7.41, 3x4 6+6 137 -> 68 us.  By the counters (4x4
+// 1.15, 1D L=16 8+8 15.98 -> 7.41, 3x4 6+6 137 -> 58 us.  By the counters (4x4
 // 5+5) the ALU pipe is now 65 % busy, the FP64 pipe 38 %, issue 64 %, and the
 // largest stall is waiting for L2 (3.8 of 10.7 warps a scheduler).
 // ---------------------------------------------------------------------------
@@ -425,6 +425,27 @@ static bool apply_staged(const OpView& v, int precision) {
   return apply_smem(v, precision, true) + 1024 <= (size_t)max_smem_optin();
 }
 
+// Threads of an apply's CTAs and how many of them an SM holds: together
+// kApplyThreads (twice that for complex64, see kApplyCtasPerSm).  Several small
+// CTAs, where their rows fit in shared memory side by side, hide each other's
+// staging and barriers, and leave fewer warps without a column group in a row's
+// last round: complex128 4x4 4+4 (1,820 columns) 219 -> 197 us, 3x4 5+4 (495)
+// 41 -> 29 us with 256 threads against 1024; complex64 4x4 5+5 (4,368) 417 ->
+// 391 us with 512, rows of up to 32 groups best with 256 (3x4 6+6: 26 -> 23 us),
+// longer ones with 512 (4x4 4+4: 64 against 68 us).  128 threads were slower
+// everywhere but on 1,001 columns.
+struct ApplyCtas {
+  int threads, per_sm;
+};
+static ApplyCtas apply_ctas(const OpView& v, int precision) {
+  const int total = kApplyThreads * (precision == MB_PREC_F32 ? kApplyCtasPerSm<float> : 1);
+  const size_t row = apply_smem(v, precision, apply_staged(v, precision)) + 2048;
+  const size_t sm = (size_t)max_smem_optin() + 1024;
+  int threads = precision == MB_PREC_F32 && v.Dd > 32 * 32 ? 512 : 256;
+  while (threads < kApplyThreads && (size_t)(total / threads) * row > sm) threads *= 2;
+  return {threads, total / threads};
+}
+
 static int csr_grid(const OpView& v, int precision);
 
 int apply_grid(const OpView& v, int precision) {
@@ -434,7 +455,7 @@ int apply_grid(const OpView& v, int precision) {
     return g;
   }
   if (v.csr_row) return csr_grid(v, precision);
-  int64_t g = (int64_t)num_sms() * (precision == MB_PREC_F32 ? kApplyCtasPerSm<float> : 1);
+  int64_t g = (int64_t)num_sms() * apply_ctas(v, precision).per_sm;
   if (g > v.Du) g = v.Du;
   return (int)(g > 0 ? g : 1);
 }
@@ -450,7 +471,7 @@ static void apply_t(const OpView& v, const void* x, void* y, double scale, doubl
   const T* su = sizeof(T) == 8 ? (const T*)v.self_up : (const T*)v.self_up_f;
   const T* sd = sizeof(T) == 8 ? (const T*)v.self_dn : (const T*)v.self_dn_f;
   const int precision = sizeof(T) == 4 ? MB_PREC_F32 : MB_PREC_F64;
-  kern<<<apply_grid(v, precision), kApplyThreads, smem, st>>>(v, (const V2*)x, (V2*)y, (T)(-v.t * scale), (T)scale,
+  kern<<<apply_grid(v, precision), apply_ctas(v, precision).threads, smem, st>>>(v, (const V2*)x, (V2*)y, (T)(-v.t * scale), (T)scale,
                                           (T)shift, (T)beta, (const V2*)z, uf, su, sd, partials);
   MB_CUDA(cudaGetLastError());
 }
@@ -681,8 +702,9 @@ void launch_eng_fused(const OpView& v, const EngFusedArgs& a, cudaStream_t st) {
   const bool staged = apply_staged(v, MB_PREC_F32);
   const size_t smem = apply_smem(v, MB_PREC_F32, staged);
   const int grid = apply_grid(v, MB_PREC_F32);
-  if (staged) k_eng_fused<true><<<grid, kApplyThreads, smem, st>>>(v, a);
-  else k_eng_fused<false><<<grid, kApplyThreads, smem, st>>>(v, a);
+  const int threads = apply_ctas(v, MB_PREC_F32).threads;
+  if (staged) k_eng_fused<true><<<grid, threads, smem, st>>>(v, a);
+  else k_eng_fused<false><<<grid, threads, smem, st>>>(v, a);
   k_eng_fused_place<<<1, 256, 0, st>>>(a, grid);
   MB_CUDA(cudaGetLastError());
 }
