@@ -133,6 +133,93 @@ std::vector<int32_t> rcm_order(const HopTable& t, int64_t D) {
   return order;
 }
 
+std::vector<int32_t> low_first_order(const SpinSector& s) {
+  std::vector<std::pair<uint32_t, int32_t>> key((size_t)s.D);
+  for (int64_t r = 0; r < s.D; ++r) {
+    uint32_t m = s.masks[(size_t)r], k = 0;
+    for (int i = 0; i < 32; ++i, m >>= 1) k = (k << 1) | (m & 1u);
+    key[(size_t)r] = {k, (int32_t)r};
+  }
+  std::sort(key.begin(), key.end());
+  std::vector<int32_t> out((size_t)s.D);
+  for (int64_t r = 0; r < s.D; ++r) out[(size_t)r] = key[(size_t)r].second;
+  return out;
+}
+
+OrderTiles order_tiles(int L, const SpinSector& up, const SpinSector& dn, int slots) {
+  OrderTiles out;
+  const Binom& B = binom_table();
+  const int h = std::min(kTileHigh, (L + 1) / 2), m = L - h;
+  // the high occupations of n particles, colex
+  auto highs = [&](int n) {
+    std::vector<uint32_t> v;
+    for (uint32_t x = 0; x < (1u << h); ++x)
+      if (__builtin_popcount(x) == n) v.push_back(x);
+    return v;
+  };
+  // columns: per low Down count, the first column of every high occupation
+  std::vector<int> col_of((size_t)m + 1, -1), col_n((size_t)m + 1, 0);
+  for (int nl = std::max(0, dn.n - h); nl <= std::min(m, dn.n); ++nl) {
+    col_of[(size_t)nl] = (int)out.cols.size();
+    for (uint32_t x : highs(dn.n - nl))
+      out.cols.push_back((int32_t)colex_rank(B, (x << m) | ((1u << nl) - 1u)));
+    col_n[(size_t)nl] = (int)out.cols.size() - col_of[(size_t)nl];
+  }
+  // slots: per high counts (Up, Down), the pairs' places in the reference
+  // order of the high part
+  std::map<std::pair<int, int>, int> place_of;
+  auto places = [&](int nu, int nd) {
+    const auto key = std::make_pair(nu, nd);
+    const auto it = place_of.find(key);
+    if (it != place_of.end()) return it->second;
+    const int at = (int)out.place.size();
+    std::vector<std::pair<int64_t, int>> rank;
+    int pair = 0;
+    for (uint32_t u : highs(nu))
+      for (uint32_t d : highs(nd)) rank.push_back({reference_rank(B, u, d, h), pair++});
+    std::sort(rank.begin(), rank.end());
+    out.place.resize((size_t)(at + pair));
+    for (int i = 0; i < pair; ++i) out.place[(size_t)(at + rank[(size_t)i].second)] = (uint8_t)i;
+    place_of[key] = at;
+    return at;
+  };
+  // low Up occupations in the reference order's sense (from orbital 0 up)
+  std::vector<std::pair<uint32_t, uint32_t>> ul;
+  for (int n = std::max(0, up.n - h); n <= std::min(m, up.n); ++n)
+    for (uint32_t x : make_sector(m, n).masks) {
+      uint32_t key = 0;
+      for (int i = 0; i < m; ++i) key = (key << 1) | ((x >> i) & 1u);
+      ul.push_back({key, x});
+    }
+  std::sort(ul.begin(), ul.end());
+  for (const auto& [key, x] : ul) {
+    (void)key;
+    const int nu = up.n - __builtin_popcount(x);
+    const int row = (int)out.rows.size();
+    for (uint32_t u : highs(nu)) out.rows.push_back((int32_t)colex_rank(B, (u << m) | x));
+    const int n_rows = (int)out.rows.size() - row;
+    for (int nl = 0; nl <= m; ++nl) {
+      if (col_of[(size_t)nl] < 0) continue;
+      const int place = places(nu, dn.n - nl), nt = n_rows * col_n[(size_t)nl];
+      const int kw = std::max(1, slots / (nt | 1));
+      const int64_t all = B.c[m][nl], step = (int64_t)kTileWarps * kw;
+      for (int64_t k0 = 0; k0 < all; k0 += step) {
+        OrderTile t{};
+        t.row = row;
+        t.n_rows = n_rows;
+        t.col = col_of[(size_t)nl];
+        t.n_cols = col_n[(size_t)nl];
+        t.k0 = (int32_t)k0;
+        t.k = (int32_t)std::min<int64_t>(step, all - k0);
+        t.place = place;
+        t.kw = kw;
+        out.tiles.push_back(t);
+      }
+    }
+  }
+  return out;
+}
+
 SignedLists signed_lists(const HopTable& t, int64_t D) {
   SignedLists s;
   s.off.resize((size_t)D + 1);

@@ -225,6 +225,9 @@ HopTable build_hop_table(const SpinSector& s, const mb_model_s& m);
 // The masks of one spin sector (n of L orbitals) in colex order.
 SpinSector make_spin_sector(int L, int n);
 
+// The states of a spin sector sorted by their masks read from orbital 0 up.
+std::vector<int32_t> low_first_order(const SpinSector& s);
+
 // Reverse Cuthill-McKee order of the states of a hop table (BFS from a
 // low-degree state, neighbours by increasing degree, reversed).
 std::vector<int32_t> rcm_order(const HopTable& t, int64_t D);
@@ -313,6 +316,15 @@ SlicedTable16 sliced_table16(const SlicedTable& s, int64_t D);
 // accumulates for k doubly occupied sites (matrix_elements.h:85-96).
 std::vector<double> u_fold_table(double u, bool has_u, int L);
 
+// dot_mode / dots of an apply whose result goes to reference order, y[out_perm[i]]
+// (no dots; a Q64 apply writes complex128).  The scattered stores ride along in
+// a kernel that is bound elsewhere, where a move of its own reads and writes the
+// vector once more.  Such a launch takes the rows by low_first_order, so that
+// the elements of a sector of the result are written close together (in the
+// Cuthill-McKee order L2 wrote them back half filled: 4x4 6+6 complex128 4.82
+// against 4.71 ms, 1D L=16 8+8 10.6 against 9.5, complex64 6.6 against 5.1).
+constexpr int kRefOut = 8;
+
 // Device-side view of an operator (POD; passed to kernels by value).
 struct OpView {
   int64_t Du, Dd, dim;
@@ -390,6 +402,8 @@ struct OpView {
   int n_blocks;
   const OpView* sub;
   const int64_t* sub_off;
+  // of launches with kRefOut: tensor -> reference index
+  const int32_t* out_perm;
   double t;
   int max_up_degree;
   int max_dn_degree;
@@ -433,6 +447,41 @@ void fill_fused_tables(OpView& v, const HopTable& tu, const HopTable& td, int64_
 
 }  // namespace mb
 
+namespace mb {
+// The reference order of a lattice operator's vectors (device arrays): perm
+// (tensor -> reference index) and the tiles that moves between the two orders
+// take (mb_rows.h).
+constexpr int kTileHigh = 4;    // the orbitals of a tile's high part, at most
+constexpr int kTileWarps = 4;   // warps of a tile's block
+constexpr int kTilePairs = 36;  // its pairs of high occupations, at most: C(4,2)^2
+struct OrderTile {
+  int32_t row, n_rows;  // rows[row ..]: the tensor rows, by high Up occupation
+  int32_t col, n_cols;  // cols[col ..]: a high Down occupation's first column
+  int32_t k0, k;        // columns k0 .. k0 + k - 1 after it
+  int32_t place;        // place[place ..]: slots of the (row, col) pairs
+  int32_t kw;           // columns a warp takes
+};
+struct RowOrder {
+  int64_t Dd = 0;
+  const int32_t* perm = nullptr;
+  const OrderTile* tiles = nullptr;  // nullptr: not a lattice operator
+  const int32_t* rows = nullptr;
+  const int32_t* cols = nullptr;
+  const uint8_t* place = nullptr;
+  int64_t n_tiles = 0;
+  int warp_slots = 0;  // a warp's shared-memory elements, and bytes with their indices
+  int warp_bytes = 0;
+};
+// The host arrays of a sector's tiles.
+struct OrderTiles {
+  std::vector<OrderTile> tiles;
+  std::vector<int32_t> rows, cols;
+  std::vector<uint8_t> place;
+};
+// slots: a warp's shared-memory elements (at least kTilePairs + 1, below 1024)
+OrderTiles order_tiles(int L, const SpinSector& up, const SpinSector& dn, int slots);
+}  // namespace mb
+
 struct mb_op_s {
   int device = 0;
   int precision = MB_PREC_F64;
@@ -447,6 +496,8 @@ struct mb_op_s {
   std::vector<void*> allocations;  // device buffers owned by the op
   int32_t* perm = nullptr;         // tensor -> reference index (lazy)
   int32_t* iperm = nullptr;        // reference -> tensor index (lazy)
+  mb::RowOrder order;              // of a lattice operator (with perm, lazy)
+  const int32_t* low_rows = nullptr;  // its rows by low_first_order
   std::mutex mu;
   std::mutex host_mu;  // host-buffer calls: the lane pool and the row groups
   std::mutex host_link_mu;  // host-buffer calls on page-locked vectors take turns
@@ -560,6 +611,27 @@ void launch_gather(int precision, int64_t n, const int32_t* perm, const void* sr
                    cudaStream_t st);   // dst[i] = src[perm[i]]
 void launch_scatter(int precision, int64_t n, const int32_t* perm, const void* src, void* dst,
                     cudaStream_t st);  // dst[perm[i]] = src[i]
+// Whether a move between the orders goes by tiles (mb_rows.h): a vector that L2
+// does not hold.  Smaller ones are gathered element by element from L2, which
+// needs fewer steps than a tile's trip through shared memory (one move, 4x4 4+4
+// complex128, 53 MB: 26 against 38 us; 1D L=14 7+7, 188 MB: 135 against 100 us;
+// 4x4 6+6, 1.03 GB: 1.2 ms against 0.52; complex64 0.85 ms against 0.27).
+constexpr int64_t kTileBytes = 100000000;
+// Whether an apply of a reference-order call writes its result itself (kRefOut).
+// complex128 always: its apply hides the scattered stores (reference-order call,
+// ms, against a tile move after it: 4x4 5+5 1.38 / 1.48, 6+6 4.71 / 5.05, 1D L=16
+// 8+8 9.46 / 9.93).  The complex64 and Q64 applies are faster and lose on
+// vectors well past L2 (4x4 5+5: 0.579 / 0.576 and 1.21 / 1.15; 6+6: 2.17 / 1.98
+// and 3.88 / 3.70; 1D L=14 7+7: 0.263 / 0.267 and 0.580 / 0.580).
+inline bool writes_reference(int precision, int64_t dim) {
+  return precision == MB_PREC_F64 ||
+         (precision == MB_PREC_F32 ? 8 : 16) * dim < 2 * kTileBytes;
+}
+// dst = src in tensor order / in reference order, a lattice operator's vectors
+void launch_to_tensor(int precision, const RowOrder& o, const void* src, void* dst,
+                      cudaStream_t st);
+void launch_from_tensor(int precision, const RowOrder& o, const void* src, void* dst,
+                        cudaStream_t st);
 void launch_fill_rng(int precision, int64_t Du, int64_t Dd, uint64_t seed, uint32_t stream_id,
                      int phase, void* dst, cudaStream_t st);
 void launch_perm(const OpView& v, int32_t* perm, cudaStream_t st);
@@ -571,6 +643,10 @@ void upload_binomials(cudaStream_t st);
 int32_t* op_perm(mb_op_s* op);
 // reference -> tensor index table (inverse of op_perm), built on first use
 int32_t* op_iperm(mb_op_s* op);
+// the operator's reference order (built on first use); perm and tiles are
+// nullptr where the operator's own index is the reference order, tiles alone
+// where it is no lattice operator of one sector
+RowOrder op_row_order(mb_op_s* op);
 // first[r] = the smallest reference index of tensor row r's states
 void launch_row_first(int64_t Du, int64_t Dd, const int32_t* perm, int32_t* first,
                       cudaStream_t st);

@@ -11,6 +11,7 @@
 
 #include "mb_internal.h"
 #include "mb_isum.h"
+#include "mb_rows.h"
 
 namespace mb {
 
@@ -354,13 +355,13 @@ __device__ __forceinline__ void apply_rows(
         out.x = fma(beta, zv.x, out.x);
         out.y = fma(beta, zv.y, out.y);
       }
-      y[idx] = out;
+      y[DOTS & kRefOut ? (int64_t)__ldcs(v.out_perm + idx) : idx] = out;
       if (DOTS & 1) { a_xy.add_prod(xv.x, out.x); a_xy.add_prod(xv.y, out.y); }
       if (DOTS & 2) { a_yy.add_prod(out.x, out.x); a_yy.add_prod(out.y, out.y); }
       if (DOTS & 4) { a_xx.add_prod(xv.x, xv.x); a_xx.add_prod(xv.y, xv.y); }
     }
   }
-  if (DOTS) {
+  if (DOTS & 7) {
     double vals[3] = {a_xy.value(), a_yy.value(), a_xx.value()};
     block_reduce_store<3>(vals, partials);
   }
@@ -486,6 +487,7 @@ static void apply_dots(const OpView& v, const void* x, void* y, double scale, do
     case 2: apply_t<T, STAGED, 2>(v, x, y, scale, shift, beta, z, partials, st); break;
     case 3: apply_t<T, STAGED, 3>(v, x, y, scale, shift, beta, z, partials, st); break;
     case 5: apply_t<T, STAGED, 5>(v, x, y, scale, shift, beta, z, partials, st); break;
+    case kRefOut: apply_t<T, STAGED, kRefOut>(v, x, y, scale, shift, beta, z, partials, st); break;
     default: apply_t<T, STAGED, 7>(v, x, y, scale, shift, beta, z, partials, st); break;
   }
 }
@@ -1048,6 +1050,26 @@ void launch_scatter(int precision, int64_t n, const int32_t* perm, const void* s
   if (precision == MB_PREC_F32) k_permute<float2, true><<<g, kBlasThreads, 0, st>>>(n, perm, (const float2*)src, (float2*)dst);
   else k_permute<double2, true><<<g, kBlasThreads, 0, st>>>(n, perm, (const double2*)src, (double2*)dst);
   MB_CUDA(cudaGetLastError());
+}
+
+namespace {
+struct Same {
+  __device__ void start() {}
+  template <typename V2>
+  __device__ V2 operator()(const V2& v) const { return v; }
+};
+}  // namespace
+
+void launch_to_tensor(int precision, const RowOrder& o, const void* src, void* dst,
+                      cudaStream_t st) {
+  if (precision == MB_PREC_F32) launch_tiles<false>(o, (const float2*)src, (float2*)dst, Same{}, st);
+  else launch_tiles<false>(o, (const double2*)src, (double2*)dst, Same{}, st);
+}
+
+void launch_from_tensor(int precision, const RowOrder& o, const void* src, void* dst,
+                        cudaStream_t st) {
+  if (precision == MB_PREC_F32) launch_tiles<true>(o, (const float2*)src, (float2*)dst, Same{}, st);
+  else launch_tiles<true>(o, (const double2*)src, (double2*)dst, Same{}, st);
 }
 
 // ---------------------------------------------------------------------------

@@ -131,7 +131,7 @@ void noalloc_apply_q64(mb_op_s* op, const void* x, void* y, int dev, cudaStream_
   const int grid = blas_grid(op->dim);
   k_noalloc_permute<double2, true><<<grid, 256, 0, st>>>(op->view, (const double2*)x, a);
   MB_CUDA(cudaGetLastError());
-  launch_f64_to_q(op->dim, a, nullptr, op->q_qbits, ints, b, st);
+  launch_f64_to_q(op->dim, a, RowOrder{}, op->q_qbits, ints, b, st);
   launch_q_plan(q_plain_plan_input(op), ints + 1, prm, st);
   launch_apply_q(op->view, b, a, nullptr, prm, nullptr, nullptr, 0, st);
   launch_q_to_f64(op->dim, a, nullptr, &prm->ey, b, st);

@@ -141,6 +141,7 @@ static void build_op(mb_op_s* op, const mb_basis_s* b, const mb_model_s* m) {
   v.L = op->L;
   v.t = m->t;
   v.up_mask = upload(op, b->up.masks);
+  op->low_rows = upload(op, low_first_order(b->up));
   v.up_off = upload(op, tu.off);
   v.up_ent = upload(op, tu.ent.empty() ? std::vector<uint32_t>{0u} : tu.ent);
   if (same) {
@@ -496,6 +497,35 @@ int32_t* op_iperm(mb_op_s* op) {
   return op->iperm;
 }
 
+// a warp's slots of 8- and 16-byte elements: 12 and 10 KB of shared memory
+constexpr int kTileSlots32 = 1016, kTileSlots64 = 512;
+
+RowOrder op_row_order(mb_op_s* op) {
+  RowOrder none;
+  none.perm = op_perm(op);
+  if (op->natural_order || op->view.n_blocks ||
+      (int64_t)elem_bytes(op->precision) * op->dim < kTileBytes)
+    return none;
+  std::lock_guard<std::mutex> lk(op->mu);
+  if (!op->order.tiles) {
+    const size_t es = elem_bytes(op->precision);
+    RowOrder o;
+    o.warp_slots = es == 8 ? kTileSlots32 : kTileSlots64;
+    o.warp_bytes = (int)((es + sizeof(int32_t)) * (size_t)o.warp_slots);
+    const OrderTiles t = order_tiles(op->L, make_spin_sector(op->L, op->n_up),
+                                     make_spin_sector(op->L, op->n_down), o.warp_slots);
+    o.Dd = op->Dd;
+    o.perm = op->perm;
+    o.rows = upload(op, t.rows);
+    o.cols = upload(op, t.cols);
+    o.place = upload(op, t.place);
+    o.n_tiles = (int64_t)t.tiles.size();
+    o.tiles = upload(op, t.tiles);
+    op->order = o;
+  }
+  return op->order;
+}
+
 static void to_tensor(mb_op_s* op, const void* src, void* dst, int order, cudaStream_t st) {
   if (order == MB_ORDER_TENSOR || op->natural_order) {
     if (src != dst)
@@ -503,8 +533,9 @@ static void to_tensor(mb_op_s* op, const void* src, void* dst, int order, cudaSt
                               cudaMemcpyDeviceToDevice, st));
     return;
   }
-  ensure_perm(op);
-  launch_gather(op->precision, op->dim, op->perm, src, dst, st);
+  const RowOrder o = op_row_order(op);
+  if (o.tiles) launch_to_tensor(op->precision, o, src, dst, st);
+  else launch_gather(op->precision, op->dim, o.perm, src, dst, st);
 }
 
 static void from_tensor(mb_op_s* op, const void* src, void* dst, int order, cudaStream_t st) {
@@ -514,8 +545,9 @@ static void from_tensor(mb_op_s* op, const void* src, void* dst, int order, cuda
                               cudaMemcpyDeviceToDevice, st));
     return;
   }
-  // y_ref[i] = y_tensor[iperm[i]]: coalesced writes, random reads
-  launch_gather(op->precision, op->dim, op_iperm(op), src, dst, st);
+  const RowOrder o = op_row_order(op);
+  if (o.tiles) launch_from_tensor(op->precision, o, src, dst, st);
+  else launch_gather(op->precision, op->dim, op_iperm(op), src, dst, st);
 }
 
 // The row groups of the pipelined host-buffer applies.  Rows are ordered by
@@ -703,13 +735,22 @@ static void apply_affine(mb_op_s* op, const void* x, void* y, double scale, doub
                  nullptr, 0, st);
     return;
   }
-  auto& s = scratch_for(op, st, 2);
+  const bool lattice = !op->natural_order && !op->view.n_blocks && !op->view.csr_row;
+  const bool fused = lattice && writes_reference(op->precision, op->dim);
+  auto& s = scratch_for(op, st, fused && beta == 0.0 ? 1 : 2);
   to_tensor(op, x, s.a, order, st);
   const void* zt = nullptr;
   if (beta != 0.0) {
     // z gathered into y's slot would clobber z when z == y; use b then swap roles.
     to_tensor(op, z, s.b, order, st);
     zt = s.b;
+  }
+  if (fused) {
+    OpView v = op->view;
+    v.out_perm = op_perm(op);
+    v.row_sched = op->low_rows;
+    launch_apply(v, op->precision, s.a, y, scale, shift, beta, zt, nullptr, kRefOut, st);
+    return;
   }
   // In-place on s.b when z is used: each element reads z[i] before writing y[i].
   launch_apply(op->view, op->precision, s.a, s.b, scale, shift, beta, zt, nullptr, 0, st);

@@ -25,6 +25,7 @@
 
 #include "mb_internal.h"
 #include "mb_q64.h"
+#include "mb_rows.h"
 
 namespace mb {
 
@@ -424,7 +425,7 @@ k_apply_q(OpView v, const longlong2* __restrict__ x, longlong2* y, const longlon
   uint32_t* s_up = reinterpret_cast<uint32_t*>(smem + (STAGED ? row_bytes + 16 * kSlicedPads : 0));
   __shared__ long long s_cq[kMaxOrbitals + 1];
   __shared__ long long s_c1, s_c3;
-  __shared__ int s_sh;
+  __shared__ int s_sh, s_ey;
   if (threadIdx.x <= (unsigned)v.L) s_cq[threadIdx.x] = prm->cq[threadIdx.x];
   if (STAGED && threadIdx.x < kSlicedPads)
     reinterpret_cast<longlong2*>(smem + row_bytes)[threadIdx.x] = make_longlong2(0, 0);
@@ -432,6 +433,7 @@ k_apply_q(OpView v, const longlong2* __restrict__ x, longlong2* y, const longlon
     s_c1 = prm->c1;
     s_c3 = prm->c3;
     s_sh = prm->sh;
+    s_ey = prm->ey;
   }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   const int64_t ngroups = (Dd + 31) >> 5;
@@ -560,14 +562,18 @@ k_apply_q(OpView v, const longlong2* __restrict__ x, longlong2* y, const longlon
       longlong2 out;
       out.x = round_shift(pr, sh);
       out.y = round_shift(pi, sh);
-      y[idx] = out;
+      if (DOTS & kRefOut)
+        reinterpret_cast<double2*>(y)[__ldcs(v.out_perm + idx)] =
+            make_double2(fixed_to_f64(out.x, s_ey), fixed_to_f64(out.y, s_ey));
+      else
+        y[idx] = out;
       if (DOTS & 1) a_xy += prod_hi(xv.x, out.x) + prod_hi(xv.y, out.y);
       if (DOTS & 2) a_yy += prod_hi(out.x, out.x) + prod_hi(out.y, out.y);
       if (DOTS & 4) mor |= mag(out.x) | mag(out.y);
     }
   }
   if (TS) asm volatile("cp.async.wait_all;" ::: "memory");
-  if (DOTS) q_block_reduce_exact(a_xy, a_yy, mor, reinterpret_cast<long long*>(partials), max_or);
+  if (DOTS & 7) q_block_reduce_exact(a_xy, a_yy, mor, reinterpret_cast<long long*>(partials), max_or);
 }
 
 static int sm_count() {
@@ -759,7 +765,9 @@ static void q_apply_sel(const OpView& v, const void* x, void* y, const void* z,
     else if (dots) q_apply_t<STAGED, 7, true, UPS, TB>(v, x, y, z, prm, partials, max_or, ups, st);
     else q_apply_t<STAGED, 0, true, UPS, TB>(v, x, y, z, prm, partials, max_or, ups, st);
   } else {
-    if (dots == 5) q_apply_t<STAGED, 5, false, UPS, TB>(v, x, y, z, prm, partials, max_or, ups, st);
+    if (dots == kRefOut)
+      q_apply_t<STAGED, kRefOut, false, UPS, TB>(v, x, y, z, prm, partials, max_or, ups, st);
+    else if (dots == 5) q_apply_t<STAGED, 5, false, UPS, TB>(v, x, y, z, prm, partials, max_or, ups, st);
     else if (dots) q_apply_t<STAGED, 7, false, UPS, TB>(v, x, y, z, prm, partials, max_or, ups, st);
     else q_apply_t<STAGED, 0, false, UPS, TB>(v, x, y, z, prm, partials, max_or, ups, st);
   }
@@ -778,7 +786,9 @@ static void q_apply_ts(const OpView& v, const void* x, void* y, const void* z,
     if (dots) q_apply_t<true, 7, true, false, 32, true>(v, x, y, z, prm, partials, max_or, nullptr, st);
     else q_apply_t<true, 0, true, false, 32, true>(v, x, y, z, prm, partials, max_or, nullptr, st);
   } else {
-    if (dots) q_apply_t<true, 7, false, false, 32, true>(v, x, y, z, prm, partials, max_or, nullptr, st);
+    if (dots == kRefOut)
+      q_apply_t<true, kRefOut, false, false, 32, true>(v, x, y, z, prm, partials, max_or, nullptr, st);
+    else if (dots) q_apply_t<true, 7, false, false, 32, true>(v, x, y, z, prm, partials, max_or, nullptr, st);
     else q_apply_t<true, 0, false, false, 32, true>(v, x, y, z, prm, partials, max_or, nullptr, st);
   }
 }
@@ -913,8 +923,9 @@ __global__ void k_exp_from_max(const int* __restrict__ emax, int qbits, int* __r
   *ex = (e == 0) ? -1074 : (e - 1022 - qbits);
 }
 
-__global__ void k_to_fixed(int64_t n, const double2* __restrict__ src, const int32_t* __restrict__ perm,
-                           const int* __restrict__ ex, longlong2* __restrict__ dst) {
+__global__ void k_to_fixed(int64_t n, const double2* __restrict__ src,
+                           const int32_t* __restrict__ perm, const int* __restrict__ ex,
+                           longlong2* __restrict__ dst) {
   const int E = *ex;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x) {
@@ -922,6 +933,24 @@ __global__ void k_to_fixed(int64_t n, const double2* __restrict__ src, const int
     dst[i] = make_longlong2(f64_to_fixed(v.x, E), f64_to_fixed(v.y, E));
   }
 }
+
+// element conversions of the moves between the two orders (mb_rows.h)
+struct ToFixed {
+  const int* ex;
+  int E;
+  __device__ void start() { E = *ex; }
+  __device__ longlong2 operator()(const double2& v) const {
+    return make_longlong2(f64_to_fixed(v.x, E), f64_to_fixed(v.y, E));
+  }
+};
+struct FromFixed {
+  const int* ex;
+  int E;
+  __device__ void start() { E = *ex; }
+  __device__ double2 operator()(const longlong2& q) const {
+    return make_double2(fixed_to_f64(q.x, E), fixed_to_f64(q.y, E));
+  }
+};
 
 // dst[i] = value(src[iperm ? iperm[i] : i]) (iperm: reference -> tensor index)
 __global__ void k_from_fixed(int64_t n, const longlong2* __restrict__ src,
@@ -974,13 +1003,16 @@ __global__ void k_plan(QPlanInput in, const int* __restrict__ ex, QParams* __res
   q_plan(p, in);
 }
 
-void launch_f64_to_q(int64_t n, const void* src, const int32_t* perm, int qbits, int* scratch_int2,
+void launch_f64_to_q(int64_t n, const void* src, const RowOrder& o, int qbits, int* scratch_int2,
                      void* dst, cudaStream_t st) {
   MB_CUDA(cudaMemsetAsync(scratch_int2, 0, sizeof(int), st));
   k_f64_maxexp<<<q_blas_grid(n), kQBlas, 0, st>>>(n, (const double2*)src, scratch_int2);
   k_exp_from_max<<<1, 1, 0, st>>>(scratch_int2, qbits, scratch_int2 + 1);
-  k_to_fixed<<<q_blas_grid(n), kQBlas, 0, st>>>(n, (const double2*)src, perm, scratch_int2 + 1,
-                                                 (longlong2*)dst);
+  if (o.tiles)
+    launch_tiles<false>(o, (const double2*)src, (longlong2*)dst, ToFixed{scratch_int2 + 1, 0}, st);
+  else
+    k_to_fixed<<<q_blas_grid(n), kQBlas, 0, st>>>(n, (const double2*)src, o.perm,
+                                                  scratch_int2 + 1, (longlong2*)dst);
   MB_CUDA(cudaGetLastError());
 }
 
@@ -1003,6 +1035,11 @@ void launch_q_to_f64(int64_t n, const void* src, const int32_t* iperm, const int
   k_from_fixed<<<q_blas_grid(n), kQBlas, 0, st>>>(n, (const longlong2*)src, iperm, e_dev,
                                                    (double2*)dst);
   MB_CUDA(cudaGetLastError());
+}
+
+void launch_q_to_f64(const RowOrder& o, const void* src, const int* e_dev, void* dst,
+                     cudaStream_t st) {
+  launch_tiles<true>(o, (const longlong2*)src, (double2*)dst, FromFixed{e_dev, 0}, st);
 }
 
 void launch_q_plan(const QPlanInput& in, const int* ex_dev, QParams* p_dev, cudaStream_t st) {

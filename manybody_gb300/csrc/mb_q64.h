@@ -48,7 +48,8 @@ QPlanInput q_plain_plan_input(const mb_op_s* op);
 // The fused apply (see mb_q64.cu).  y must not alias x or z.  With ups (the
 // column pass's up-hop sums of x, launch_upcol_q) the up hops are read from
 // it; without, they are gathered from x in the same pass.  dots: 0 none;
-// 5 Re<x,y> and max |y| (<y,y> left 0); any other non-zero value all three.
+// 5 Re<x,y> and max |y| (<y,y> left 0); kRefOut (no z) none, y complex128 in
+// reference order; any other non-zero value all three.
 void launch_apply_q(const OpView& v, const void* x, void* y, const void* z, const QParams* prm_dev,
                     double* partials, unsigned long long* max_or, int dots, cudaStream_t st,
                     const void* ups = nullptr);
@@ -67,10 +68,10 @@ int q_apply_grid(const OpView& v);
 int q_blas_grid(int64_t n);
 int q_multi_dot_grid(int64_t n);
 
-// FP64 (tensor or, through perm, reference order) -> Q64 with the exponent
+// FP64 (tensor order, or with o.perm reference order) -> Q64 with the exponent
 // chosen from the vector's largest magnitude; scratch_int2 = 2 device ints
 // (max biased exponent, resulting E).
-void launch_f64_to_q(int64_t n, const void* src, const int32_t* perm, int qbits, int* scratch_int2,
+void launch_f64_to_q(int64_t n, const void* src, const RowOrder& o, int qbits, int* scratch_int2,
                      void* dst, cudaStream_t st);
 // dst[iperm[i]] = src[i] for a reference-order complex128 chunk, its largest
 // biased exponent folded into *emax (atomic max; zero it before the first).
@@ -82,6 +83,9 @@ void launch_f64_to_q_inplace(int64_t n, void* buf, int qbits, int* scratch_int2,
 // Q64 (tensor order) -> FP64; with iperm (reference -> tensor index) the
 // output is in reference order.
 void launch_q_to_f64(int64_t n, const void* src, const int32_t* iperm, const int* e_dev, void* dst,
+                     cudaStream_t st);
+// the whole vector to reference order by tiles
+void launch_q_to_f64(const RowOrder& o, const void* src, const int* e_dev, void* dst,
                      cudaStream_t st);
 void launch_q_plan(const QPlanInput& in, const int* ex_dev, QParams* p_dev, cudaStream_t st);
 void launch_q_lincomb(int64_t n, const void* a, long long ar, long long ai, const void* b,

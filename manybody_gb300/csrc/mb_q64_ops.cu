@@ -152,7 +152,7 @@ void q_tune_prepare(mb_op_s* op, void** xq, void** yq, void** prm, cudaStream_t 
     MB_CUDA(cudaMalloc(&b, vb));
     MB_CUDA(cudaMalloc(&p, sizeof(QParams)));
     launch_fill_rng(MB_PREC_F64, op->Du, op->Dd, 12345, 0, 0, x64.p, st);
-    launch_f64_to_q(op->dim, x64.p, nullptr, op->q_qbits, (int*)ints.p, a, st);
+    launch_f64_to_q(op->dim, x64.p, RowOrder{}, op->q_qbits, (int*)ints.p, a, st);
     launch_q_plan(q_plain_plan_input(op), (const int*)ints.p + 1, (QParams*)p, st);
     MB_CUDA(cudaStreamSynchronize(st));
   } catch (...) {
@@ -169,27 +169,43 @@ void q_tune_apply(mb_op_s* op, const void* xq, void* yq, const void* prm, cudaSt
   q_apply_whole(op, xq, yq, nullptr, (const QParams*)prm, nullptr, nullptr, 0, st);
 }
 
+// Q64 (tensor order) -> complex128 in `order`.
+static void q_to_order(mb_op_s* op, const void* src, int order, const int* e_dev, void* dst,
+                       cudaStream_t st) {
+  const RowOrder o = order == MB_ORDER_REFERENCE ? op_row_order(op) : RowOrder{};
+  if (o.tiles) launch_q_to_f64(o, src, e_dev, dst, st);
+  else launch_q_to_f64(op->dim, src, o.perm ? op_iperm(op) : nullptr, e_dev, dst, st);
+}
+
 // y = scale (H - shift) x + beta z on complex128 vectors through Q64.
 // z, when used, is folded in FP64 after the Q64 apply (z keeps its own
 // magnitude): y = Q64[scale (H - shift) x] + beta z.
 void q_apply_affine(mb_op_s* op, const void* x, void* y, double scale, double shift, double beta,
                     const void* z, int order, cudaStream_t st) {
   auto& s = qscratch_for(op, st);
-  int32_t* perm = order == MB_ORDER_REFERENCE ? op_perm(op) : nullptr;
-  int32_t* iperm = order == MB_ORDER_REFERENCE ? op_iperm(op) : nullptr;
-  launch_f64_to_q(op->dim, x, perm, op->q_qbits, s.ints, s.xq, st);
+  const RowOrder o = order == MB_ORDER_REFERENCE ? op_row_order(op) : RowOrder{};
+  launch_f64_to_q(op->dim, x, o, op->q_qbits, s.ints, s.xq, st);
   launch_q_plan(plan_input(op, scale, shift, 0.0, 0, 0, false), s.ints + 1, (QParams*)s.prm, st);
+  if (!z && o.perm && !op->view.csr_row && writes_reference(MB_PREC_Q64, op->dim)) {
+    OpView v = op->view;
+    v.out_perm = o.perm;
+    v.row_sched = op->low_rows;
+    void* ups = q_ups_for(op, st);
+    if (ups) launch_upcol_q(v, s.xq, ups, st);
+    launch_apply_q(v, s.xq, y, nullptr, (const QParams*)s.prm, nullptr, nullptr, kRefOut, st, ups);
+    return;
+  }
   q_apply_whole(op, s.xq, s.yq, nullptr, (const QParams*)s.prm, nullptr, nullptr, 0, st);
   // the output exponent sits in the planned QParams (field ey)
   const int* ey = (const int*)((const char*)s.prm + offsetof(QParams, ey));
   if (!z) {
-    launch_q_to_f64(op->dim, s.yq, iperm, ey, y, st);
+    q_to_order(op, s.yq, order, ey, y, st);
     return;
   }
   // y = beta z + (Q64 result): z may alias y; convert into a tensor-order
   // temporary, then combine with the FP64 vector kernel.
   QBuf tmp(sizeof(double2) * (size_t)op->dim);
-  launch_q_to_f64(op->dim, s.yq, iperm, ey, tmp.p, st);
+  q_to_order(op, s.yq, order, ey, tmp.p, st);
   launch_axpby(MB_PREC_F64, op->dim, beta, 0.0, z, 1.0, 0.0, tmp.p, nullptr, 0, st);
   MB_CUDA(cudaMemcpyAsync(y, tmp.p, sizeof(double2) * (size_t)op->dim, cudaMemcpyDeviceToDevice, st));
   MB_CUDA(cudaStreamSynchronize(st));
@@ -616,9 +632,9 @@ struct QKrylov {
 
   // complex128 (order) -> Q64 tensor order; returns ||b||.
   double load(const void* src, int order, QRef& out) {
-    int32_t* perm = order == MB_ORDER_REFERENCE ? op_perm(op) : nullptr;
+    const RowOrder o = order == MB_ORDER_REFERENCE ? op_row_order(op) : RowOrder{};
     QBuf ints(4 * sizeof(int));
-    launch_f64_to_q(n, src, perm, qbits, (int*)ints.p, out.p, st);
+    launch_f64_to_q(n, src, o, qbits, (int*)ints.p, out.p, st);
     int hE[2];
     MB_CUDA(cudaMemcpyAsync(hE, ints.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
     MB_CUDA(cudaStreamSynchronize(st));
@@ -630,10 +646,9 @@ struct QKrylov {
   }
 
   void store(const QRef& x, int order, void* dst) {
-    int32_t* iperm = order == MB_ORDER_REFERENCE ? op_iperm(op) : nullptr;
     QBuf e(sizeof(int));
     MB_CUDA(cudaMemcpyAsync(e.p, &x.E, sizeof(int), cudaMemcpyHostToDevice, st));
-    launch_q_to_f64(n, x.p, iperm, (const int*)e.p, dst, st);
+    q_to_order(op, x.p, order, (const int*)e.p, dst, st);
     MB_CUDA(cudaStreamSynchronize(st));
   }
 };
@@ -777,9 +792,9 @@ int mb_q64_from_f64(mb_op_t op, const void* x_dev, int order, void* xq_dev, int*
     MB_REQUIRE(order == MB_ORDER_REFERENCE || order == MB_ORDER_TENSOR, MB_ERR_INVALID_ARG,
                "bad order");
     cudaStream_t st = (cudaStream_t)stream;
-    int32_t* perm = order == MB_ORDER_REFERENCE ? op_perm(op) : nullptr;
+    const RowOrder o = order == MB_ORDER_REFERENCE ? op_row_order(op) : RowOrder{};
     QBuf ints(4 * sizeof(int));
-    launch_f64_to_q(op->dim, x_dev, perm, op->q_qbits, (int*)ints.p, xq_dev, st);
+    launch_f64_to_q(op->dim, x_dev, o, op->q_qbits, (int*)ints.p, xq_dev, st);
     int h[2];
     MB_CUDA(cudaMemcpyAsync(h, ints.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
     MB_CUDA(cudaStreamSynchronize(st));
@@ -794,10 +809,9 @@ int mb_q64_to_f64(mb_op_t op, const void* xq_dev, int exponent, int order, void*
     MB_REQUIRE(order == MB_ORDER_REFERENCE || order == MB_ORDER_TENSOR, MB_ERR_INVALID_ARG,
                "bad order");
     cudaStream_t st = (cudaStream_t)stream;
-    int32_t* iperm = order == MB_ORDER_REFERENCE ? op_iperm(op) : nullptr;
     QBuf e(sizeof(int));
     MB_CUDA(cudaMemcpyAsync(e.p, &exponent, sizeof(int), cudaMemcpyHostToDevice, st));
-    launch_q_to_f64(op->dim, xq_dev, iperm, (const int*)e.p, x_dev, st);
+    q_to_order(op, xq_dev, order, (const int*)e.p, x_dev, st);
     MB_CUDA(cudaStreamSynchronize(st));
   });
 }
