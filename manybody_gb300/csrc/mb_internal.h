@@ -298,6 +298,9 @@ struct SlicedTable {
 SlicedTable sliced_table(const HopTable& t, int64_t D);
 // 1 + ceil(log2(terms)), at least 6: the bits an integer sum (mb_isum.h) of that
 // many terms keeps free above its largest term, sign included.
+// Up to kISumBaseMax a sum keeps its largest term's whole significand (512
+// terms, one bit to spare).
+constexpr int kISumBaseMax = 10;
 inline int isum_base(int64_t terms) {
   int b = 6;
   while ((int64_t(1) << (b - 1)) < terms) ++b;
@@ -381,7 +384,8 @@ struct OpView {
   int dn_max_words;
   int max_up_list;
   // headroom bits of the complex128 applies' integer hop sums (isum_base of the
-  // most hops one state can have)
+  // most hops one state can have; of a lane's entries of a sparse matrix's row,
+  // 0: sums in FP64)
   int isum_base;
   // Operators made from a sparse matrix instead of a lattice (mb_op_create_csr):
   // CSR on the device, values complex128 (and complex64 copies for MB_PREC_F32).

@@ -493,18 +493,23 @@ static void apply_dots(const OpView& v, const void* x, void* y, double scale, do
 }
 
 // ---------------------------------------------------------------------------
-// The same contract for an operator given as a sparse matrix (CSR): one warp
-// per row (rows grid-strided over a fixed grid), lanes over the row's
+// The same contract for an operator given as a sparse matrix (CSR): a few
+// lanes per row (rows grid-strided over a fixed grid), lanes over the row's
 // entries, complex products, a fixed-order shuffle sum, then the affine
 // epilogue and the fused dots in lane 0.  Deterministic.  In the signed-
-// column form (no values) every entry is +-off and the diagonal comes apart.
+// column form (no values) every entry is +-off and the diagonal comes apart;
+// complex128 sums it on the integer pipes (mb_isum.h), a lane's part of a row a
+// sum, the lanes' sums in FP64: 4x4 5+5, K = (0,0) (200 entries a row) 1.17 ->
+// 0.70 ms, 6+6 4.47 -> 2.78 ms, 12 sites 6+6 70 -> 49 us.  What is left is the
+// gathers of x, one 32-byte sector for each 16-byte element (11 TB/s from L2);
+// the Q64 kernel, with cheaper sums, takes as long.
 // ---------------------------------------------------------------------------
 constexpr int kCsrThreads = 256;
 // Lanes per CSR row: a row's partial sums meet in a log2(lanes)-step shuffle
 // reduction, which on this GPU's slow FP64 pipe cost as much as the row's own
 // adds at 32 lanes.  Measured at 4x4 6+6, K = (0,0) (~210 entries a row):
-// complex128 10.85 / 6.72 / 5.11 / 4.47 ms at 32 / 16 / 8 / 4 lanes,
-// complex64 2.95 / 2.32 / 2.02 / 2.07 ms.
+// complex128 3.54 / 2.97 / 2.78 ms at 16 / 8 / 4 lanes (with FP64 sums 6.72 /
+// 5.11 / 4.47), complex64 2.95 / 2.32 / 2.02 / 2.07 ms at 32 / 16 / 8 / 4.
 template <typename T> constexpr int csr_lanes() { return sizeof(T) == 8 ? 4 : 8; }
 
 // v with its sign flipped when bit 31 of e is set
@@ -520,8 +525,9 @@ __global__ void __launch_bounds__(kCsrThreads)
 k_csr_apply(int64_t n, const int64_t* __restrict__ rp, const int32_t* __restrict__ ci,
             const typename C2<T>::type* __restrict__ val, const double* __restrict__ diag, T off,
             const typename C2<T>::type* __restrict__ x, typename C2<T>::type* y, T scale, T shift,
-            T beta, const typename C2<T>::type* z, double* __restrict__ partials) {
+            T beta, const typename C2<T>::type* z, double* __restrict__ partials, int base) {
   using V2 = typename C2<T>::type;
+  const ISumForm form(base);
   // LPR lanes per row, 32 / LPR rows per warp; the warp steps through its rows
   // together (the shuffles need every lane), groups past the last row idle
   constexpr int RPW = 32 / LPR;
@@ -542,31 +548,54 @@ k_csr_apply(int64_t n, const int64_t* __restrict__ rp, const int32_t* __restrict
         ai = fma(a.x, b.y, fma(a.y, b.x, ai));
       }
     } else {  // signed columns: entries +-1 (times off below), diagonal apart
-      // the sign goes onto the sign bit, so no lane branches per entry; for
-      // complex64 two independent sums (even / odd strides) halve the add
-      // chains (measured at 4x4 6+6, K=0, 32 lanes a row: 3.19 -> 2.81 ms),
-      // for complex128 one (9.1 ms, against 12.9 ms with two)
-      T br = T(0), bi = T(0);
-      const int64_t k1 = rp[row + 1];
-      int64_t k = rp[row] + lane;
-#pragma unroll 4
-      for (; sizeof(T) == 4 && k + LPR < k1; k += 2 * LPR) {
-        const uint32_t e0 = (uint32_t)__ldg(&ci[k]), e1 = (uint32_t)__ldg(&ci[k + LPR]);
-        const V2 b0 = __ldg(&x[e0 & 0x7FFFFFFFu]), b1 = __ldg(&x[e1 & 0x7FFFFFFFu]);
-        ar += flip_sign(b0.x, e0);
-        ai += flip_sign(b0.y, e0);
-        br += flip_sign(b1.x, e1);
-        bi += flip_sign(b1.y, e1);
+      const int64_t k0 = rp[row] + lane, k1 = rp[row + 1];
+      bool fp = sizeof(T) == 4 || base == 0;
+      if constexpr (sizeof(T) == 8) {
+        if (!fp) {  // on the integer pipes; a missing entry is a zero
+          ISum2 sum;
+          for (int64_t k = k0; k < k1; k += 4 * LPR) {
+            uint32_t e[4];
+            V2 b[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+              e[u] = k + u * LPR < k1 ? (uint32_t)__ldg(&ci[k + u * LPR]) : 0x7FFFFFFFu;
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+              b[u] = k + u * LPR < k1 ? __ldg(&x[e[u] & 0x7FFFFFFFu]) : make_double2(0.0, 0.0);
+            sum.add<4>(form, b, e);
+          }
+          const double2 v2 = sum.value(form);
+          ar = v2.x;
+          ai = v2.y;
+          fp = sum.odd();
+          if (fp) ar = ai = T(0);
+        }
       }
+      if (fp) {
+        // the sign goes onto the sign bit, so no lane branches per entry; for
+        // complex64 two independent sums (even / odd strides) halve the add
+        // chains (measured at 4x4 6+6, K=0, 32 lanes a row: 3.19 -> 2.81 ms)
+        T br = T(0), bi = T(0);
+        int64_t k = k0;
 #pragma unroll 4
-      for (; k < k1; k += LPR) {
-        const uint32_t e0 = (uint32_t)__ldg(&ci[k]);
-        const V2 b0 = __ldg(&x[e0 & 0x7FFFFFFFu]);
-        ar += flip_sign(b0.x, e0);
-        ai += flip_sign(b0.y, e0);
+        for (; sizeof(T) == 4 && k + LPR < k1; k += 2 * LPR) {
+          const uint32_t e0 = (uint32_t)__ldg(&ci[k]), e1 = (uint32_t)__ldg(&ci[k + LPR]);
+          const V2 b0 = __ldg(&x[e0 & 0x7FFFFFFFu]), b1 = __ldg(&x[e1 & 0x7FFFFFFFu]);
+          ar += flip_sign(b0.x, e0);
+          ai += flip_sign(b0.y, e0);
+          br += flip_sign(b1.x, e1);
+          bi += flip_sign(b1.y, e1);
+        }
+#pragma unroll 4
+        for (; k < k1; k += LPR) {
+          const uint32_t e0 = (uint32_t)__ldg(&ci[k]);
+          const V2 b0 = __ldg(&x[e0 & 0x7FFFFFFFu]);
+          ar += flip_sign(b0.x, e0);
+          ai += flip_sign(b0.y, e0);
+        }
+        ar += br;
+        ai += bi;
       }
-      ar += br;
-      ai += bi;
     }
 #pragma unroll
     for (int o = LPR / 2; o > 0; o >>= 1) {
@@ -623,7 +652,7 @@ static void csr_apply_l(const OpView& v, const void* x, void* y, double scale, d
   k_csr_apply<T, DOTS, LPR><<<csr_grid(v, sizeof(T) == 4 ? MB_PREC_F32 : MB_PREC_F64),
                               kCsrThreads, 0, st>>>(
       v.dim, v.csr_row, v.csr_col, val, v.csr_diag, (T)v.csr_off, (const V2*)x, (V2*)y,
-      (T)scale, (T)shift, (T)beta, (const V2*)z, partials);
+      (T)scale, (T)shift, (T)beta, (const V2*)z, partials, v.isum_base);
   MB_CUDA(cudaGetLastError());
 }
 

@@ -88,3 +88,25 @@ def test_non_finite_terms_reach_their_rows_only(mb, cuda, dims, nu, nd, bad):
     x[at] = complex(0, vector("uniform", basis.size(), np.random.default_rng(1))[at].imag)
     im, size = exact(m, x.imag)
     assert np.all(np.abs(y.imag - im) <= eps * size)
+
+
+@pytest.mark.parametrize("kind", ["uniform", "wide", "real", "sparse", "extreme", "growing"])
+@pytest.mark.parametrize("dims,n,k,lanes", [((6,), 4, (2,), 4), ((3, 3), 6, (1, 0), 4),
+                                            ((4, 3), 7, (1, 2), 8), ((4, 4), 6, (0, 1), 32)])
+def test_integer_row_sums_of_a_momentum_sector(mb, cuda, dims, n, k, lanes, kind):
+    torch = cuda
+    L, sz = int(np.prod(dims)), n % 2
+    basis = mb.FermionBasis.with_fixed_particle_number_spin_momentum(L, n, sz, dims, k)
+    model = mb.HubbardModelMomentum(1.0, 3.0, dims)
+    m = mb.compute_matrix_elements(basis, model)
+    op = mb.GpuHubbardOperator(basis, model, mb.PREC_F64)
+    op.set_apply_shape(csr_lanes=lanes)
+    x = vector(kind, basis.size(), np.random.default_rng(n))
+    y = op.apply(torch.from_numpy(x).cuda()).cpu().numpy()
+    # as above; the lanes' sums, the off-diagonal factor and the shift round too,
+    # and the diagonal is summed in another order than the exported one's
+    eps = (int(np.diff(m.row_ptr).max()) + 16) * 2.0 ** -53
+    for got, part in ((y.real, x.real), (y.imag, x.imag)):
+        want, size = exact(m, part)
+        off = np.abs(got.astype(np.longdouble) - want)
+        assert np.all(off <= eps * size + 16 * 2.0 ** -1074), float(np.max(off / np.maximum(size, 1e-300)))
