@@ -319,6 +319,26 @@ SlicedTable16 sliced_table16(const SlicedTable& s, int64_t D);
 // accumulates for k doubly occupied sites (matrix_elements.h:85-96).
 std::vector<double> u_fold_table(double u, bool has_u, int L);
 
+// One step of a recurrence that stays on the device: an apply or a vector update
+// whose fused dot products are summed by the last of its blocks to finish (in
+// block order, so the sums do not depend on which one that is), and, in a
+// Lanczos step (alpha set), whose coefficients come from the sums of the steps
+// before it.  The vectors are u_j = s_j v_j, s_j = beta_(j-1) (s_0 = 1):
+//   apply   w = (scale / s_j) H u_j - (s_j / s_(j-1)) u_(j-1),  alpha_j = Re<u_j, w> / s_j
+//   update  w -= (alpha_j / s_j) u_j,                           beta_j = ||w||
+// so a step is two launches with no normalisation pass, no reduction launch
+// and no wait of the host.
+struct KrylovStep {
+  unsigned* ticket = nullptr;     // 0 between launches; nullptr: partials only
+  int blocks = 0;                 // blocks of the launch (of all launches of a block-diagonal apply)
+  const double* part = nullptr;   // their partials, three sums each
+  double* dots = nullptr;         // the three sums, unless a Lanczos step:
+  double* alpha = nullptr;
+  double* beta = nullptr;
+  int j = 0;
+  double scale = 0.0;
+};
+
 // dot_mode / dots of an apply whose result goes to reference order, y[out_perm[i]]
 // (no dots; a Q64 apply writes complex128).  The scattered stores ride along in
 // a kernel that is bound elsewhere, where a move of its own reads and writes the
@@ -406,6 +426,7 @@ struct OpView {
   int n_blocks;
   const OpView* sub;
   const int64_t* sub_off;
+  KrylovStep step;  // see there
   // of launches with kRefOut: tensor -> reference index
   const int32_t* out_perm;
   double t;
@@ -599,6 +620,11 @@ int blas_grid(int64_t n);
 // y = a*x + b*y (complex coefficients); dots of the result if dot_mode.
 void launch_axpby(int precision, int64_t n, double ar, double ai, const void* x, double br,
                   double bi, void* y, double* partials, int dot_mode, cudaStream_t st);
+// w += c u (c real; a Lanczos step takes its own), <w,w> of the result in comp 1
+void launch_update(int precision, int64_t n, double c, const void* u, void* w, double* partials,
+                   const KrylovStep& step, cudaStream_t st);
+// partials for <x,x> (comp 1)
+void launch_norm2(int precision, int64_t n, const void* x, double* partials, cudaStream_t st);
 // partials for Re<x,y> (comp 0), Im<x,y> (comp 1), <y,y> (comp 2).
 void launch_dot(int precision, int64_t n, const void* x, const void* y, double* partials,
                 cudaStream_t st);

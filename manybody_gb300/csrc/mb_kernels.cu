@@ -47,13 +47,17 @@ template <> struct DotAcc<float> {
   __device__ double value() const { return (double)hi + (double)lo; }
 };
 
-// Block reduction of NC doubles; thread 0 writes partials[blockIdx.x*NC + k].
-template <int NC>
-__device__ void block_reduce_store(double (&v)[NC], double* partials) {
-  __shared__ double red[32][NC > 0 ? NC : 1];
+// Block reduction of three doubles, those of MASK's bits (the others count as
+// zero: a warp's shuffle tree is five FP64 adds, 17 cycles of an SM each, and
+// four blocks of eight warps share one pipe); thread 0 writes
+// partials[blockIdx.x*3 + k].
+template <int MASK>
+__device__ void block_reduce_store(double (&v)[3], double* partials) {
+  __shared__ double red[32][3];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-  for (int k = 0; k < NC; ++k) {
+  for (int k = 0; k < 3; ++k) {
+    if (!(MASK >> k & 1)) continue;
     double a = v[k];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
@@ -61,16 +65,83 @@ __device__ void block_reduce_store(double (&v)[NC], double* partials) {
   }
   __syncthreads();
   if (lane == 0)
-    for (int k = 0; k < NC; ++k) red[warp][k] = v[k];
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+      if (MASK >> k & 1) red[warp][k] = v[k];
   __syncthreads();
   if (warp == 0) {
     const int nw = (blockDim.x + 31) >> 5;
-    for (int k = 0; k < NC; ++k) {
-      double a = lane < nw ? red[lane][k] : 0.0;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      double a = 0.0;
+      if (MASK >> k & 1) {
+        a = lane < nw ? red[lane][k] : 0.0;
+        for (int o = 16; o > 0; o >>= 1)
+          if (o < nw) a += __shfl_down_sync(0xffffffffu, a, o);
+      }
+      if (lane == 0) partials[(size_t)blockIdx.x * 3 + k] = a;
+    }
+  }
+}
+
+// A Lanczos step's vector scale s_j.
+__device__ __forceinline__ double krylov_scale(const KrylovStep& s, int j) {
+  return j > 0 ? __ldcg(s.beta + j - 1) : 1.0;
+}
+
+// (scale, factor of z) of a Lanczos step's apply
+__device__ __forceinline__ void step_coefs(const KrylovStep& s, double (&c)[2]) {
+  const double sj = krylov_scale(s, s.j);
+  c[0] = s.scale / sj;
+  c[1] = s.j > 0 ? -sj / krylov_scale(s, s.j - 1) : 0.0;
+}
+
+// The last block of a launch to get here sums every block's partials (thread 0
+// of each wrote its own, see block_reduce_store), those of MASK's bits, and
+// stores the result.  UPDATE: of a vector update, else of an apply.
+template <bool UPDATE, int MASK>
+__device__ void finish_step(const KrylovStep& s) {
+  __shared__ bool last;
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(s.ticket, 1u) + 1u == (unsigned)s.blocks;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  __shared__ double red[32][3];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    if (!(MASK >> k & 1)) continue;
+    double a = 0.0;
+    if (32 * warp < s.blocks) {
+      for (int b = threadIdx.x; b < s.blocks; b += blockDim.x)
+        a += __ldcg(s.part + 3 * (size_t)b + k);
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
-      if (lane == 0) partials[(size_t)blockIdx.x * NC + k] = a;
     }
+    if (lane == 0) red[warp][k] = a;
+  }
+  __syncthreads();
+  if (warp != 0) return;
+  double sum[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    if (!(MASK >> k & 1)) continue;
+    sum[k] = lane < nw ? red[lane][k] : 0.0;
+    for (int o = 16; o > 0; o >>= 1)
+      if (o < nw) sum[k] += __shfl_down_sync(0xffffffffu, sum[k], o);
+  }
+  if (lane == 0) {
+    if (!s.alpha) {
+      for (int k = 0; k < 3; ++k) s.dots[k] = sum[k];
+    } else if (UPDATE) {
+      s.beta[s.j] = sqrt(sum[1]);
+    } else {
+      s.alpha[s.j] = sum[0] / krylov_scale(s, s.j);
+    }
+    *s.ticket = 0;
   }
 }
 
@@ -167,7 +238,7 @@ __device__ __forceinline__ void apply_rows(
     const OpView& v, const typename C2<T>::type* __restrict__ x, typename C2<T>::type* y,
     T hop_coef, T dscale, T shift, T beta, const typename C2<T>::type* z,
     const T* __restrict__ ufold, const T* __restrict__ self_up, const T* __restrict__ self_dn,
-    double* __restrict__ partials) {
+    double* __restrict__ partials, const volatile T* s_coef = nullptr) {
   using V2 = typename C2<T>::type;
   constexpr int kShift = sizeof(V2) == 16 ? 4 : 3;
   constexpr bool kInt = sizeof(T) == 8;  // hop sums on the integer pipes (mb_isum.h)
@@ -345,15 +416,19 @@ __device__ __forceinline__ void apply_rows(
       const V2 xv = STAGED && !kInt ? reinterpret_cast<const V2*>(smem)[c] : xrow[c];
       T dv = ufold[__popc(um & v.dn_mask[c])] + su;
       if (self_dn) dv += self_dn[c];
-      const T ds = dscale * (dv - shift);
+      // (coefficients from shared memory, where given, only now: registers)
+      const bool given = (DOTS & 1) && s_coef;
+      const T hc = given ? s_coef[0] : hop_coef;
+      const T ds = (given ? s_coef[1] : dscale) * (dv - shift);
       V2 out;
-      out.x = fma(hop_coef, ar, ds * xv.x);
-      out.y = fma(hop_coef, ai, ds * xv.y);
+      out.x = fma(hc, ar, ds * xv.x);
+      out.y = fma(hc, ai, ds * xv.y);
       const int64_t idx = r * Dd + c;
       if (z) {
         const V2 zv = z[idx];
-        out.x = fma(beta, zv.x, out.x);
-        out.y = fma(beta, zv.y, out.y);
+        const T be = given ? s_coef[2] : beta;
+        out.x = fma(be, zv.x, out.x);
+        out.y = fma(be, zv.y, out.y);
       }
       y[DOTS & kRefOut ? (int64_t)__ldcs(v.out_perm + idx) : idx] = out;
       if (DOTS & 1) { a_xy.add_prod(xv.x, out.x); a_xy.add_prod(xv.y, out.y); }
@@ -363,7 +438,7 @@ __device__ __forceinline__ void apply_rows(
   }
   if (DOTS & 7) {
     double vals[3] = {a_xy.value(), a_yy.value(), a_xx.value()};
-    block_reduce_store<3>(vals, partials);
+    block_reduce_store<DOTS & 7>(vals, partials);
   }
 }
 
@@ -373,8 +448,17 @@ k_apply(OpView v, const typename C2<T>::type* __restrict__ x, typename C2<T>::ty
         T hop_coef, T dscale, T shift, T beta, const typename C2<T>::type* z,
         const T* __restrict__ ufold, const T* __restrict__ self_up, const T* __restrict__ self_dn,
         double* __restrict__ partials) {
+  __shared__ T s_coef[3];  // hop_coef, dscale, beta: read past apply_rows' barriers
+  if ((DOTS & 1) && threadIdx.x == 0) {
+    double c[2] = {0.0, 0.0};
+    if (v.step.alpha) step_coefs(v.step, c);
+    s_coef[0] = v.step.alpha ? (T)(-v.t * c[0]) : hop_coef;
+    s_coef[1] = v.step.alpha ? (T)c[0] : dscale;
+    s_coef[2] = v.step.alpha ? (T)c[1] : beta;
+  }
   apply_rows<T, STAGED, DOTS>(v, x, y, hop_coef, dscale, shift, beta, z, ufold, self_up, self_dn,
-                              partials);
+                              partials, DOTS & 1 ? s_coef : nullptr);
+  if ((DOTS & 7) && v.step.ticket) finish_step<false, DOTS & 7>(v.step);
 }
 
 // One engine step of a large slot through the fused complex64 apply: the
@@ -423,7 +507,7 @@ static size_t apply_smem(const OpView& v, int precision, bool staged) {
 }
 
 static bool apply_staged(const OpView& v, int precision) {
-  return apply_smem(v, precision, true) + 1024 <= (size_t)max_smem_optin();
+  return apply_smem(v, precision, true) + 3072 <= (size_t)max_smem_optin();
 }
 
 // Threads of an apply's CTAs and how many of them an SM holds: together
@@ -440,7 +524,7 @@ struct ApplyCtas {
 };
 static ApplyCtas apply_ctas(const OpView& v, int precision) {
   const int total = kApplyThreads * (precision == MB_PREC_F32 ? kApplyCtasPerSm<float> : 1);
-  const size_t row = apply_smem(v, precision, apply_staged(v, precision)) + 2048;
+  const size_t row = apply_smem(v, precision, apply_staged(v, precision)) + 3072;
   const size_t sm = (size_t)max_smem_optin() + 1024;
   int threads = precision == MB_PREC_F32 && v.Dd > 32 * 32 ? 512 : 256;
   while (threads < kApplyThreads && (size_t)(total / threads) * row > sm) threads *= 2;
@@ -525,9 +609,17 @@ __global__ void __launch_bounds__(kCsrThreads)
 k_csr_apply(int64_t n, const int64_t* __restrict__ rp, const int32_t* __restrict__ ci,
             const typename C2<T>::type* __restrict__ val, const double* __restrict__ diag, T off,
             const typename C2<T>::type* __restrict__ x, typename C2<T>::type* y, T scale, T shift,
-            T beta, const typename C2<T>::type* z, double* __restrict__ partials, int base) {
+            T beta, const typename C2<T>::type* z, double* __restrict__ partials, int base,
+            KrylovStep step) {
   using V2 = typename C2<T>::type;
   const ISumForm form(base);
+  if ((DOTS & 1) && step.alpha) {
+    __shared__ double c[2];
+    if (threadIdx.x == 0) step_coefs(step, c);
+    __syncthreads();
+    scale = (T)c[0];
+    beta = (T)c[1];
+  }
   // LPR lanes per row, 32 / LPR rows per warp; the warp steps through its rows
   // together (the shuffles need every lane), groups past the last row idle
   constexpr int RPW = 32 / LPR;
@@ -625,7 +717,8 @@ k_csr_apply(int64_t n, const int64_t* __restrict__ rp, const int32_t* __restrict
   }
   if (DOTS) {
     double vals[3] = {a_xy.value(), a_yy.value(), a_xx.value()};
-    block_reduce_store<3>(vals, partials);
+    block_reduce_store<DOTS & 7>(vals, partials);
+    if (step.ticket) finish_step<false, DOTS & 7>(step);
   }
 }
 
@@ -652,7 +745,7 @@ static void csr_apply_l(const OpView& v, const void* x, void* y, double scale, d
   k_csr_apply<T, DOTS, LPR><<<csr_grid(v, sizeof(T) == 4 ? MB_PREC_F32 : MB_PREC_F64),
                               kCsrThreads, 0, st>>>(
       v.dim, v.csr_row, v.csr_col, val, v.csr_diag, (T)v.csr_off, (const V2*)x, (V2*)y,
-      (T)scale, (T)shift, (T)beta, (const V2*)z, partials, v.isum_base);
+      (T)scale, (T)shift, (T)beta, (const V2*)z, partials, v.isum_base, v.step);
   MB_CUDA(cudaGetLastError());
 }
 
@@ -689,7 +782,9 @@ void launch_apply(const OpView& v, int precision, const void* x, void* y, double
     int64_t first = 0;
     for (int b = 0; b < v.n_blocks; ++b) {
       const size_t off = es * (size_t)v.sub_off[b];
-      launch_apply(v.sub[b], precision, (const char*)x + off, (char*)y + off, scale, shift, beta,
+      OpView sub = v.sub[b];
+      sub.step = v.step;
+      launch_apply(sub, precision, (const char*)x + off, (char*)y + off, scale, shift, beta,
                    z ? (const char*)z + off : nullptr, partials ? partials + 3 * first : nullptr,
                    dot_mode, st);
       first += apply_grid(v.sub[b], precision);
@@ -752,8 +847,9 @@ int blas_grid(int64_t n) {
   return (int)(g > 0 ? g : 1);
 }
 
-// y = a*x + b*y, complex a, b; dot_mode bit1: <y,y> of the result.
-template <typename T, int DOTS>
+// y = a*x + b*y, complex a, b (REAL: ai = bi = 0, half the products, on the
+// slow FP64 pipe the longer part of a pass); dot_mode bit1: <y,y> of the result.
+template <typename T, int DOTS, bool REAL>
 __global__ void k_axpby(int64_t n, T ar, T ai, const typename C2<T>::type* __restrict__ x, T br,
                         T bi, typename C2<T>::type* __restrict__ y, double* __restrict__ partials) {
   using V2 = typename C2<T>::type;
@@ -763,27 +859,110 @@ __global__ void k_axpby(int64_t n, T ar, T ai, const typename C2<T>::type* __res
     const V2 xv = x ? x[i] : V2{T(0), T(0)};
     const V2 yv = (br != T(0) || bi != T(0)) ? y[i] : V2{T(0), T(0)};
     V2 o;
-    o.x = ar * xv.x - ai * xv.y + br * yv.x - bi * yv.y;
-    o.y = ar * xv.y + ai * xv.x + br * yv.y + bi * yv.x;
+    if (REAL) {
+      o.x = fma(ar, xv.x, br * yv.x);
+      o.y = fma(ar, xv.y, br * yv.y);
+    } else {
+      o.x = ar * xv.x - ai * xv.y + br * yv.x - bi * yv.y;
+      o.y = ar * xv.y + ai * xv.x + br * yv.y + bi * yv.x;
+    }
     y[i] = o;
     if (DOTS & 2) { acc.add_prod(o.x, o.x); acc.add_prod(o.y, o.y); }
   }
   if (DOTS) {
     double vals[3] = {0.0, acc.value(), 0.0};
-    block_reduce_store<3>(vals, partials);
+    block_reduce_store<2>(vals, partials);
   }
+}
+
+template <typename T, bool REAL>
+static void axpby_t(int64_t n, double ar, double ai, const void* x, double br, double bi, void* y,
+                    double* partials, int dot_mode, cudaStream_t st) {
+  using V2 = typename C2<T>::type;
+  const int g = blas_grid(n);
+  if (dot_mode)
+    k_axpby<T, 2, REAL><<<g, kBlasThreads, 0, st>>>(n, (T)ar, (T)ai, (const V2*)x, (T)br, (T)bi,
+                                                    (V2*)y, partials);
+  else
+    k_axpby<T, 0, REAL><<<g, kBlasThreads, 0, st>>>(n, (T)ar, (T)ai, (const V2*)x, (T)br, (T)bi,
+                                                    (V2*)y, partials);
+  MB_CUDA(cudaGetLastError());
 }
 
 void launch_axpby(int precision, int64_t n, double ar, double ai, const void* x, double br,
                   double bi, void* y, double* partials, int dot_mode, cudaStream_t st) {
-  const int g = blas_grid(n);
+  const bool real = ai == 0.0 && bi == 0.0;
   if (precision == MB_PREC_F32) {
-    if (dot_mode) k_axpby<float, 2><<<g, kBlasThreads, 0, st>>>(n, (float)ar, (float)ai, (const float2*)x, (float)br, (float)bi, (float2*)y, partials);
-    else k_axpby<float, 0><<<g, kBlasThreads, 0, st>>>(n, (float)ar, (float)ai, (const float2*)x, (float)br, (float)bi, (float2*)y, partials);
+    if (real) axpby_t<float, true>(n, ar, ai, x, br, bi, y, partials, dot_mode, st);
+    else axpby_t<float, false>(n, ar, ai, x, br, bi, y, partials, dot_mode, st);
   } else {
-    if (dot_mode) k_axpby<double, 2><<<g, kBlasThreads, 0, st>>>(n, ar, ai, (const double2*)x, br, bi, (double2*)y, partials);
-    else k_axpby<double, 0><<<g, kBlasThreads, 0, st>>>(n, ar, ai, (const double2*)x, br, bi, (double2*)y, partials);
+    if (real) axpby_t<double, true>(n, ar, ai, x, br, bi, y, partials, dot_mode, st);
+    else axpby_t<double, false>(n, ar, ai, x, br, bi, y, partials, dot_mode, st);
   }
+}
+
+// w += c u with <w,w> of the result; a Lanczos step's c from its own scalars.
+// NORM: <w,w> alone (u unused).  Four elements a thread in flight.
+template <typename T, bool NORM>
+__global__ void __launch_bounds__(kBlasThreads)
+k_update(int64_t n, T c, const typename C2<T>::type* __restrict__ u,
+         typename C2<T>::type* __restrict__ w, double* __restrict__ partials, KrylovStep step) {
+  using V2 = typename C2<T>::type;
+  if (!NORM && step.alpha) {
+    __shared__ double s_c;
+    if (threadIdx.x == 0) s_c = -__ldcg(step.alpha + step.j) / krylov_scale(step, step.j);
+    __syncthreads();
+    c = (T)s_c;
+  }
+  DotAcc<T> acc;
+  constexpr int U = 4;
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t i0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i0 < n; i0 += U * stride) {
+    V2 a[U], b[U];
+#pragma unroll
+    for (int k = 0; k < U; ++k)
+      if (i0 + k * stride < n) {
+        if (!NORM) a[k] = u[i0 + k * stride];
+        b[k] = w[i0 + k * stride];
+      }
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+      if (i0 + k * stride >= n) break;
+      V2 o = b[k];
+      if (!NORM) {
+        o.x = fma(c, a[k].x, o.x);
+        o.y = fma(c, a[k].y, o.y);
+        w[i0 + k * stride] = o;
+      }
+      acc.add_prod(o.x, o.x);
+      acc.add_prod(o.y, o.y);
+    }
+  }
+  double vals[3] = {0.0, acc.value(), 0.0};
+  block_reduce_store<2>(vals, partials);
+  if (!NORM && step.ticket) finish_step<true, 2>(step);
+}
+
+void launch_update(int precision, int64_t n, double c, const void* u, void* w, double* partials,
+                   const KrylovStep& step, cudaStream_t st) {
+  const int g = blas_grid(n);
+  if (precision == MB_PREC_F32)
+    k_update<float, false><<<g, kBlasThreads, 0, st>>>(n, (float)c, (const float2*)u, (float2*)w,
+                                                       partials, step);
+  else
+    k_update<double, false><<<g, kBlasThreads, 0, st>>>(n, c, (const double2*)u, (double2*)w,
+                                                        partials, step);
+  MB_CUDA(cudaGetLastError());
+}
+
+void launch_norm2(int precision, int64_t n, const void* x, double* partials, cudaStream_t st) {
+  const int g = blas_grid(n);
+  if (precision == MB_PREC_F32)
+    k_update<float, true><<<g, kBlasThreads, 0, st>>>(n, 0.f, nullptr, (float2*)x, partials,
+                                                      KrylovStep{});
+  else
+    k_update<double, true><<<g, kBlasThreads, 0, st>>>(n, 0.0, nullptr, (double2*)x, partials,
+                                                       KrylovStep{});
   MB_CUDA(cudaGetLastError());
 }
 
@@ -804,7 +983,7 @@ __global__ void k_dot(int64_t n, const typename C2<T>::type* __restrict__ x,
     yy.add_prod(b.y, b.y);
   }
   double vals[3] = {re.value(), im.value(), yy.value()};
-  block_reduce_store<3>(vals, partials);
+  block_reduce_store<7>(vals, partials);
 }
 
 void launch_dot(int precision, int64_t n, const void* x, const void* y, double* partials,
@@ -1007,7 +1186,7 @@ k_multi_axpy(int64_t n, const typename C2<TV>::type* __restrict__ V, int64_t ld,
     ww.add_prod((double)o.y, (double)o.y);
   }
   double vals[3] = {0.0, ww.value(), 0.0};
-  block_reduce_store<3>(vals, partials);
+  block_reduce_store<2>(vals, partials);
 }
 
 void launch_multi_axpy(int vprec, int wprec, int64_t n, const void* V, int64_t ld, int m,

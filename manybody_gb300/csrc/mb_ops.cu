@@ -771,22 +771,65 @@ struct Krylov {
   int64_t n;
   int prec;
   size_t vb;
-  DevBuf v_prev, v_curr, w, basis, coef;
+  DevBuf rot[3];  // rotating vectors, each made on first use
+  DevBuf basis, coef, basis_part;
   int basis_prec = MB_PREC_F64;
   int64_t basis_cap = 0;
   Reducer red;
   int grid_apply, grid_blas;
+  // alpha_j, beta_j of the plain recurrence on the device, and the blocks'
+  // ticket (KrylovStep)
+  DevBuf scalars;
+  int64_t scalar_cap = 0;
 
   Krylov(mb_op_s* o, cudaStream_t s)
       : op(o), st(s), n(o->dim), prec(o->precision), vb(elem_bytes(o->precision) * (size_t)o->dim),
-        v_prev(vb), v_curr(vb), w(vb),
-        red(std::max(std::max(apply_grid(o->view, o->precision), blas_grid(o->dim)), 1024) , 2 * 1024 + 8),
+        red(std::max(apply_grid(o->view, o->precision), blas_grid(o->dim)), 3),
         grid_apply(apply_grid(o->view, o->precision)), grid_blas(blas_grid(o->dim)) {}
 
   double norm_of(const void* x) {
-    launch_dot(prec, n, x, x, red.p(), st);
+    launch_norm2(prec, n, x, red.p(), st);
     const double* h = red.fetch(grid_blas, 3, st);
-    return std::sqrt(h[2]);
+    return std::sqrt(h[1]);
+  }
+
+  void* rot_vec(int64_t j) {
+    DevBuf& b = rot[j % 3];
+    if (!b.p) b = DevBuf(vb);
+    return b.p;
+  }
+
+  // The device scalars of a run of up to k steps.
+  KrylovStep scalars_for(int64_t k, double scale) {
+    if (scalar_cap < k) {
+      scalars = DevBuf(sizeof(double) * (2 * (size_t)k + 1));
+      scalar_cap = k;
+    }
+    KrylovStep s;
+    s.alpha = (double*)scalars.p;
+    s.beta = s.alpha + scalar_cap;
+    s.ticket = (unsigned*)(s.beta + scalar_cap);
+    s.part = red.p();
+    s.scale = scale;
+    MB_CUDA(cudaMemsetAsync(s.ticket, 0, sizeof(unsigned), st));
+    return s;
+  }
+
+  // u_j of the plain recurrence: a kept column, else a rotating vector.
+  void* plain_vec(int64_t j, bool keep_vectors) {
+    if (keep_vectors && kept == j && keep_room(j)) kept = j + 1;
+    return keep_vectors && j < kept ? keep_col(j) : rot_vec(j);
+  }
+
+  // Step j of the plain recurrence from u_(j-1), u_j to u_(j+1) (KrylovStep).
+  void plain_step(KrylovStep s, int64_t j, const void* prev, const void* cur, void* next) {
+    s.j = (int)j;
+    s.blocks = grid_apply;
+    OpView v = op->view;
+    v.step = s;
+    launch_apply(v, prec, cur, next, 0.0, 0.0, 0.0, j > 0 ? prev : nullptr, red.p(), 1, st);
+    s.blocks = grid_blas;
+    launch_update(prec, n, 0.0, cur, next, red.p(), s, st);
   }
 
   void reserve_basis(int64_t k, int want_prec) {
@@ -802,6 +845,7 @@ struct Krylov {
     basis = DevBuf(need);
     basis_prec = p;
     basis_cap = k;
+    basis_part = DevBuf(sizeof(double) * 2 * (size_t)k * (size_t)multi_dot_grid(n));
     coef = DevBuf(sizeof(double) * 2 * (size_t)std::max<int64_t>(k, 1));
   }
 
@@ -810,8 +854,8 @@ struct Krylov {
   }
 
   // Kept Lanczos vectors: a run without re-orthogonalisation that needs its
-  // Ritz vector keeps the vectors pass one applies (u_0, u_1, ..., in chunks
-  // of kKeepChunk) while a tenth of the device memory stays free, and sums
+  // Ritz vector makes the vectors of pass one (u_0, u_1, ..., in chunks of
+  // kKeepChunk) where it keeps them, while a tenth of the device memory stays free, and sums
   // the Ritz vector from them instead of replaying the recurrence; pass two
   // remains for a run whose Ritz vector needs more vectors than it kept.
   static constexpr int64_t kKeepChunk = 16;
@@ -841,14 +885,12 @@ struct Krylov {
     return true;
   }
 
-  // x = sum_(j < m) y_j v_j from the kept vectors, v_j = u_j / s_j (s_j =
-  // beta_(j-1) for pass one's unnormalised FP32 vectors, 1 otherwise).
+  // x = sum_(j < m) y_j v_j from the kept vectors, v_j = u_j / s_j.
   void combine_kept(int64_t m, const std::vector<double>& betas,
                     const std::vector<std::complex<double>>& y, void* x) {
-    const bool fold = prec == MB_PREC_F32;
     std::vector<double> c(2 * (size_t)m);
     for (int64_t j = 0; j < m; ++j) {
-      const double sj = fold && j > 0 ? betas[(size_t)j - 1] : 1.0;
+      const double sj = j > 0 ? betas[(size_t)j - 1] : 1.0;
       c[2 * (size_t)j] = -y[(size_t)j].real() / sj;  // multi_axpy subtracts
       c[2 * (size_t)j + 1] = -y[(size_t)j].imag() / sj;
     }
@@ -870,12 +912,12 @@ struct Krylov {
   // below 1/sqrt(2) of its norm, where cancellation can leave components
   // along V.  A Lanczos vector is already nearly orthogonal to V, so one pass
   // is the rule.  Returns ||w||^2 after the last pass.
-  double reorth(int m, double nrm2) {
+  double reorth(int m, double nrm2, void* w) {
     for (int pass = 0; pass < 2; ++pass) {
       const double before = nrm2;
-      launch_multi_dot(basis_prec, prec, n, basis.p, n, m, w.p, red.p(), st);
-      launch_reduce(red.p(), multi_dot_grid(n), 2 * m, (double*)coef.p, st);
-      launch_multi_axpy(basis_prec, prec, n, basis.p, n, m, (const double*)coef.p, w.p, red.p(),
+      launch_multi_dot(basis_prec, prec, n, basis.p, n, m, w, (double*)basis_part.p, st);
+      launch_reduce((const double*)basis_part.p, multi_dot_grid(n), 2 * m, (double*)coef.p, st);
+      launch_multi_axpy(basis_prec, prec, n, basis.p, n, m, (const double*)coef.p, w, red.p(),
                         st);
       nrm2 = red.fetch(grid_blas, 3, st)[1];
       if (nrm2 >= 0.5 * before) break;
@@ -886,84 +928,117 @@ struct Krylov {
   // Pass one from b (tensor order, op precision).  Returns steps taken.
   int64_t pass_one(const void* b, int64_t k, double scale, std::vector<double>& alphas,
                    std::vector<double>& betas, double& b_norm, bool reorth, double conv_tol,
-                   int check_every, std::vector<double>* ritz_trace = nullptr,
-                   bool keep_vectors = false) {
+                   int check_every, bool keep_vectors = false) {
     b_norm = norm_of(b);
     MB_REQUIRE(b_norm > kTol, MB_ERR_ZERO_NORM, "Input vector has zero norm");
     alphas.clear();
     betas.clear();
+    kept = 0;
     if (k == 0) return 0;
-    // v_curr = b / ||b||, v_prev = 0
-    launch_axpby(prec, n, 1.0 / b_norm, 0.0, b, 0.0, 0.0, v_curr.p, nullptr, 0, st);
-    MB_CUDA(cudaMemsetAsync(v_prev.p, 0, vb, st));
+    last_ritz = 0.0;
+    have_ritz = false;
+    const int64_t steps = reorth ? reorth_steps(b, k, scale, alphas, betas, b_norm, conv_tol, check_every)
+                                 : plain_steps(b, k, scale, alphas, betas, b_norm, conv_tol,
+                                               check_every, keep_vectors);
+    if ((int64_t)betas.size() > std::max<int64_t>(steps - 1, 0)) betas.resize((size_t)steps - 1);
+    return steps;
+  }
+
+  // Whether the largest Ritz value moved by at most conv_tol since the last check.
+  double last_ritz = 0.0;
+  bool have_ritz = false;
+  bool settled(const std::vector<double>& alphas, const std::vector<double>& betas, double conv_tol) {
+    std::vector<double> d(alphas), e(betas);
+    e.resize(d.size() - 1);
+    if (!tridiag_eig((int)d.size(), d, e, nullptr)) return false;
+    const double ritz = d.back();
+    if (have_ritz && std::fabs(ritz - last_ritz) <= conv_tol * std::fabs(ritz)) return true;
+    last_ritz = ritz;
+    have_ritz = true;
+    return false;
+  }
+
+  // The recurrence (lanczos.h:25-36,113-121) without re-orthogonalisation: the
+  // steps between two looks at the scalars are queued at once.
+  static constexpr int64_t kPlainLook = 64;
+  int64_t plain_steps(const void* b, int64_t k, double scale, std::vector<double>& alphas,
+                      std::vector<double>& betas, double b_norm, double conv_tol, int check_every,
+                      bool keep_vectors) {
+    const bool check = conv_tol > 0.0 && check_every > 0;
+    const KrylovStep s = scalars_for(k, scale);
+    std::vector<double> host(2 * (size_t)k);
+    void* prev = nullptr;
+    void* cur = plain_vec(0, keep_vectors);
+    launch_axpby(prec, n, 1.0 / b_norm, 0.0, b, 0.0, 0.0, cur, nullptr, 0, st);
+    int64_t steps = 0;
+    for (int64_t at = 0; at < k;) {
+      const int64_t to = std::min(k, at + (check ? check_every : kPlainLook));
+      for (int64_t j = at; j < to; ++j) {
+        void* next = plain_vec(j + 1, keep_vectors && j + 1 < k);
+        plain_step(s, j, prev, cur, next);
+        prev = cur;
+        cur = next;
+      }
+      const size_t len = sizeof(double) * (size_t)(to - at);
+      MB_CUDA(cudaMemcpyAsync(host.data() + at, s.alpha + at, len, cudaMemcpyDeviceToHost, st));
+      MB_CUDA(cudaMemcpyAsync(host.data() + k + at, s.beta + at, len, cudaMemcpyDeviceToHost, st));
+      MB_CUDA(cudaStreamSynchronize(st));
+      for (; at < to; ++at) {
+        alphas.push_back(host[(size_t)at]);
+        steps += 1;
+        const double beta = host[(size_t)(k + at)];
+        if (beta <= kTol) return steps;
+        if (at + 1 < k) betas.push_back(beta);
+      }
+      if (check && steps < k && settled(alphas, betas, conv_tol)) return steps;
+    }
+    return steps;
+  }
+
+  // The same with full re-orthogonalisation against the stored, normalised
+  // vectors.
+  int64_t reorth_steps(const void* b, int64_t k, double scale, std::vector<double>& alphas,
+                       std::vector<double>& betas, double b_norm, double conv_tol, int check_every) {
+    void* prev = rot_vec(0);
+    void* cur = rot_vec(1);
+    void* w = rot_vec(2);
+    launch_axpby(prec, n, 1.0 / b_norm, 0.0, b, 0.0, 0.0, cur, nullptr, 0, st);
     double beta_prev = 0.0;
     int64_t steps = 0;
-    double last_ritz = 0.0;
-    bool have_ritz = false;
-    // FP32 runs without re-orthogonalisation keep their Lanczos vectors
-    // unnormalised, u_j = s_j v_j with s_j = beta_(j-1): the next apply and
-    // the combination take 1/s_j in their coefficients, so a step is two
-    // vector passes (apply, combination) instead of three.  Other runs keep
-    // s_j = 1 and normalise as the reference does.
-    const bool fold = prec == MB_PREC_F32 && !reorth;
-    double s_curr = 1.0, s_prev = 1.0;
-    kept = 0;
     for (int64_t it = 0; it < k; ++it) {
-      if (reorth) launch_convert(prec, basis_prec, n, v_curr.p, basis_col(it), st);
-      if (keep_vectors && kept == it && keep_room(it)) {
-        MB_CUDA(cudaMemcpyAsync(keep_col(it), v_curr.p, vb, cudaMemcpyDeviceToDevice, st));
-        kept = it + 1;
-      }
+      launch_convert(prec, basis_prec, n, cur, basis_col(it), st);
       // w = scale*H v - beta_prev v_prev ; alpha = Re<v, w>   (lanczos.h:25-33)
-      launch_apply(op->view, prec, v_curr.p, w.p, scale / s_curr, 0.0, -beta_prev / s_prev,
-                   beta_prev != 0.0 ? v_prev.p : nullptr, red.p(), 1, st);
-      const double alpha = red.fetch(grid_apply, 3, st)[0] / s_curr;
+      launch_apply(op->view, prec, cur, w, scale, 0.0, -beta_prev,
+                   beta_prev != 0.0 ? prev : nullptr, red.p(), 1, st);
+      const double alpha = red.fetch(grid_apply, 3, st)[0];
       // w -= alpha v ; beta = ||w||                             (lanczos.h:34-36)
-      launch_axpby(prec, n, -alpha / s_curr, 0.0, v_curr.p, 1.0, 0.0, w.p, red.p(), 1, st);
+      launch_update(prec, n, -alpha, cur, w, red.p(), KrylovStep{}, st);
       double nrm2 = red.fetch(grid_blas, 3, st)[1];
-      if (reorth) nrm2 = this->reorth((int)(it + 1), nrm2);
+      nrm2 = this->reorth((int)(it + 1), nrm2, w);
       const double beta = std::sqrt(nrm2);
       alphas.push_back(alpha);
       steps += 1;
       if (beta <= kTol) break;
       if (it + 1 < k) betas.push_back(beta);
       // v_prev <- v, v <- w / beta                               (lanczos.h:113-121)
-      std::swap(v_prev.p, v_curr.p);
-      std::swap(v_curr.p, w.p);
-      if (fold) {
-        s_prev = s_curr;
-        s_curr = beta;
-      } else {
-        launch_axpby(prec, n, 0.0, 0.0, nullptr, 1.0 / beta, 0.0, v_curr.p, nullptr, 0, st);
-      }
+      std::swap(prev, cur);
+      std::swap(cur, w);
+      launch_axpby(prec, n, 0.0, 0.0, nullptr, 1.0 / beta, 0.0, cur, nullptr, 0, st);
       beta_prev = beta;
-      if (conv_tol > 0.0 && check_every > 0 && (steps % check_every) == 0 && it + 1 < k) {
-        std::vector<double> d(alphas), e(betas);
-        e.resize(d.size() > 0 ? d.size() - 1 : 0);
-        if (tridiag_eig((int)d.size(), d, e, nullptr)) {
-          const double ritz = d.back();
-          if (ritz_trace) ritz_trace->push_back(ritz);
-          if (have_ritz && std::fabs(ritz - last_ritz) <= conv_tol * std::fabs(ritz)) {
-            betas.resize(steps > 0 ? steps - 1 : 0);
-            break;
-          }
-          last_ritz = ritz;
-          have_ritz = true;
-        }
-      }
+      if (conv_tol > 0.0 && check_every > 0 && (steps % check_every) == 0 && it + 1 < k &&
+          settled(alphas, betas, conv_tol))
+        break;
     }
-    if ((int64_t)betas.size() > std::max<int64_t>(steps - 1, 0)) betas.resize(steps - 1);
     return steps;
   }
 
   // Pass two (lanczos.h:177-218): x = sum_j y_j v_j by re-running the
-  // recurrence; y complex.  x in tensor order, op precision.  Each step runs
-  // pass one's kernels with pass one's coefficients (the apply, the update,
-  // the normalisation of an FP64 run), so the replayed vectors are pass one's
-  // bits: after a Ritz pair converges the recurrence amplifies any rounding
-  // difference, and a replay in other arithmetic drifted from the vectors
-  // whose T_m gave y (an FP32 Ritz vector 6 % off the ground state of a
-  // 49-state sector).
+  // recurrence; y complex.  x in tensor order, op precision.  The steps are
+  // pass one's own kernels on the given alpha and beta, so the replayed
+  // vectors are pass one's bits: after a Ritz pair converges the recurrence
+  // amplifies any rounding difference, and a replay in other arithmetic drifted
+  // from the vectors whose T_m gave y (an FP32 Ritz vector 6 % off the ground
+  // state of a 49-state sector).
   void pass_two(const void* b, int64_t steps, double scale, const std::vector<double>& alphas,
                 const std::vector<double>& betas, double b_norm,
                 const std::vector<std::complex<double>>& y, void* x) {
@@ -974,28 +1049,26 @@ struct Krylov {
       MB_CUDA(cudaMemsetAsync(x, 0, vb, st));
       return;
     }
-    launch_axpby(prec, n, 1.0 / b_norm, 0.0, b, 0.0, 0.0, v_curr.p, nullptr, 0, st);
-    MB_CUDA(cudaMemsetAsync(v_prev.p, 0, vb, st));
-    launch_axpby(prec, n, y[0].real(), y[0].imag(), v_curr.p, 0.0, 0.0, x, nullptr, 0, st);
-    const bool fold = prec == MB_PREC_F32;  // pass one's unnormalised FP32 vectors
-    double s_curr = 1.0, s_prev = 1.0;
+    KrylovStep s = scalars_for(steps, scale);
+    MB_CUDA(cudaMemcpyAsync(s.alpha, alphas.data(), sizeof(double) * (size_t)steps,
+                            cudaMemcpyHostToDevice, st));
+    if (steps > 1)
+      MB_CUDA(cudaMemcpyAsync(s.beta, betas.data(), sizeof(double) * (size_t)(steps - 1),
+                              cudaMemcpyHostToDevice, st));
+    s.ticket = nullptr;  // the scalars are given
+    void* prev = nullptr;
+    void* cur = rot_vec(0);
+    launch_axpby(prec, n, 1.0 / b_norm, 0.0, b, 0.0, 0.0, cur, nullptr, 0, st);
+    launch_axpby(prec, n, y[0].real(), y[0].imag(), cur, 0.0, 0.0, x, nullptr, 0, st);
     for (int64_t j = 0; j + 1 < steps; ++j) {
-      const double alpha_j = alphas[(size_t)j], beta_j = betas[(size_t)j];
-      const double beta_prev = j == 0 ? 0.0 : betas[(size_t)j - 1];
-      launch_apply(op->view, prec, v_curr.p, w.p, scale / s_curr, 0.0, -beta_prev / s_prev,
-                   beta_prev != 0.0 ? v_prev.p : nullptr, red.p(), 1, st);
-      launch_axpby(prec, n, -alpha_j / s_curr, 0.0, v_curr.p, 1.0, 0.0, w.p, red.p(), 1, st);
-      std::swap(v_prev.p, v_curr.p);
-      std::swap(v_curr.p, w.p);
-      if (fold) {
-        s_prev = s_curr;
-        s_curr = beta_j;
-      } else {
-        launch_axpby(prec, n, 0.0, 0.0, nullptr, 1.0 / beta_j, 0.0, v_curr.p, nullptr, 0, st);
-      }
+      void* next = rot_vec(j + 1);
+      plain_step(s, j, prev, cur, next);
+      prev = cur;
+      cur = next;
       // x += y_(j+1) v_(j+1), v_(j+1) = u_(j+1) / s_(j+1)
-      launch_axpby(prec, n, y[(size_t)j + 1].real() / s_curr, y[(size_t)j + 1].imag() / s_curr,
-                   v_curr.p, 1.0, 0.0, x, nullptr, 0, st);
+      const double sj = betas[(size_t)j];
+      launch_axpby(prec, n, y[(size_t)j + 1].real() / sj, y[(size_t)j + 1].imag() / sj, cur, 1.0,
+                   0.0, x, nullptr, 0, st);
     }
   }
 
@@ -1265,7 +1338,7 @@ static void eigenpair(mb_op_s* op, int64_t k, const void* seed, int order,
   const bool refine = o.refine && op->precision == MB_PREC_F32;
   // find_min_eigenpair runs find_max_eigenpair on Negated<Op> (lanczos.h:283-290).
   const int64_t m = kr.pass_one(bt.p, k, sign, alphas, betas, b_norm, reorth, o.conv_tol,
-                                o.check_every, nullptr, !reorth && (vec || refine));
+                                o.check_every, !reorth && (vec || refine));
   if (steps_out) *steps_out = m;
   if (m == 0) {
     *e_out = 0.0;
@@ -1342,7 +1415,7 @@ static void evolve(mb_op_s* op, const void* psi0, int order, double t, int64_t k
   if (k > op->dim) k = op->dim;
   std::vector<double> alphas, betas;
   double b_norm = 0.0;
-  const int64_t m = kr.pass_one(bt.p, k, 1.0, alphas, betas, b_norm, false, 0.0, 0, nullptr, true);
+  const int64_t m = kr.pass_one(bt.p, k, 1.0, alphas, betas, b_norm, false, 0.0, 0, true);
   // expm_tridiagonal_first_column_{unitary,imaginary} (evolve_state.h:22-106)
   std::vector<double> d(alphas), z, e(betas);
   e.resize((size_t)std::max<int64_t>(m - 1, 0));
