@@ -1271,7 +1271,7 @@ struct EngBuf {
   cudaStream_t ps = nullptr;
   EngBuf() = default;
   explicit EngBuf(size_t b) : bytes(b) {
-    if (b) MB_CUDA(cudaMalloc(&p, b));
+    if (b) MB_CUDA(dev_malloc(&p, b));
   }
   EngBuf(size_t b, cudaMemPool_t mp, cudaStream_t st) : bytes(b), pool(mp), ps(st) {
     if (b) MB_CUDA(cudaMallocFromPoolAsync(&p, b, mp, st));
@@ -1346,6 +1346,7 @@ struct EngineSlot {
 }  // namespace mb
 
 struct mb_engine_s {
+  mb::WsHold hold;
   int64_t budget = 0, in_use = 0;
   int warps = 8;                  // chosen by the autotuner
   bool tuned = false;
@@ -2089,6 +2090,7 @@ int mb_engine_create(int64_t device_bytes_budget, mb_engine_t* out) {
     MB_REQUIRE(cudaGetDeviceCount(&n) == cudaSuccess && n > 0, MB_ERR_NO_DEVICE,
                "no CUDA device available");
     auto e = std::make_unique<mb_engine_s>();
+    ws_trim();  // the budget is of what is free
     size_t free_b = 0, total_b = 0;
     MB_CUDA(cudaMemGetInfo(&free_b, &total_b));
     e->budget = device_bytes_budget > 0 ? device_bytes_budget : (int64_t)(free_b * 0.8);

@@ -473,6 +473,29 @@ void fill_fused_tables(OpView& v, const HopTable& tu, const HopTable& td, int64_
 }  // namespace mb
 
 namespace mb {
+// Workspaces kept between calls (mb_pool.cu).  Device memory by stream order
+// (bytes = 0: nullptr), what the device's pool holds idle, and giving that back;
+// cudaMalloc that gives it back where it would not fit otherwise; page-locked
+// host memory (given back with the size it was taken with).  Operators and
+// engines hold the pools while they live.
+void* ws_alloc(size_t bytes, cudaStream_t st);
+void ws_free(void* p, cudaStream_t st);
+size_t ws_idle();
+void ws_trim();
+cudaError_t dev_malloc(void** p, size_t bytes);
+void* pinned_take(size_t bytes);
+void pinned_give(void* p, size_t bytes);
+void ws_hold();
+void ws_drop();
+struct WsHold {
+  WsHold() { ws_hold(); }
+  ~WsHold() { ws_drop(); }
+  WsHold(const WsHold&) = delete;
+  WsHold& operator=(const WsHold&) = delete;
+};
+}  // namespace mb
+
+namespace mb {
 // The reference order of a lattice operator's vectors (device arrays): perm
 // (tensor -> reference index) and the tiles that moves between the two orders
 // take (mb_rows.h).
@@ -508,6 +531,7 @@ OrderTiles order_tiles(int L, const SpinSector& up, const SpinSector& dn, int sl
 }  // namespace mb
 
 struct mb_op_s {
+  mb::WsHold hold;
   int device = 0;
   int precision = MB_PREC_F64;
   int L = 0, n_up = 0, n_down = 0;

@@ -37,22 +37,21 @@ int32_t* op_perm(mb_op_s* op);
 
 namespace {
 
+// Workspace memory of one stream's work (the default stream unless given).
 struct DevBuf {
   void* p = nullptr;
   size_t bytes = 0;
+  cudaStream_t st = 0;
   DevBuf() = default;
-  explicit DevBuf(size_t b) : bytes(b) {
-    if (b) MB_CUDA(cudaMalloc(&p, b));
-  }
-  ~DevBuf() {
-    if (p) cudaFree(p);
-  }
+  explicit DevBuf(size_t b, cudaStream_t s = 0) : bytes(b), st(s) { p = ws_alloc(b, s); }
+  ~DevBuf() { ws_free(p, st); }
   DevBuf(const DevBuf&) = delete;
   DevBuf& operator=(const DevBuf&) = delete;
-  DevBuf(DevBuf&& o) noexcept : p(o.p), bytes(o.bytes) { o.p = nullptr; o.bytes = 0; }
+  DevBuf(DevBuf&& o) noexcept : p(o.p), bytes(o.bytes), st(o.st) { o.p = nullptr; o.bytes = 0; }
   DevBuf& operator=(DevBuf&& o) noexcept {
     std::swap(p, o.p);
     std::swap(bytes, o.bytes);
+    std::swap(st, o.st);
     return *this;
   }
 };
@@ -61,7 +60,7 @@ template <typename T>
 T* upload(mb_op_s* op, const std::vector<T>& h) {
   if (h.empty()) return nullptr;
   void* p = nullptr;
-  MB_CUDA(cudaMalloc(&p, sizeof(T) * h.size()));
+  MB_CUDA(dev_malloc((void**)&p, sizeof(T) * h.size()));
   op->allocations.push_back(p);
   MB_CUDA(cudaMemcpy(p, h.data(), sizeof(T) * h.size(), cudaMemcpyHostToDevice));
   return (T*)p;
@@ -93,13 +92,10 @@ struct Reducer {
   double* host = nullptr;
   int cap_blocks, cap_comp;
   Reducer(int blocks, int comps) : partials(sizeof(double) * (size_t)blocks * comps),
-                                   out(sizeof(double) * (size_t)comps), cap_blocks(blocks),
-                                   cap_comp(comps) {
-    MB_CUDA(cudaMallocHost(&host, sizeof(double) * (size_t)comps));
-  }
-  ~Reducer() {
-    if (host) cudaFreeHost(host);
-  }
+                                   out(sizeof(double) * (size_t)comps),
+                                   host((double*)pinned_take(sizeof(double) * (size_t)comps)),
+                                   cap_blocks(blocks), cap_comp(comps) {}
+  ~Reducer() { pinned_give(host, sizeof(double) * (size_t)cap_comp); }
   double* p() { return (double*)partials.p; }
   // Reduce `nblocks` x `ncomp` partials and copy to host; waits on st.
   const double* fetch(int nblocks, int ncomp, cudaStream_t st) {
@@ -157,7 +153,7 @@ static void build_op(mb_op_s* op, const mb_basis_s* b, const mb_model_s* m) {
   v.max_dn_degree = td.max_degree;
   fill_fused_tables(v, tu, td, op->Du, op->Dd, [op](const void* h, size_t bytes) -> const void* {
     void* p = nullptr;
-    MB_CUDA(cudaMalloc(&p, std::max<size_t>(bytes, 16)));
+    MB_CUDA(dev_malloc((void**)&p, std::max<size_t>(bytes, 16)));
     op->allocations.push_back(p);
     if (bytes) MB_CUDA(cudaMemcpy(p, h, bytes, cudaMemcpyHostToDevice));
     return p;
@@ -311,7 +307,7 @@ static void build_momentum(mb_op_s* op, const mb_basis_s* b, const mb_model_s* m
   if (out.n == 0) return;
   DevBuf cnt(sizeof(int32_t) * (size_t)out.n);
   void* dg = nullptr;
-  MB_CUDA(cudaMalloc(&dg, sizeof(double) * (size_t)out.n));
+  MB_CUDA(dev_malloc((void**)&dg, sizeof(double) * (size_t)out.n));
   op->allocations.push_back(dg);
   out.diag = (double*)dg;
   launch_mom_count(t, (int32_t*)cnt.p, out.diag, st);
@@ -321,7 +317,7 @@ static void build_momentum(mb_op_s* op, const mb_basis_s* b, const mb_model_s* m
   out.nnz = out.row_ptr[(size_t)out.n];
   const int64_t* drp = upload(op, out.row_ptr);
   void* dc = nullptr;
-  MB_CUDA(cudaMalloc(&dc, sizeof(int32_t) * (size_t)std::max<int64_t>(out.nnz, 1)));
+  MB_CUDA(dev_malloc((void**)&dc, sizeof(int32_t) * (size_t)std::max<int64_t>(out.nnz, 1)));
   op->allocations.push_back(dc);
   out.col = (int32_t*)dc;
   launch_mom_fill(t, drp, out.col, st);
@@ -456,14 +452,14 @@ static mb_op_s::Scratch& scratch_for(mb_op_s* op, cudaStream_t st, int nvec, boo
   auto& s = op->scratch[st];
   const size_t vb = elem_bytes(op->precision) * (size_t)op->dim;
   if (nvec >= 1 && !s.a) {
-    MB_CUDA(cudaMalloc(&s.a, vb));
+    MB_CUDA(dev_malloc((void**)&s.a, vb));
   }
   if (nvec >= 2 && !s.b) {
-    MB_CUDA(cudaMalloc(&s.b, vb));
+    MB_CUDA(dev_malloc((void**)&s.b, vb));
   }
   if (staging && !s.hx) {
-    MB_CUDA(cudaMalloc(&s.hx, vb));
-    MB_CUDA(cudaMalloc(&s.hy, vb));
+    MB_CUDA(dev_malloc((void**)&s.hx, vb));
+    MB_CUDA(dev_malloc((void**)&s.hy, vb));
   }
   return s;
 }
@@ -472,7 +468,7 @@ static void ensure_perm(mb_op_s* op) {
   std::lock_guard<std::mutex> lk(op->mu);
   if (op->perm) return;
   void* p = nullptr;
-  MB_CUDA(cudaMalloc(&p, sizeof(int32_t) * (size_t)op->dim));
+  MB_CUDA(dev_malloc((void**)&p, sizeof(int32_t) * (size_t)op->dim));
   op->allocations.push_back(p);
   launch_perm(op->view, (int32_t*)p, 0);
   MB_CUDA(cudaStreamSynchronize(0));
@@ -493,7 +489,7 @@ int32_t* op_iperm(mb_op_s* op) {
   std::lock_guard<std::mutex> lk(op->mu);
   if (!op->iperm) {
     void* p = nullptr;
-    MB_CUDA(cudaMalloc(&p, sizeof(int32_t) * (size_t)op->dim));
+    MB_CUDA(dev_malloc((void**)&p, sizeof(int32_t) * (size_t)op->dim));
     op->allocations.push_back(p);
     launch_invert_perm(op->dim, op->perm, (int32_t*)p, 0);
     MB_CUDA(cudaStreamSynchronize(0));
@@ -609,7 +605,7 @@ void ensure_host_groups(mb_op_s* op) {
   // callers hold host_mu, so no other thread builds the groups meanwhile
   std::lock_guard<std::mutex> lk(op->mu);
   void* p = nullptr;
-  MB_CUDA(cudaMalloc(&p, sizeof(int32_t) * (size_t)std::max<int64_t>(Du, 1)));
+  MB_CUDA(dev_malloc((void**)&p, sizeof(int32_t) * (size_t)std::max<int64_t>(Du, 1)));
   op->allocations.push_back(p);
   MB_CUDA(cudaMemcpy(p, order.data(), sizeof(int32_t) * (size_t)Du, cudaMemcpyHostToDevice));
   op->host_row0 = std::move(row0);
@@ -835,6 +831,7 @@ struct Krylov {
   void reserve_basis(int64_t k, int want_prec) {
     size_t free_b = 0, total_b = 0;
     MB_CUDA(cudaMemGetInfo(&free_b, &total_b));
+    free_b += ws_idle();
     int p = want_prec;
     const size_t need64 = (size_t)k * 16 * (size_t)n, need32 = (size_t)k * 8 * (size_t)n;
     if (p < 0) p = (need64 + (size_t)(1u << 30) < free_b) ? MB_PREC_F64 : MB_PREC_F32;
@@ -874,6 +871,7 @@ struct Krylov {
       cudaGetLastError();
       return false;
     }
+    free_b += ws_idle();
     const size_t need = vb * (size_t)kKeepChunk;
     if (need + total_b / 10 > free_b) return false;
     try {
@@ -1156,11 +1154,12 @@ struct RefineBufs {
   double* host = nullptr;
   cudaStream_t lane[kRefineLanes] = {};
   cudaEvent_t fork = nullptr, done[kRefineLanes] = {};
-  explicit RefineBufs(const RefineSizes& z)
-      : q(z.qbytes), c(sizeof(double) * z.cwords),
-        part(sizeof(double) * kRefineLanes * (size_t)z.pblocks * z.pcomps),
-        pstride((size_t)z.pblocks * z.pcomps) {
-    MB_CUDA(cudaMallocHost(&host, sizeof(double) * z.cwords));
+  size_t host_bytes = 0;
+  RefineBufs(const RefineSizes& z, cudaStream_t st)
+      : q(z.qbytes, st), c(sizeof(double) * z.cwords, st),
+        part(sizeof(double) * kRefineLanes * (size_t)z.pblocks * z.pcomps, st),
+        pstride((size_t)z.pblocks * z.pcomps), host_bytes(sizeof(double) * z.cwords) {
+    host = (double*)pinned_take(host_bytes);
     MB_CUDA(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
     for (int k = 0; k < kRefineLanes; ++k) {
       MB_CUDA(cudaStreamCreateWithFlags(&lane[k], cudaStreamNonBlocking));
@@ -1168,12 +1167,17 @@ struct RefineBufs {
     }
   }
   ~RefineBufs() {
+    // the buffers go back in the caller's stream's order: nothing of a lane may
+    // still be in flight (after an error; a finished call waited already)
     for (int k = 0; k < kRefineLanes; ++k) {
-      if (lane[k]) cudaStreamDestroy(lane[k]);
+      if (lane[k]) {
+        cudaStreamSynchronize(lane[k]);
+        cudaStreamDestroy(lane[k]);
+      }
       if (done[k]) cudaEventDestroy(done[k]);
     }
     if (fork) cudaEventDestroy(fork);
-    if (host) cudaFreeHost(host);
+    pinned_give(host, host_bytes);
   }
   RefineBufs(const RefineBufs&) = delete;
   RefineBufs& operator=(const RefineBufs&) = delete;
@@ -1299,7 +1303,7 @@ void fp64_refine_many(RefineProblem* probs, int count, cudaStream_t st) {
   }
   RefineSizes most;
   for (const auto& z : sizes) most.widen(z);
-  RefineBufs bufs(most);
+  RefineBufs bufs(most, st);
   for (auto& g : groups) refine_chunk(g, bufs, st);
 }
 
@@ -1458,7 +1462,7 @@ int mb_alloc(void** dev_ptr, size_t bytes) {
   return guard([&] {
     MB_REQUIRE(dev_ptr, MB_ERR_INVALID_ARG, "NULL argument");
     require_device();
-    MB_CUDA(cudaMalloc(dev_ptr, bytes));
+    MB_CUDA(dev_malloc(dev_ptr, bytes));
   });
 }
 
@@ -1735,9 +1739,9 @@ int mb_op_autotune(mb_op_t op, void* stream, mb_apply_shape* chosen, double* bes
         own = {x, y, prm};
       } else {
         const size_t vb = elem_bytes(op->precision) * (size_t)op->dim;
-        MB_CUDA(cudaMalloc(&x, vb));
+        MB_CUDA(dev_malloc((void**)&x, vb));
         own.push_back(x);
-        MB_CUDA(cudaMalloc(&y, vb));
+        MB_CUDA(dev_malloc((void**)&y, vb));
         own.push_back(y);
         launch_fill_rng(op->precision, op->Du, op->Dd, 12345, 0, 0, x, st);
       }

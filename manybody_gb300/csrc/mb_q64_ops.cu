@@ -18,20 +18,19 @@ namespace mb {
 
 namespace {
 
+// Workspace memory of one stream's work (the default stream unless given).
 struct QBuf {
   void* p = nullptr;
+  cudaStream_t st = 0;
   QBuf() = default;
-  explicit QBuf(size_t b) {
-    if (b) MB_CUDA(cudaMalloc(&p, b));
-  }
-  ~QBuf() {
-    if (p) cudaFree(p);
-  }
+  explicit QBuf(size_t b, cudaStream_t s = 0) : st(s) { p = ws_alloc(b, s); }
+  ~QBuf() { ws_free(p, st); }
   QBuf(const QBuf&) = delete;
   QBuf& operator=(const QBuf&) = delete;
-  QBuf(QBuf&& o) noexcept : p(o.p) { o.p = nullptr; }
+  QBuf(QBuf&& o) noexcept : p(o.p), st(o.st) { o.p = nullptr; }
   QBuf& operator=(QBuf&& o) noexcept {
     std::swap(p, o.p);
+    std::swap(st, o.st);
     return *this;
   }
 };
@@ -114,10 +113,10 @@ static mb_op_s::QScratch& qscratch_for(mb_op_s* op, cudaStream_t st) {
   auto& s = op->qscratch[st];
   if (!s.xq) {
     const size_t vb = sizeof(longlong2) * (size_t)op->dim;
-    MB_CUDA(cudaMalloc(&s.xq, vb));
-    MB_CUDA(cudaMalloc(&s.yq, vb));
-    MB_CUDA(cudaMalloc(&s.prm, sizeof(QParams)));
-    MB_CUDA(cudaMalloc((void**)&s.ints, 4 * sizeof(int)));
+    MB_CUDA(dev_malloc((void**)&s.xq, vb));
+    MB_CUDA(dev_malloc((void**)&s.yq, vb));
+    MB_CUDA(dev_malloc((void**)&s.prm, sizeof(QParams)));
+    MB_CUDA(dev_malloc((void**)&s.ints, 4 * sizeof(int)));
   }
   return s;
 }
@@ -128,7 +127,7 @@ static void* q_ups_for(mb_op_s* op, cudaStream_t st) {
   if (op->apply_passes != 2 || !q_upcol_fits(op->view)) return nullptr;
   std::lock_guard<std::mutex> lk(op->mu);
   void*& p = op->ups_scratch[st];
-  if (!p) MB_CUDA(cudaMalloc(&p, sizeof(longlong2) * (size_t)op->dim));
+  if (!p) MB_CUDA(dev_malloc((void**)&p, sizeof(longlong2) * (size_t)op->dim));
   return p;
 }
 
@@ -148,9 +147,9 @@ void q_tune_prepare(mb_op_s* op, void** xq, void** yq, void** prm, cudaStream_t 
   QBuf x64(vb), ints(4 * sizeof(int));
   void *a = nullptr, *b = nullptr, *p = nullptr;
   try {
-    MB_CUDA(cudaMalloc(&a, vb));
-    MB_CUDA(cudaMalloc(&b, vb));
-    MB_CUDA(cudaMalloc(&p, sizeof(QParams)));
+    MB_CUDA(dev_malloc((void**)&a, vb));
+    MB_CUDA(dev_malloc((void**)&b, vb));
+    MB_CUDA(dev_malloc((void**)&p, sizeof(QParams)));
     launch_fill_rng(MB_PREC_F64, op->Du, op->Dd, 12345, 0, 0, x64.p, st);
     launch_f64_to_q(op->dim, x64.p, RowOrder{}, op->q_qbits, (int*)ints.p, a, st);
     launch_q_plan(q_plain_plan_input(op), (const int*)ints.p + 1, (QParams*)p, st);
@@ -204,7 +203,7 @@ void q_apply_affine(mb_op_s* op, const void* x, void* y, double scale, double sh
   }
   // y = beta z + (Q64 result): z may alias y; convert into a tensor-order
   // temporary, then combine with the FP64 vector kernel.
-  QBuf tmp(sizeof(double2) * (size_t)op->dim);
+  QBuf tmp(sizeof(double2) * (size_t)op->dim, st);
   q_to_order(op, s.yq, order, ey, tmp.p, st);
   launch_axpby(MB_PREC_F64, op->dim, beta, 0.0, z, 1.0, 0.0, tmp.p, nullptr, 0, st);
   MB_CUDA(cudaMemcpyAsync(y, tmp.p, sizeof(double2) * (size_t)op->dim, cudaMemcpyDeviceToDevice, st));
@@ -337,15 +336,13 @@ struct QKrylov {
         prm(sizeof(QParams)),
         grid_apply(q_apply_grid(o->view)), grid_blas(q_blas_grid(o->dim)),
         grid_md(q_multi_dot_grid(o->dim)), coef(sizeof(long long) * 2 * kQMaxBasis) {
-    MB_CUDA(cudaMallocHost((void**)&host, sizeof(double) * (2 * kQMaxBasis + 8)));
-    MB_CUDA(cudaMallocHost((void**)&hprm, sizeof(QParams)));
-    MB_CUDA(cudaMallocHost((void**)&hcoef, sizeof(long long) * 2 * kQMaxBasis));
+    host = (double*)pinned_take(kPinnedBytes);
+    hcoef = (long long*)(host + 2 * kQMaxBasis + 8);
+    hprm = (QParams*)(hcoef + 2 * kQMaxBasis);
   }
-  ~QKrylov() {
-    if (host) cudaFreeHost(host);
-    if (hprm) cudaFreeHost(hprm);
-    if (hcoef) cudaFreeHost(hcoef);
-  }
+  ~QKrylov() { pinned_give(host, kPinnedBytes); }
+  static constexpr size_t kPinnedBytes =
+      sizeof(double) * (2 * kQMaxBasis + 8) + sizeof(long long) * 2 * kQMaxBasis + sizeof(QParams);
 
   double* part() { return (double*)partials.p; }
   unsigned long long* mor() { return (unsigned long long*)maxor.p; }
@@ -442,6 +439,7 @@ struct QKrylov {
   void reserve_basis(int64_t k) {
     size_t free_b = 0, total_b = 0;
     MB_CUDA(cudaMemGetInfo(&free_b, &total_b));
+    free_b += ws_idle();
     const size_t need = (size_t)k * sizeof(longlong2) * (size_t)n;
     MB_REQUIRE(need + (size_t)(512u << 20) < free_b, MB_ERR_OOM,
                "Krylov basis for full re-orthogonalisation does not fit in device memory");
@@ -587,6 +585,7 @@ struct QKrylov {
       cudaGetLastError();
       return false;
     }
+    free_b += ws_idle();
     const size_t need = sizeof(longlong2) * (size_t)n * (size_t)kQKeepChunk;
     if (need + total_b / 10 > free_b) return false;
     try {
@@ -793,7 +792,7 @@ int mb_q64_from_f64(mb_op_t op, const void* x_dev, int order, void* xq_dev, int*
                "bad order");
     cudaStream_t st = (cudaStream_t)stream;
     const RowOrder o = order == MB_ORDER_REFERENCE ? op_row_order(op) : RowOrder{};
-    QBuf ints(4 * sizeof(int));
+    QBuf ints(4 * sizeof(int), st);
     launch_f64_to_q(op->dim, x_dev, o, op->q_qbits, (int*)ints.p, xq_dev, st);
     int h[2];
     MB_CUDA(cudaMemcpyAsync(h, ints.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -809,7 +808,7 @@ int mb_q64_to_f64(mb_op_t op, const void* xq_dev, int exponent, int order, void*
     MB_REQUIRE(order == MB_ORDER_REFERENCE || order == MB_ORDER_TENSOR, MB_ERR_INVALID_ARG,
                "bad order");
     cudaStream_t st = (cudaStream_t)stream;
-    QBuf e(sizeof(int));
+    QBuf e(sizeof(int), st);
     MB_CUDA(cudaMemcpyAsync(e.p, &exponent, sizeof(int), cudaMemcpyHostToDevice, st));
     q_to_order(op, xq_dev, order, (const int*)e.p, x_dev, st);
     MB_CUDA(cudaStreamSynchronize(st));
