@@ -2324,20 +2324,26 @@ int mb_kpm_dos_moments(mb_op_t op, int64_t n_moments, int64_t n_probes, uint64_t
     // Device-side moment sums per step, read once per probe.  Step s produces
     // T_{s+1}; moments up to n_moments-1 need T_j for j <= n_moments/2.
     const int64_t nsteps = std::max<int64_t>(n_moments / 2, 1);
-    DevBuf dots(sizeof(double) * 3 * (size_t)nsteps);
+    DevBuf dots(sizeof(double) * (3 * (size_t)nsteps + 1));
     std::vector<double> acc((size_t)n_moments, 0.0), hd(3 * (size_t)nsteps);
+    // a step's sums are finished by the last block of its apply
+    OpView v = op->view;
+    v.step.ticket = (unsigned*)((double*)dots.p + 3 * nsteps);
+    v.step.blocks = ga;
+    v.step.part = red.p();
+    MB_CUDA(cudaMemsetAsync(v.step.ticket, 0, sizeof(unsigned), st));
     for (int64_t p = 0; p < n_probes; ++p) {
       void* cur = t0.p;   // T_n
       void* oth = t1.p;   // T_{n-1}, then T_{n+1}
       launch_fill_rng(op->precision, op->Du, op->Dd, seed, (uint32_t)(1 + p), 1, cur, st);
       // step 0: T1 = Ht T0 into oth; dots <T0,T1>, <T1,T1>, <T0,T0>
-      launch_apply(op->view, op->precision, cur, oth, 1.0 / a, b, 0.0, nullptr, red.p(), 7, st);
-      launch_reduce(red.p(), ga, 3, (double*)dots.p, st);
+      v.step.dots = (double*)dots.p;
+      launch_apply(v, op->precision, cur, oth, 1.0 / a, b, 0.0, nullptr, red.p(), 7, st);
       std::swap(cur, oth);  // cur = T1, oth = T0
       for (int64_t s = 1; s < nsteps; ++s) {
         // T_{s+1} = 2 Ht T_s - T_{s-1}, written over T_{s-1}
-        launch_apply(op->view, op->precision, cur, oth, 2.0 / a, b, -1.0, oth, red.p(), 3, st);
-        launch_reduce(red.p(), ga, 3, (double*)dots.p + 3 * s, st);
+        v.step.dots = (double*)dots.p + 3 * s;
+        launch_apply(v, op->precision, cur, oth, 2.0 / a, b, -1.0, oth, red.p(), 3, st);
         std::swap(cur, oth);
       }
       MB_CUDA(cudaMemcpyAsync(hd.data(), dots.p, sizeof(double) * hd.size(), cudaMemcpyDeviceToHost, st));

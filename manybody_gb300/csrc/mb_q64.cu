@@ -182,9 +182,8 @@ __device__ void q_block_reduce_exact(__int128 xy, __int128 yy, unsigned long lon
 }
 
 // The exact sum of nblocks such partials, converted once to double: out[0]
-// (xy), out[1] (yy).
-__global__ void k_q_reduce128(const long long* __restrict__ part, int nblocks,
-                              double* __restrict__ out) {
+// (xy), out[1] (yy), in thread 0.
+__device__ void q_sum128(const long long* __restrict__ part, int nblocks, double (&out)[2]) {
   __int128 a = 0, b = 0;
   for (int i = threadIdx.x; i < nblocks; i += blockDim.x) {
     const long long* p = part + 4 * (size_t)i;
@@ -211,6 +210,16 @@ __global__ void k_q_reduce128(const long long* __restrict__ part, int nblocks,
     }
     out[0] = i128_to_f64(sa);
     out[1] = i128_to_f64(sb);
+  }
+}
+
+__global__ void k_q_reduce128(const long long* __restrict__ part, int nblocks,
+                              double* __restrict__ out) {
+  double s[2];
+  q_sum128(part, nblocks, s);
+  if (threadIdx.x == 0) {
+    out[0] = s[0];
+    out[1] = s[1];
   }
 }
 
@@ -719,15 +728,6 @@ static void launch_csr_apply_q(const OpView& v, const void* x, void* y, const vo
   }
 }
 
-int q_apply_grid(const OpView& v) {
-  if (v.csr_row) return q_csr_grid(v);
-  const int split = v.row_split > 1 ? v.row_split : 1;
-  int64_t g = sm_count();
-  if (g > v.Du * split) g = v.Du * split;
-  g -= g % split;
-  return (int)std::max<int64_t>(g, split);
-}
-
 // the table width a launch uses: 16-bit where the view has the copies
 static int q_table_bits(const OpView& v, bool rows) {
   if (v.table_bits != 16) return 32;
@@ -743,6 +743,34 @@ static size_t q_apply_smem(const OpView& v, bool staged, bool ups, bool ts) {
   return smem;
 }
 
+// Threads of the apply's CTAs and how many of them an SM holds, kQThreads
+// together: small CTAs, where their rows fit in shared memory side by side, hide
+// each other's staging and barriers and leave fewer warps without a column group
+// in a row's last round (4x4 4+4, 1,820 columns:
+// 113 -> 101 us with 256; 3x4 5+4, 495: 26.7 -> 20.6; 4x4 5+5, 4,368: 677 -> 647
+// with 512).
+struct QCtas {
+  int threads, per_sm;
+};
+static QCtas q_ctas(const OpView& v) {
+  if (v.table_stage) return {kQThreads, 1};  // the warps' buffers take the rest
+  const bool staged = q_apply_smem(v, true, false, false) + 2048 <= (size_t)smem_optin();
+  const size_t row = q_apply_smem(v, staged, false, false) + 5120;
+  int threads = 256;
+  while (threads < kQThreads && (size_t)(kQThreads / threads) * row > (size_t)smem_optin() + 1024)
+    threads *= 2;
+  return {threads, kQThreads / threads};
+}
+
+int q_apply_grid(const OpView& v) {
+  if (v.csr_row) return q_csr_grid(v);
+  const int split = v.row_split > 1 ? v.row_split : 1;
+  int64_t g = (int64_t)sm_count() * q_ctas(v).per_sm;
+  if (g > v.Du * split) g = v.Du * split;
+  g -= g % split;
+  return (int)std::max<int64_t>(g, split);
+}
+
 template <bool STAGED, int DOTS, bool HAS_Z, bool UPS, int TB, bool TS = false>
 static void q_apply_t(const OpView& v, const void* x, void* y, const void* z, const QParams* prm,
                       double* partials, unsigned long long* max_or, const void* ups,
@@ -750,7 +778,7 @@ static void q_apply_t(const OpView& v, const void* x, void* y, const void* z, co
   const size_t smem = q_apply_smem(v, STAGED, UPS, TS);
   auto kern = k_apply_q<STAGED, DOTS, HAS_Z, UPS, TB, TS>;
   MB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  kern<<<q_apply_grid(v), kQThreads, smem, st>>>(v, (const longlong2*)x, (longlong2*)y,
+  kern<<<q_apply_grid(v), q_ctas(v).threads, smem, st>>>(v, (const longlong2*)x, (longlong2*)y,
                                                    (const longlong2*)z, prm, partials, max_or,
                                                    (const longlong2*)ups);
   MB_CUDA(cudaGetLastError());
@@ -1001,6 +1029,37 @@ __global__ void k_plan(QPlanInput in, const int* __restrict__ ex, QParams* __res
   in.ex = *ex;
   in.ez = in.ex;
   q_plan(p, in);
+}
+
+// One turn of a recurrence planned on the device: the dots of the apply before
+// (of x to y, their exponents given) and the plan of the one after.
+__global__ void k_q_turn(QTurn t) {
+  if (t.part) {
+    double s[2];
+    q_sum128((const long long*)t.part, t.nblocks, s);
+    if (threadIdx.x == 0) {
+      t.dots[0] = ldexp(s[0], t.x->E + t.y->E + 32);
+      t.dots[1] = ldexp(s[1], 2 * t.y->E + 32);
+    }
+  }
+  if (!t.prm || threadIdx.x != 0) return;
+  QPlanInput in = t.in;
+  auto frac = [&](const QVecState* v) {  // bound on max |q| over 2^qbits: max < 2^bitlen(OR)
+    const double m = v->max_or ? ldexp(1.0, 64 - __clzll((long long)v->max_or)) : 1.0;
+    return fmin(ldexp(m, -t.qbits), 1.0);
+  };
+  in.ex = t.nx->E;
+  in.x_frac = frac(t.nx);
+  in.ez = in.has_z ? t.nz->E : in.ex;
+  in.z_frac = in.has_z ? frac(t.nz) : 1.0;
+  q_plan(t.prm, in);
+  t.ny->E = t.prm->ey;
+  t.ny->max_or = 0;
+}
+
+void launch_q_turn(const QTurn& t, cudaStream_t st) {
+  k_q_turn<<<1, 256, 0, st>>>(t);
+  MB_CUDA(cudaGetLastError());
 }
 
 void launch_f64_to_q(int64_t n, const void* src, const RowOrder& o, int qbits, int* scratch_int2,

@@ -45,6 +45,32 @@ __host__ __device__ void q_plan(QParams* p, const QPlanInput& in);
 // operator, the exponent of x read on the device.
 QPlanInput q_plain_plan_input(const mb_op_s* op);
 
+// A vector of a recurrence that is planned on the device (QTurn): its exponent
+// and the OR of its mantissas' magnitudes, which the apply that writes it
+// collects (an apply's max_or).
+struct QVecState {
+  unsigned long long max_or;
+  int E;
+  int pad;
+};
+
+// Between two applies of such a recurrence: the dots of the one before, <x,y>
+// and <y,y> to dots[0..1] (part = its 128-bit partials; nullptr: none), and the
+// plan of the one after, ny = scale (H - shift) nx + beta nz (prm = nullptr:
+// none; in: q_turn_input), so that no step waits for the host.
+struct QTurn {
+  const void* part;
+  int nblocks;
+  const QVecState *x, *y;
+  double* dots;
+  QParams* prm;
+  QPlanInput in;
+  int qbits;
+  const QVecState *nx, *nz;
+  QVecState* ny;
+};
+void launch_q_turn(const QTurn& t, cudaStream_t st);
+
 // The fused apply (see mb_q64.cu).  y must not alias x or z.  With ups (the
 // column pass's up-hop sums of x, launch_upcol_q) the up hops are read from
 // it; without, they are gathered from x in the same pass.  dots: 0 none;

@@ -708,32 +708,50 @@ void q_kpm_dos_moments(mb_op_s* op, int64_t n_moments, int64_t n_probes, uint64_
   QVec v0(n), v1(n), v2(n);
   QBuf probe(sizeof(double2) * (size_t)n);
   const int64_t nsteps = std::max<int64_t>(n_moments / 2, 1);
-  std::vector<double> acc((size_t)n_moments, 0.0), self((size_t)nsteps + 1), cross((size_t)nsteps);
+  std::vector<double> acc((size_t)n_moments, 0.0), dots(2 * (size_t)nsteps);
+  // the steps are planned on the device: the vectors' states, the steps' dots
+  QBuf dev(sizeof(double) * dots.size() + 3 * sizeof(QVecState));
+  double* ddots = (double*)dev.p;
+  QVecState* state = (QVecState*)(ddots + dots.size());
   for (int64_t p = 0; p < n_probes; ++p) {
     launch_fill_rng(MB_PREC_F64, op->Du, op->Dd, seed, (uint32_t)(1 + p), 1, probe.p, st);
     const double nrm = kr.load(probe.p, MB_ORDER_TENSOR, v0.r);
-    QRef* prev = &v0.r;
-    QRef* cur = &v1.r;
-    QRef* nxt = &v2.r;
     const double mu0 = nrm * nrm;
-    const auto first = kr.apply_affine(*cur, *prev, 1.0 / a, b, 0.0, nullptr);
-    cross[0] = first.first;
-    self[1] = first.second;
-    for (int64_t s = 1; s < nsteps; ++s) {
-      const auto r = kr.apply_affine(*nxt, *cur, 2.0 / a, b, -1.0, prev);
-      cross[(size_t)s] = r.first;
-      self[(size_t)s + 1] = r.second;
-      QRef* old = prev;
-      prev = cur;
-      cur = nxt;
-      nxt = old;
+    // an OR whose length is qbits: the bound of a loaded vector
+    const QVecState first{(1ull << kr.qbits) - 1ull, v0.r.E, 0};
+    MB_CUDA(cudaMemcpyAsync(state, &first, sizeof(first), cudaMemcpyHostToDevice, st));
+    void* vec[3] = {v0.r.p, v1.r.p, v2.r.p};
+    QTurn t{};
+    t.qbits = kr.qbits;
+    t.nblocks = kr.grid_apply;
+    for (int64_t s = 0; s < nsteps; ++s) {
+      // T_(s+1) from T_s and T_(s-1): vectors s + 1, s and s - 1 mod 3
+      const int next = (int)((s + 1) % 3), cur = (int)(s % 3), prev = (int)((s + 2) % 3);
+      t.prm = (QParams*)kr.prm.p;
+      t.in = plan_input(op, (s ? 2.0 : 1.0) / a, b, s ? -1.0 : 0.0, 0, 0, s > 0);
+      t.nx = state + cur;
+      t.nz = state + prev;
+      t.ny = state + next;
+      launch_q_turn(t, st);
+      q_apply_whole(op, vec[cur], vec[next], s ? vec[prev] : nullptr, t.prm, kr.part(),
+                    &t.ny->max_or, 1, st);
+      t.part = kr.part();
+      t.x = t.nx;
+      t.y = t.ny;
+      t.dots = ddots + 2 * s;
     }
-    const double mu1 = cross[0];
+    t.prm = nullptr;
+    launch_q_turn(t, st);
+    MB_CUDA(cudaMemcpyAsync(dots.data(), ddots, sizeof(double) * dots.size(),
+                            cudaMemcpyDeviceToHost, st));
+    MB_CUDA(cudaStreamSynchronize(st));
+    // dots[2s] = <T_s,T_(s+1)>, dots[2s+1] = <T_(s+1),T_(s+1)>
+    const double mu1 = dots[0];
     acc[0] += mu0;
     if (n_moments > 1) acc[1] += mu1;
     for (int64_t s = 1; 2 * s < n_moments; ++s) {
-      acc[(size_t)(2 * s)] += 2.0 * self[(size_t)s] - mu0;
-      if (2 * s + 1 < n_moments) acc[(size_t)(2 * s + 1)] += 2.0 * cross[(size_t)s] - mu1;
+      acc[(size_t)(2 * s)] += 2.0 * dots[2 * (size_t)s - 1] - mu0;
+      if (2 * s + 1 < n_moments) acc[(size_t)(2 * s + 1)] += 2.0 * dots[2 * (size_t)s] - mu1;
     }
   }
   const double norm = 1.0 / ((double)n_probes * (double)n);
