@@ -1274,7 +1274,11 @@ struct EngBuf {
     if (b) MB_CUDA(dev_malloc(&p, b));
   }
   EngBuf(size_t b, cudaMemPool_t mp, cudaStream_t st) : bytes(b), pool(mp), ps(st) {
-    if (b) MB_CUDA(cudaMallocFromPoolAsync(&p, b, mp, st));
+    if (b && cudaMallocFromPoolAsync(&p, b, mp, st) != cudaSuccess) {
+      cudaGetLastError();
+      ws_trim();
+      MB_CUDA(cudaMallocFromPoolAsync(&p, b, mp, st));
+    }
   }
   ~EngBuf() {
     if (!p) return;
@@ -2090,9 +2094,9 @@ int mb_engine_create(int64_t device_bytes_budget, mb_engine_t* out) {
     MB_REQUIRE(cudaGetDeviceCount(&n) == cudaSuccess && n > 0, MB_ERR_NO_DEVICE,
                "no CUDA device available");
     auto e = std::make_unique<mb_engine_s>();
-    ws_trim();  // the budget is of what is free
     size_t free_b = 0, total_b = 0;
     MB_CUDA(cudaMemGetInfo(&free_b, &total_b));
+    free_b += ws_idle();  // given back where an allocation needs it
     e->budget = device_bytes_budget > 0 ? device_bytes_budget : (int64_t)(free_b * 0.8);
     MB_CUDA(cudaStreamCreateWithFlags(&e->st, cudaStreamNonBlocking));
     for (cudaEvent_t& x : e->ev) MB_CUDA(cudaEventCreate(&x));

@@ -653,12 +653,16 @@ void launch_norm2(int precision, int64_t n, const void* x, double* partials, cud
 void launch_dot(int precision, int64_t n, const void* x, const void* y, double* partials,
                 cudaStream_t st);
 int multi_dot_grid(int64_t n);
-// c[j] = <V_j, w> for j < m (complex, 2 comps each) -> partials [blocks][2m]
+// out[j] = <V_j, w> for j < m (complex, 2 comps each), through partials
+// [multi_dot_grid][2m] and a ticket that is 0 between launches
 void launch_multi_dot(int vprec, int wprec, int64_t n, const void* V, int64_t ld, int m,
-                      const void* w, double* partials, cudaStream_t st);
-// w -= sum_j c[j] V_j ; c on device (interleaved complex), then <w,w> partials
+                      const void* w, double* partials, unsigned* ticket, double* out,
+                      cudaStream_t st);
+// w -= sum_j c[j] V_j ; c on device (interleaved complex), then <w,w> partials,
+// summed to step.dots where it has a ticket
 void launch_multi_axpy(int vprec, int wprec, int64_t n, const void* V, int64_t ld, int m,
-                       const double* c, void* w, double* partials, cudaStream_t st);
+                       const double* c, void* w, double* partials, const KrylovStep& step,
+                       cudaStream_t st);
 void launch_convert(int from_prec, int to_prec, int64_t n, const void* x, void* y,
                     cudaStream_t st);
 void launch_gather(int precision, int64_t n, const int32_t* perm, const void* src, void* dst,

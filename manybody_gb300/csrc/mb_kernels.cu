@@ -1010,7 +1010,8 @@ constexpr int kMaxBasis = 1024;
 template <typename TV, typename TW>
 __global__ void __launch_bounds__(kMdThreads)
 k_multi_dot(int64_t n, const typename C2<TV>::type* __restrict__ V, int64_t ld, int m,
-            const typename C2<TW>::type* __restrict__ w, double* __restrict__ partials) {
+            const typename C2<TW>::type* __restrict__ w, double* partials, unsigned* ticket,
+            double* __restrict__ out) {
   using VV = typename C2<TV>::type;
   using VW = typename C2<TW>::type;
   __shared__ double acc[2 * kMaxBasis];
@@ -1092,6 +1093,28 @@ k_multi_dot(int64_t n, const typename C2<TV>::type* __restrict__ V, int64_t ld, 
   __syncthreads();
   for (int j = threadIdx.x; j < 2 * m; j += blockDim.x)
     partials[(size_t)blockIdx.x * 2 * m + j] = acc[j];
+  // the last block to finish sums every block's partials in block order: warp w
+  // the sums w, w + 8, ..., four chains a lane
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(ticket, 1u) + 1u == gridDim.x;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  const int nb = (int)gridDim.x, nc = 2 * m;
+  for (int k = warp; k < nc; k += nwarps) {
+    double a[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int b = lane; b < nb; b += 128)
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (b + 32 * q < nb) a[q] += __ldcg(partials + (size_t)(b + 32 * q) * nc + k);
+    double t = (a[0] + a[1]) + (a[2] + a[3]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+    if (lane == 0) out[k] = t;
+  }
+  if (threadIdx.x == 0) *ticket = 0;
 }
 
 static int md_grid(int64_t n) {
@@ -1105,19 +1128,23 @@ static int md_grid(int64_t n) {
 
 int multi_dot_grid(int64_t n) { return md_grid(n); }
 
-void launch_multi_dot(int vprec, int wprec, int64_t n, const void* V, int64_t ld, int m,
-                      const void* w, double* partials, cudaStream_t st) {
-  MB_REQUIRE(m <= kMaxBasis, MB_ERR_CAPACITY, "re-orthogonalisation basis larger than 1024");
-  const int g = md_grid(n);
-  if (vprec == MB_PREC_F32 && wprec == MB_PREC_F32)
-    k_multi_dot<float, float><<<g, kMdThreads, 0, st>>>(n, (const float2*)V, ld, m, (const float2*)w, partials);
-  else if (vprec == MB_PREC_F32)
-    k_multi_dot<float, double><<<g, kMdThreads, 0, st>>>(n, (const float2*)V, ld, m, (const double2*)w, partials);
-  else if (wprec == MB_PREC_F32)
-    k_multi_dot<double, float><<<g, kMdThreads, 0, st>>>(n, (const double2*)V, ld, m, (const float2*)w, partials);
-  else
-    k_multi_dot<double, double><<<g, kMdThreads, 0, st>>>(n, (const double2*)V, ld, m, (const double2*)w, partials);
+template <typename TV, typename TW>
+static void multi_dot_t(int64_t n, const void* V, int64_t ld, int m, const void* w,
+                        double* partials, unsigned* ticket, double* out, cudaStream_t st) {
+  k_multi_dot<TV, TW><<<md_grid(n), kMdThreads, 0, st>>>(
+      n, (const typename C2<TV>::type*)V, ld, m, (const typename C2<TW>::type*)w, partials, ticket, out);
   MB_CUDA(cudaGetLastError());
+}
+
+void launch_multi_dot(int vprec, int wprec, int64_t n, const void* V, int64_t ld, int m,
+                      const void* w, double* partials, unsigned* ticket, double* out,
+                      cudaStream_t st) {
+  MB_REQUIRE(m <= kMaxBasis, MB_ERR_CAPACITY, "re-orthogonalisation basis larger than 1024");
+  const bool v32 = vprec == MB_PREC_F32, w32 = wprec == MB_PREC_F32;
+  if (v32 && w32) multi_dot_t<float, float>(n, V, ld, m, w, partials, ticket, out, st);
+  else if (v32) multi_dot_t<float, double>(n, V, ld, m, w, partials, ticket, out, st);
+  else if (w32) multi_dot_t<double, float>(n, V, ld, m, w, partials, ticket, out, st);
+  else multi_dot_t<double, double>(n, V, ld, m, w, partials, ticket, out, st);
 }
 
 // w -= sum_j c_j V_j (c complex, on device), then <w,w> partials.
@@ -1125,7 +1152,7 @@ template <typename TV, typename TW>
 __global__ void __launch_bounds__(kBlasThreads)
 k_multi_axpy(int64_t n, const typename C2<TV>::type* __restrict__ V, int64_t ld, int m,
              const double* __restrict__ c, typename C2<TW>::type* __restrict__ w,
-             double* __restrict__ partials) {
+             double* __restrict__ partials, KrylovStep step) {
   using VV = typename C2<TV>::type;
   using VW = typename C2<TW>::type;
   __shared__ double sc[2 * kMaxBasis];
@@ -1172,9 +1199,14 @@ k_multi_axpy(int64_t n, const typename C2<TV>::type* __restrict__ V, int64_t ld,
 #pragma unroll
         for (int u = 0; u < kMdBatch; ++u) {
           if (j0 + u >= m) break;
+          // four multiply-adds (a difference of products would take six)
           const double cr = sc[2 * (j0 + u)], ci = sc[2 * (j0 + u) + 1];
-          sr -= cr * (double)a[u].x - ci * (double)a[u].y;
-          si -= cr * (double)a[u].y + ci * (double)a[u].x;
+          sr = fma(-cr, (double)a[u].x, sr);
+          si = fma(-cr, (double)a[u].y, si);
+          if (ci != 0.0) {
+            sr = fma(ci, (double)a[u].y, sr);
+            si = fma(-ci, (double)a[u].x, si);
+          }
         }
       }
     }
@@ -1187,20 +1219,22 @@ k_multi_axpy(int64_t n, const typename C2<TV>::type* __restrict__ V, int64_t ld,
   }
   double vals[3] = {0.0, ww.value(), 0.0};
   block_reduce_store<2>(vals, partials);
+  if (step.ticket) finish_step<true, 2>(step);
 }
 
 void launch_multi_axpy(int vprec, int wprec, int64_t n, const void* V, int64_t ld, int m,
-                       const double* c, void* w, double* partials, cudaStream_t st) {
+                       const double* c, void* w, double* partials, const KrylovStep& step,
+                       cudaStream_t st) {
   MB_REQUIRE(m <= kMaxBasis, MB_ERR_CAPACITY, "re-orthogonalisation basis larger than 1024");
   const int g = blas_grid(n);
   if (vprec == MB_PREC_F32 && wprec == MB_PREC_F32)
-    k_multi_axpy<float, float><<<g, kBlasThreads, 0, st>>>(n, (const float2*)V, ld, m, c, (float2*)w, partials);
+    k_multi_axpy<float, float><<<g, kBlasThreads, 0, st>>>(n, (const float2*)V, ld, m, c, (float2*)w, partials, step);
   else if (vprec == MB_PREC_F32)
-    k_multi_axpy<float, double><<<g, kBlasThreads, 0, st>>>(n, (const float2*)V, ld, m, c, (double2*)w, partials);
+    k_multi_axpy<float, double><<<g, kBlasThreads, 0, st>>>(n, (const float2*)V, ld, m, c, (double2*)w, partials, step);
   else if (wprec == MB_PREC_F32)
-    k_multi_axpy<double, float><<<g, kBlasThreads, 0, st>>>(n, (const double2*)V, ld, m, c, (float2*)w, partials);
+    k_multi_axpy<double, float><<<g, kBlasThreads, 0, st>>>(n, (const double2*)V, ld, m, c, (float2*)w, partials, step);
   else
-    k_multi_axpy<double, double><<<g, kBlasThreads, 0, st>>>(n, (const double2*)V, ld, m, c, (double2*)w, partials);
+    k_multi_axpy<double, double><<<g, kBlasThreads, 0, st>>>(n, (const double2*)V, ld, m, c, (double2*)w, partials, step);
   MB_CUDA(cudaGetLastError());
 }
 

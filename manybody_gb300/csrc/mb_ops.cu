@@ -769,6 +769,7 @@ struct Krylov {
   size_t vb;
   DevBuf rot[3];  // rotating vectors, each made on first use
   DevBuf basis, coef, basis_part;
+  unsigned* basis_ticket = nullptr;
   int basis_prec = MB_PREC_F64;
   int64_t basis_cap = 0;
   Reducer red;
@@ -843,7 +844,9 @@ struct Krylov {
     basis_prec = p;
     basis_cap = k;
     basis_part = DevBuf(sizeof(double) * 2 * (size_t)k * (size_t)multi_dot_grid(n));
-    coef = DevBuf(sizeof(double) * 2 * (size_t)std::max<int64_t>(k, 1));
+    coef = DevBuf(sizeof(double) * (2 * (size_t)std::max<int64_t>(k, 1) + 1));
+    basis_ticket = (unsigned*)((double*)coef.p + 2 * (size_t)std::max<int64_t>(k, 1));
+    MB_CUDA(cudaMemsetAsync(basis_ticket, 0, sizeof(unsigned), st));
   }
 
   void* basis_col(int64_t j) {
@@ -899,7 +902,7 @@ struct Krylov {
     for (int64_t j0 = 0; j0 < m; j0 += kKeepChunk) {
       const int cnt = (int)std::min<int64_t>(kKeepChunk, m - j0);
       launch_multi_axpy(prec, prec, n, keep_col(j0), n, cnt, (const double*)keep_coef.p + 2 * j0,
-                        x, red.p(), st);
+                        x, red.p(), KrylovStep{}, st);
     }
   }
 
@@ -913,10 +916,10 @@ struct Krylov {
   double reorth(int m, double nrm2, void* w) {
     for (int pass = 0; pass < 2; ++pass) {
       const double before = nrm2;
-      launch_multi_dot(basis_prec, prec, n, basis.p, n, m, w, (double*)basis_part.p, st);
-      launch_reduce((const double*)basis_part.p, multi_dot_grid(n), 2 * m, (double*)coef.p, st);
+      launch_multi_dot(basis_prec, prec, n, basis.p, n, m, w, (double*)basis_part.p, basis_ticket,
+                       (double*)coef.p, st);
       launch_multi_axpy(basis_prec, prec, n, basis.p, n, m, (const double*)coef.p, w, red.p(),
-                        st);
+                        KrylovStep{}, st);
       nrm2 = red.fetch(grid_blas, 3, st)[1];
       if (nrm2 >= 0.5 * before) break;
     }
@@ -1080,7 +1083,7 @@ struct Krylov {
     MB_CUDA(cudaMemcpyAsync(coef.p, c.data(), sizeof(double) * c.size(), cudaMemcpyHostToDevice, st));
     MB_CUDA(cudaMemsetAsync(x, 0, vb, st));
     launch_multi_axpy(basis_prec, prec, n, basis.p, n, (int)steps, (const double*)coef.p, x,
-                      red.p(), st);
+                      red.p(), KrylovStep{}, st);
     MB_CUDA(cudaStreamSynchronize(st));
   }
 };
@@ -1089,23 +1092,30 @@ struct Krylov {
 // FP64 Rayleigh-Ritz refinement of ground-state estimates, many at once.  A
 // problem is an operator view and a start vector x (complex128, tensor
 // order).  Its Krylov space span{x, Hx, H^2 x, ...} is built with FP64
-// vectors and arithmetic: Lanczos with full re-orthogonalisation (w = H q_j
-// orthogonalised against q_0..q_j by classical Gram-Schmidt, kRefinePasses
-// passes; alpha_j is w's total coefficient on q_j, beta_j the norm of what
-// remains).  Two passes (CGS2): with one, orthogonality decays by about
-// |theta| / beta a step, and a start vector close to an eigenvector of an
-// operator far from zero (beta_0 ~ 1e-5, |E0| ~ 100: 1D L=14 13+13 at U=9.2)
-// lost it within six steps, its lowest Ritz value falling 7 % below E0; the
-// second pass holds it at ~1e-17.  After each step the lowest
-// eigenvalue of T_(j+1) is the estimate; steps continue until it settles to
-// kRefineSettle relative (at least kRefineMinSteps), the space breaks down,
-// or the problem's step budget (kRefineMaxSteps, fewer where the basis would
-// pass kRefineBasisBytes).  The problems advance in lockstep: their kernels
-// queue on kRefineLanes streams and the host waits once per step for all of
-// them.
+// vectors and arithmetic: Lanczos with full re-orthogonalisation.  w = (H -
+// theta_0) q_j, theta_0 the first step's Rayleigh quotient (0 in the first
+// step), is orthogonalised against q_0..q_j by classical Gram-Schmidt; a
+// second pass runs where the first took w below a tenth of its norm
+// (kRefineAgain); alpha_j is theta_0 plus w's total coefficient on q_j, beta_j
+// the norm of what remains.  The shift matters: x is close to an eigenvector
+// of an operator that may be far from zero, H q_j is then almost theta q_j,
+// and one pass without the shift leaves an orthogonality of |theta| / beta
+// times the rounding, worse by that factor every step (1D L=14 13+13 at U=9.2,
+// beta_0 ~ 1e-5, |E0| ~ 100: the lowest Ritz value fell 7 % below E0 within six
+// steps).  Two passes in every step held it too, at twice the FP64 work: 27 of
+// the 65 ms of a 40-step 4x4 5+5 solve were these projections, now 14 of 52.
+// After each step the lowest eigenvalue of T_(j+1) is the estimate; steps
+// continue until it settles to kRefineSettle relative (at least
+// kRefineMinSteps), the space breaks down, or the problem's step budget
+// (kRefineMaxSteps, fewer where the basis would pass kRefineBasisBytes).  The
+// problems advance in lockstep: their kernels queue on kRefineLanes streams and
+// the host waits once per step for all of them (twice where a second pass is
+// due).
 // ---------------------------------------------------------------------------
 namespace {
-constexpr int kRefinePasses = 2;
+// squared norms' ratio below which a projection is repeated: one pass loses the
+// norms' ratio, 10, of its 16 digits at most
+constexpr double kRefineAgain = 0.01;
 constexpr size_t kRefineBasisBytes = (size_t)24 << 30;  // one problem's basis at most
 constexpr size_t kRefineChunkBytes = (size_t)4 << 30;   // bases of problems run together
 
@@ -1115,11 +1125,15 @@ struct RefineRun {
   size_t vb;
   int steps, cap;
   char* q = nullptr;     // cap vectors
-  double* dc = nullptr;  // device: 2 passes x 2 cap coefficients, then 3 reduced norms
+  // device: a pass's 2 cap coefficients, then the dots (Re<x,w>, <w,w>, ...) of
+  // the apply and of the pass
+  double* dc = nullptr;
   double* hc = nullptr;  // host mirror
   std::vector<double> alpha, beta;
   double theta = 0.0;
-  bool done = false;
+  double shift = 0.0, a = 0.0;  // of the running step: theta_0, the coefficient on q_j
+  bool done = false, again = false;
+  size_t words() const { return 2 * (size_t)cap + 6; }
   char* col(int k) const { return q + vb * (size_t)k; }
 };
 }  // namespace
@@ -1131,7 +1145,7 @@ struct RefineSizes {
   int pblocks = 1, pcomps = 3;
   void add(const RefineRun& r) {
     qbytes += r.vb * (size_t)r.cap;
-    cwords += 4 * (size_t)r.cap + 4;
+    cwords += r.words();
     pblocks = std::max({pblocks, apply_grid(r.p->v, MB_PREC_F64), blas_grid(r.n),
                         multi_dot_grid(r.n)});
     pcomps = std::max(pcomps, 2 * r.cap);
@@ -1149,7 +1163,7 @@ struct RefineSizes {
 // kernels and their order are the same as on one stream, so are its bits.
 constexpr int kRefineLanes = 8;
 struct RefineBufs {
-  DevBuf q, c, part;
+  DevBuf q, c, part, tickets;
   size_t pstride = 0;  // doubles of partial sums a lane
   double* host = nullptr;
   cudaStream_t lane[kRefineLanes] = {};
@@ -1158,8 +1172,9 @@ struct RefineBufs {
   RefineBufs(const RefineSizes& z, cudaStream_t st)
       : q(z.qbytes, st), c(sizeof(double) * z.cwords, st),
         part(sizeof(double) * kRefineLanes * (size_t)z.pblocks * z.pcomps, st),
-        pstride((size_t)z.pblocks * z.pcomps), host_bytes(sizeof(double) * z.cwords) {
+        tickets(sizeof(unsigned) * kRefineLanes, st), pstride((size_t)z.pblocks * z.pcomps), host_bytes(sizeof(double) * z.cwords) {
     host = (double*)pinned_take(host_bytes);
+    MB_CUDA(cudaMemsetAsync(tickets.p, 0, sizeof(unsigned) * kRefineLanes, st));
     MB_CUDA(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
     for (int k = 0; k < kRefineLanes; ++k) {
       MB_CUDA(cudaStreamCreateWithFlags(&lane[k], cudaStreamNonBlocking));
@@ -1197,7 +1212,7 @@ static void refine_chunk(std::vector<RefineRun>& runs, RefineBufs& bufs, cudaStr
       r.dc = (double*)cbuf.p + co;
       r.hc = host + co;
       qo += r.vb * (size_t)r.cap;
-      co += 4 * (size_t)r.cap + 4;
+      co += r.words();
     }
   }
   const int nl = std::min<int>(kRefineLanes, (int)runs.size());
@@ -1215,49 +1230,72 @@ static void refine_chunk(std::vector<RefineRun>& runs, RefineBufs& bufs, cudaStr
     MB_CUDA(cudaMemcpyAsync(host, cbuf.p, sizeof(double) * cwords, cudaMemcpyDeviceToHost, st));
     MB_CUDA(cudaStreamSynchronize(st));
   };
-  auto nn_off = [](const RefineRun& r) { return 4 * (size_t)r.cap; };
+  auto step = [&](size_t i, int blocks, size_t at) {
+    KrylovStep s;
+    s.ticket = (unsigned*)bufs.tickets.p + i % kRefineLanes;
+    s.blocks = blocks;
+    s.part = pp(i);
+    s.dots = runs[i].dc + 2 * (size_t)runs[i].cap + at;
+    return s;
+  };
   // q_0 = x / |x|
   for (size_t i = 0; i < runs.size(); ++i) {
     RefineRun& r = runs[i];
     MB_CUDA(cudaMemcpyAsync(r.col(0), r.p->x, r.vb, cudaMemcpyDeviceToDevice, ls(i)));
-    launch_dot(MB_PREC_F64, r.n, r.col(0), r.col(0), pp(i), ls(i));
-    launch_reduce(pp(i), blas_grid(r.n), 3, r.dc + nn_off(r), ls(i));
+    launch_norm2(MB_PREC_F64, r.n, r.col(0), pp(i), ls(i));
+    launch_reduce(pp(i), blas_grid(r.n), 3, r.dc + 2 * (size_t)r.cap, ls(i));
   }
   sync_all();
   for (size_t i = 0; i < runs.size(); ++i) {
     RefineRun& r = runs[i];
-    const double nx = std::sqrt(r.hc[nn_off(r) + 2]);
+    const double nx = std::sqrt(r.hc[2 * (size_t)r.cap + 1]);
     MB_REQUIRE(nx > 0.0, MB_ERR_ZERO_NORM, "refinement start vector has zero norm");
     launch_axpby(MB_PREC_F64, r.n, 1.0 / nx, 0.0, r.col(0), 0.0, 0.0, r.col(0), nullptr, 0, ls(i));
   }
+  // w -= Q Q^H w against q_0..q_j: the coefficients at dc[0..), the norm of
+  // the rest in the second dots
+  auto project = [&](size_t i, int j) {
+    RefineRun& r = runs[i];
+    void* w = r.col(j + 1);
+    launch_multi_dot(MB_PREC_F64, MB_PREC_F64, r.n, r.q, r.n, j + 1, w, pp(i),
+                     (unsigned*)bufs.tickets.p + i % kRefineLanes, r.dc, ls(i));
+    launch_multi_axpy(MB_PREC_F64, MB_PREC_F64, r.n, r.q, r.n, j + 1, r.dc, w, pp(i),
+                      step(i, blas_grid(r.n), 3), ls(i));
+  };
   for (int j = 0;; ++j) {
     bool any = false;
     for (size_t i = 0; i < runs.size(); ++i) {
       RefineRun& r = runs[i];
       if (r.done) continue;
       any = true;
-      // w = H q_j in the next basis slot, then w -= Q Q^H w twice against
-      // q_0..q_j: the passes' coefficients at dc[0..) and dc[2 cap..), the
-      // norm of the rest at dc[4 cap + 1]
-      void* w = r.col(j + 1);
-      launch_apply(r.p->v, MB_PREC_F64, r.col(j), w, 1.0, 0.0, 0.0, nullptr, nullptr, 0, ls(i));
-      for (int pass = 0; pass < kRefinePasses; ++pass) {
-        double* c = r.dc + 2 * (size_t)r.cap * pass;
-        launch_multi_dot(MB_PREC_F64, MB_PREC_F64, r.n, r.q, r.n, j + 1, w, pp(i), ls(i));
-        launch_reduce(pp(i), multi_dot_grid(r.n), 2 * (j + 1), c, ls(i));
-        launch_multi_axpy(MB_PREC_F64, MB_PREC_F64, r.n, r.q, r.n, j + 1, c, w, pp(i), ls(i));
-      }
-      launch_reduce(pp(i), blas_grid(r.n), 3, r.dc + nn_off(r), ls(i));
+      // w = (H - shift) q_j in the next basis slot
+      OpView v = r.p->v;
+      v.step = step(i, apply_grid(v, MB_PREC_F64), 0);
+      launch_apply(v, MB_PREC_F64, r.col(j), r.col(j + 1), 1.0, r.shift, 0.0, nullptr, pp(i), 2,
+                   ls(i));
+      project(i, j);
     }
     if (!any) break;
     sync_all();
+    any = false;
     for (size_t i = 0; i < runs.size(); ++i) {
       RefineRun& r = runs[i];
       if (r.done) continue;
-      double a = 0.0;
-      for (int pass = 0; pass < kRefinePasses; ++pass) a += r.hc[2 * (size_t)r.cap * pass + 2 * j];
-      r.alpha.push_back(a);
-      const double b = std::sqrt(r.hc[nn_off(r) + 1]);
+      const double* dots = r.hc + 2 * (size_t)r.cap;
+      r.a = r.shift + r.hc[2 * j];
+      r.again = dots[4] < kRefineAgain * dots[1];
+      if (!r.again) continue;
+      any = true;
+      project(i, j);
+    }
+    if (any) sync_all();
+    for (size_t i = 0; i < runs.size(); ++i) {
+      RefineRun& r = runs[i];
+      if (r.done) continue;
+      if (r.again) r.a += r.hc[2 * j];
+      r.alpha.push_back(r.a);
+      if (j == 0) r.shift = r.a;
+      const double b = std::sqrt(r.hc[2 * (size_t)r.cap + 4]);
       std::vector<double> d(r.alpha), e(r.beta);
       MB_REQUIRE(tridiag_eig((int)d.size(), d, e, nullptr), MB_ERR_EIG_FAILED,
                  "Eigenvalue decomposition of T_k failed");
