@@ -1459,7 +1459,7 @@ std::shared_ptr<TableSet> get_tables(mb_engine_s* e, const mb_sector_desc& d) {
   ts->max_up_deg = tu.max_degree;
   ts->max_dn_deg = td.max_degree;
   TableSet* tsp = ts.get();
-  fill_fused_tables(ts->fused, tu, td, ts->basis.up.D, ts->basis.down.D,
+  fill_fused_tables(ts->fused, tu, td, ts->basis.up.D, ts->basis.down.D, 16,
                     [tsp](const void* h, size_t bytes) -> const void* {
                       auto b = std::make_unique<EngBuf>(std::max<size_t>(bytes, 16));
                       if (bytes) MB_CUDA(cudaMemcpy(b->p, h, bytes, cudaMemcpyHostToDevice));

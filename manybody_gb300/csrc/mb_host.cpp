@@ -247,38 +247,39 @@ SignedLists signed_lists(const HopTable& t, int64_t D) {
 
 namespace {
 
-// Orders the entries of one quarter warp (8 lanes) over k slots: in each slot
-// a maximum matching of lanes to bank groups (target mod 8), lanes that must
+// Orders the entries of N lanes (one wavefront of a gather) over k slots: in each
+// slot a maximum matching of lanes to bank groups (target mod N), lanes that must
 // take an entry now (as many left as slots) first, entries of the groups with
 // the most entries left preferred (the greedy form of Koenig's edge
 // colouring).  A lane left unmatched takes a padding zero element of a group
 // no entry uses in that slot, or, if it must take an entry, its first one.
-void order_quarter(std::vector<uint32_t> (&lst)[8], int k, uint32_t D, uint32_t* out) {
+template <int N>
+void order_lanes(std::vector<uint32_t>* lst, int k, uint32_t D, uint32_t* out) {
   constexpr uint32_t kIdx = 0x7FFFFFFFu;
   for (int j = 0; j < k; ++j) {
     const int left = k - j;
-    int gdeg[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    for (auto& l : lst)
-      for (uint32_t w : l) ++gdeg[(w & kIdx) & 7u];
-    int order[8];
-    for (int l = 0; l < 8; ++l) order[l] = l;
-    std::stable_sort(order, order + 8, [&](int a, int b) {
+    int gdeg[N] = {};
+    for (int l = 0; l < N; ++l)
+      for (uint32_t w : lst[l]) ++gdeg[(w & kIdx) % N];
+    int order[N];
+    for (int l = 0; l < N; ++l) order[l] = l;
+    std::stable_sort(order, order + N, [&](int a, int b) {
       const bool fa = (int)lst[a].size() >= left, fb = (int)lst[b].size() >= left;
       if (fa != fb) return fa;
       return lst[a].size() > lst[b].size();
     });
-    int match_g[8], pick[8];
-    for (int i = 0; i < 8; ++i) match_g[i] = pick[i] = -1;
+    int match_g[N], pick[N];
+    for (int i = 0; i < N; ++i) match_g[i] = pick[i] = -1;
     // Kuhn's augmenting paths; candidates by descending group degree
     std::function<bool(int, unsigned&)> augment = [&](int l, unsigned& seen) -> bool {
       int cand[64];
       int nc = 0;
       for (int i = 0; i < (int)lst[l].size() && nc < 64; ++i) cand[nc++] = i;
       std::stable_sort(cand, cand + nc, [&](int a, int b) {
-        return gdeg[(lst[l][(size_t)a] & kIdx) & 7u] > gdeg[(lst[l][(size_t)b] & kIdx) & 7u];
+        return gdeg[(lst[l][(size_t)a] & kIdx) % N] > gdeg[(lst[l][(size_t)b] & kIdx) % N];
       });
       for (int ci = 0; ci < nc; ++ci) {
-        const int g = (int)((lst[l][(size_t)cand[ci]] & kIdx) & 7u);
+        const int g = (int)((lst[l][(size_t)cand[ci]] & kIdx) % N);
         if (seen & (1u << g)) continue;
         seen |= 1u << g;
         if (match_g[g] < 0 || augment(match_g[g], seen)) {
@@ -289,29 +290,29 @@ void order_quarter(std::vector<uint32_t> (&lst)[8], int k, uint32_t D, uint32_t*
       }
       return false;
     };
-    for (int oi = 0; oi < 8; ++oi) {
+    for (int oi = 0; oi < N; ++oi) {
       const int l = order[oi];
       if (lst[l].empty()) continue;
       unsigned seen = 0;
       augment(l, seen);
     }
     unsigned used = 0;
-    uint32_t slot[8];
-    bool taken[8] = {false, false, false, false, false, false, false, false};
-    for (int l = 0; l < 8; ++l) {
+    uint32_t slot[N];
+    bool taken[N] = {};
+    for (int l = 0; l < N; ++l) {
       if (pick[l] < 0 && !lst[l].empty() && (int)lst[l].size() >= left) pick[l] = 0;
       if (pick[l] >= 0) {
         slot[l] = lst[l][(size_t)pick[l]];
-        used |= 1u << ((slot[l] & kIdx) & 7u);
+        used |= 1u << ((slot[l] & kIdx) % N);
         taken[l] = true;
       }
     }
     // one padding element for every unmatched lane (same address: a broadcast)
     int pg = 0;
-    while (pg < 8 && (used & (1u << pg))) ++pg;
-    if (pg == 8) pg = 0;
-    const uint32_t pad = D + ((uint32_t)pg + 8u - (D & 7u)) % 8u;
-    for (int l = 0; l < 8; ++l) {
+    while (pg < N && (used & (1u << pg))) ++pg;
+    if (pg == N) pg = 0;
+    const uint32_t pad = D + ((uint32_t)pg + N - D % N) % N;
+    for (int l = 0; l < N; ++l) {
       if (taken[l]) {
         lst[l].erase(lst[l].begin() + pick[l]);
       } else {
@@ -324,40 +325,51 @@ void order_quarter(std::vector<uint32_t> (&lst)[8], int k, uint32_t D, uint32_t*
 
 }  // namespace
 
-SlicedTable sliced_table(const HopTable& t, int64_t D) {
+SlicedTable sliced_table(const HopTable& t, int64_t D, int lanes) {
   MB_REQUIRE(D + kSlicedPads < (int64_t(1) << 27), MB_ERR_CAPACITY,
              "sector too large for the sliced table");
   SlicedTable s;
   const int64_t ng = (D + 31) / 32;
   s.grp.resize((size_t)(2 * ng));
   s.nneg.assign((size_t)D, 0);
-  std::vector<uint32_t> lst[4][8];
-  std::vector<uint32_t> slots;
+  // the groups' slots and places first, then the groups independently
+  size_t total = 0;
   for (int64_t g = 0; g < ng; ++g) {
     int k = 0;
+    for (int64_t c = 32 * g; c < std::min<int64_t>(D, 32 * g + 32); ++c) {
+      int n = 0;
+      for (int32_t j = t.off[(size_t)c]; j < t.off[(size_t)c + 1]; ++j)
+        n += (t.ent[(size_t)j] & 2u) ? 2 : 1;
+      k = std::max(k, n);
+    }
+    s.grp[(size_t)(2 * g)] = (int32_t)total;
+    s.grp[(size_t)(2 * g + 1)] = k;
+    total += (size_t)32 * ((k + 3) & ~3);
+    MB_REQUIRE(total < (size_t)INT32_MAX, MB_ERR_CAPACITY, "hop table too large");
+  }
+  s.ent.assign(total, (uint32_t)D);
+#pragma omp parallel for schedule(dynamic, 2) if (ng >= 8)
+  for (int64_t g = 0; g < ng; ++g) {
+    const size_t base = (size_t)s.grp[(size_t)(2 * g)];
+    const int k = s.grp[(size_t)(2 * g + 1)];
+    std::vector<uint32_t> lst[32];
     for (int l = 0; l < 32; ++l) {
-      auto& col = lst[l >> 3][l & 7];
-      col.clear();
       const int64_t c = 32 * g + l;
       if (c >= D) continue;
       for (int32_t j = t.off[(size_t)c]; j < t.off[(size_t)c + 1]; ++j) {
         const uint32_t e = t.ent[(size_t)j];
         const uint32_t w = (e >> 8) | ((e & 1u) << 31);
-        col.push_back(w);
-        if (e & 2u) col.push_back(w);
+        lst[l].push_back(w);
+        if (e & 2u) lst[l].push_back(w);
         s.nneg[(size_t)c] += (uint8_t)((e & 1u) * ((e & 2u) ? 2 : 1));
       }
-      k = std::max(k, (int)col.size());
     }
-    const size_t base = s.ent.size();
-    const int k4 = (k + 3) & ~3;
-    MB_REQUIRE(base + (size_t)32 * k4 < (size_t)INT32_MAX, MB_ERR_CAPACITY, "hop table too large");
-    s.grp[(size_t)(2 * g)] = (int32_t)base;
-    s.grp[(size_t)(2 * g + 1)] = k;
-    slots.assign((size_t)32 * k, (uint32_t)D);
-    for (int q = 0; q < 4; ++q) order_quarter(lst[q], k, (uint32_t)D, slots.data() + 8 * q);
+    std::vector<uint32_t> slots((size_t)32 * k, (uint32_t)D);
+    for (int l = 0; l < 32; l += lanes) {
+      if (lanes == 16) order_lanes<16>(lst + l, k, (uint32_t)D, slots.data() + l);
+      else order_lanes<8>(lst + l, k, (uint32_t)D, slots.data() + l);
+    }
     // slots 4i..4i+3 of a lane are one 16-byte word; the last word is padded
-    s.ent.resize(base + (size_t)32 * k4, (uint32_t)D);
     for (int j = 0; j < k; ++j)
       for (int l = 0; l < 32; ++l)
         s.ent[base + 128 * (size_t)(j >> 2) + 4 * (size_t)l + (size_t)(j & 3)] =
@@ -437,7 +449,7 @@ int ritz_vector_steps(const std::vector<double>& a, const std::vector<double>& b
 }
 
 void fill_fused_tables(OpView& v, const HopTable& tu, const HopTable& td, int64_t Du, int64_t Dd,
-                       const TableUpload& upload) {
+                       int lanes, const TableUpload& upload) {
   auto put = [&](const auto& vec) {
     using T = typename std::decay_t<decltype(vec)>::value_type;
     return (const T*)upload(vec.data(), sizeof(T) * vec.size());
@@ -449,7 +461,7 @@ void fill_fused_tables(OpView& v, const HopTable& tu, const HopTable& td, int64_
   v.up_loff = put(ul.off);
   v.up_lpos = put(ul.pos);
   v.max_up_list = ul.max_len;
-  const SlicedTable sd = sliced_table(td, Dd);
+  const SlicedTable sd = sliced_table(td, Dd, lanes);
   v.dn_sell = put(sd.ent);
   v.dn_sgrp = put(sd.grp);
   v.dn_nneg = put(sd.nneg);
@@ -465,7 +477,7 @@ void fill_fused_tables(OpView& v, const HopTable& tu, const HopTable& td, int64_
     v.up_sell16 = v.dn_sell16;
     v.up_sgrp16 = v.dn_sgrp16;
   } else {
-    const SlicedTable su = sliced_table(tu, Du);
+    const SlicedTable su = sliced_table(tu, Du, lanes);
     v.up_sell = put(su.ent);
     v.up_sgrp = put(su.grp);
     v.up_nneg = put(su.nneg);

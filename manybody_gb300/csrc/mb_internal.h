@@ -265,11 +265,13 @@ SignedLists signed_lists(const HopTable& t, int64_t D);
 // of kSlicedPads zero elements past the row); grp[2g+1] = slots of group g,
 // stored rounded up to a multiple of 4 with padding.
 // Within a group each lane's entries are ordered (the hop sum does not
-// depend on the order) so that in every slot the eight lanes of a quarter
-// warp read distinct 16-byte shared-memory bank groups (index mod 8): a
-// warp's 16-byte gather from the staged row then takes 4 wavefronts, not
-// the ~8 of the hop order.  Padding takes a zero element in a free group.
-constexpr int kSlicedPads = 8;
+// depend on the order) so that in every slot the `lanes` lanes that share a
+// wavefront read distinct shared-memory bank groups (index mod lanes): 8 lanes
+// for 16-byte elements, whose gather from the staged row then takes 4
+// wavefronts, not the ~8 of the hop order; 16 for 8-byte elements (2
+// wavefronts, ~3.5 in the order for 8).  Padding takes a zero element in a
+// free group.
+constexpr int kSlicedPads = 16;
 
 #ifdef __CUDACC__
 // Apply shape prefetch = 1: before its down hops, a warp asks L2 for the
@@ -295,7 +297,7 @@ struct SlicedTable {
   std::vector<int32_t> grp;
   std::vector<uint8_t> nneg;  // [D] negative entries per state
 };
-SlicedTable sliced_table(const HopTable& t, int64_t D);
+SlicedTable sliced_table(const HopTable& t, int64_t D, int lanes = 8);
 // 1 + ceil(log2(terms)), at least 6: the bits an integer sum (mb_isum.h) of that
 // many terms keeps free above its largest term, sign included.
 // Up to kISumBaseMax a sum keeps its largest term's whole significand (512
@@ -468,7 +470,7 @@ int eng_fused_blocks(const OpView& v);
 
 using TableUpload = std::function<const void*(const void* host, size_t bytes)>;
 void fill_fused_tables(OpView& v, const HopTable& tu, const HopTable& td, int64_t Du, int64_t Dd,
-                       const TableUpload& upload);
+                       int lanes, const TableUpload& upload);
 
 }  // namespace mb
 

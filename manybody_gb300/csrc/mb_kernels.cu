@@ -210,6 +210,14 @@ static int max_smem_optin() {
 // memory.  Warp w takes the 32-column groups w, w + nwarps, ... (with
 // up_prefetch set it asks L2 for the group's up-hop lines before its down hops).
 //
+// complex64: by the counters (4x4 5+5) the L1 data path was 83 % busy with
+// shared-memory and global wavefronts (162 a group of 32 columns), nothing else
+// above half.  Its sliced table is ordered for 8-byte elements now (2
+// wavefronts a slot instead of ~3.5), the up list is read four entries at a
+// time, whose neighbours are loaded together and added or subtracted without a
+// sign each: 123 wavefronts; 5+5 417 -> 314 us, 6+6 1.44 -> 1.18 ms, 3x4 6+6 26 ->
+// 20.6 us, 1D L=14 7+7 165 -> 149.  Issue (68 %) and waits for L2 are next.
+//
 // complex128: the hop sums run on the integer pipes (mb_isum.h), the FP64 pipe
 // converts them and does the diagonal, the affine part and the dots.  A staged
 // row is decoded once (each element is a down neighbour about 16 times), up
@@ -219,11 +227,13 @@ static int max_smem_optin() {
 // 5+5) the ALU pipe is now 65 % busy, the FP64 pipe 38 %, issue 64 %, and the
 // largest stall is waiting for L2 (3.8 of 10.7 warps a scheduler).
 // ---------------------------------------------------------------------------
-constexpr int kApplyThreads = 1024;
-// CTAs per SM: complex64 rows are half the size, and two CTAs per SM (32
-// registers a thread) beat one with 64 registers (measured 2.03 -> 1.75 ms at
-// 4x4 6+6, 3.41 -> 2.98 ms at 1D L=16 8+8); complex128 keeps one.
-template <typename T> constexpr int kApplyCtasPerSm = sizeof(T) == 4 ? 2 : 1;
+// Most threads of a CTA, and the threads an SM holds: 64 registers a thread for
+// complex128; complex64 rows are half the size and 2,048 threads of 32 registers
+// beat 1,536 of 42 (4x4 6+6 1.18 against 1.28 ms, 5+5 314 against 335 us; 1D L=14
+// 7+7 149 against 141).
+template <typename T> constexpr int kApplyMax = 1024;
+template <typename T> constexpr int kApplyResident = sizeof(T) == 4 ? 2048 : 1024;
+template <typename T> constexpr int kApplyCtasPerSm = kApplyResident<T> / kApplyMax<T>;
 
 // +-1 from the sign bit of a table entry
 __device__ __forceinline__ double unit_sign(uint32_t e, double) {
@@ -245,8 +255,9 @@ __device__ __forceinline__ void apply_rows(
   extern __shared__ __align__(16) unsigned char smem[];
   const int64_t Dd = v.Dd;
   const uint32_t row_bytes = (uint32_t)(sizeof(V2) * Dd);
-  uint32_t* s_up =
-      reinterpret_cast<uint32_t*>(smem + (STAGED ? row_bytes + sizeof(V2) * kSlicedPads : 0));
+  // (the list is read four entries at a time: 16-byte aligned, see apply_smem)
+  uint32_t* s_up = reinterpret_cast<uint32_t*>(
+      smem + (STAGED ? (row_bytes + sizeof(V2) * kSlicedPads + 15u) & ~size_t(15) : 0));
   // a staged complex128 row is kept decoded; s_wide[row parity]: it holds a
   // value that does not fit there
   __shared__ int s_wide[2];
@@ -269,8 +280,7 @@ __device__ __forceinline__ void apply_rows(
     __syncthreads();
     const int u0 = __ldg(&v.up_loff[r]), nu = __ldg(&v.up_loff[r + 1]) - u0;
     const int npos = __ldg(&v.up_lpos[r]);
-    // complex128: the sign in bit 31
-    for (int j = threadIdx.x; j < nu; j += blockDim.x)
+    for (int j = threadIdx.x; j < nu; j += blockDim.x)  // complex128: the sign in bit 31
       s_up[j] = __ldg(&v.up_list[u0 + j]) | (kInt && j >= npos ? 0x80000000u : 0u);
     if (STAGED) {
       if constexpr (kInt) {
@@ -303,8 +313,8 @@ __device__ __forceinline__ void apply_rows(
       const char* xc = reinterpret_cast<const char*>(x + cl);
       // an up neighbour by its list entry
       auto up = [&](uint32_t e) -> V2 {
-        const uint64_t r2 = kInt ? e & 0x7FFFFFFFu : e;
-        return __ldg(reinterpret_cast<const V2*>(xc + r2 * row_bytes));
+        if (kInt) e &= 0x7FFFFFFFu;
+        return __ldg(reinterpret_cast<const V2*>(xc + (uint64_t)e * row_bytes));
       };
       // a down neighbour by table entry, in place or from global memory (the
       // sign bit shifts out)
@@ -334,17 +344,31 @@ __device__ __forceinline__ void apply_rows(
           hop(e.z, dn(e.z));
           hop(e.w, dn(e.w));
         }
-#pragma unroll 4
-        for (int j = 0; j < npos; ++j) {
-          const V2 val = up(s_up[j]);
-          ar += val.x;
-          ai += val.y;
-        }
-#pragma unroll 4
-        for (int j = npos; j < nu; ++j) {
-          const V2 val = up(s_up[j]);
-          ar -= val.x;
-          ai -= val.y;
+        // four list entries per 16-byte load, all four neighbours in flight:
+        // added, subtracted, or (where the signs change) either
+        const uint4* up4 = reinterpret_cast<const uint4*>(s_up);
+        V2 zero;
+        zero.x = T(0);
+        zero.y = T(0);
+#pragma unroll 2
+        for (int j = 0; j < nu; j += 4) {
+          const uint4 e = up4[j >> 2];
+          const V2 v0 = up(e.x);
+          const V2 v1 = j + 1 < nu ? up(e.y) : zero;
+          const V2 v2 = j + 2 < nu ? up(e.z) : zero;
+          const V2 v3 = j + 3 < nu ? up(e.w) : zero;
+          if (j + 4 <= npos) {
+            ar += (v0.x + v1.x) + (v2.x + v3.x);
+            ai += (v0.y + v1.y) + (v2.y + v3.y);
+          } else if (j >= npos) {
+            ar -= (v0.x + v1.x) + (v2.x + v3.x);
+            ai -= (v0.y + v1.y) + (v2.y + v3.y);
+          } else {  // v0 is positive
+            const T w1 = j + 1 < npos ? T(1) : T(-1), w2 = j + 2 < npos ? T(1) : T(-1),
+                    w3 = j + 3 < npos ? T(1) : T(-1);
+            ar = fma(w3, v3.x, fma(w2, v2.x, fma(w1, v1.x, ar + v0.x)));
+            ai = fma(w3, v3.y, fma(w2, v2.y, fma(w1, v1.y, ai + v0.y)));
+          }
         }
       };
       if constexpr (kInt) {
@@ -443,7 +467,7 @@ __device__ __forceinline__ void apply_rows(
 }
 
 template <typename T, bool STAGED, int DOTS>
-__global__ void __launch_bounds__(kApplyThreads, kApplyCtasPerSm<T>)
+__global__ void __launch_bounds__(kApplyMax<T>, kApplyCtasPerSm<T>)
 k_apply(OpView v, const typename C2<T>::type* __restrict__ x, typename C2<T>::type* y,
         T hop_coef, T dscale, T shift, T beta, const typename C2<T>::type* z,
         const T* __restrict__ ufold, const T* __restrict__ self_up, const T* __restrict__ self_dn,
@@ -467,7 +491,7 @@ k_apply(OpView v, const typename C2<T>::type* __restrict__ x, typename C2<T>::ty
 // Chebyshev: w = c (H - b) v - [k > 0] T_{k-1}, c = (k ? 2 : 1) / a.
 // Block partials (Re<v,w>, <w,w>) go to a.scratch.
 template <bool STAGED>
-__global__ void __launch_bounds__(kApplyThreads, kApplyCtasPerSm<float>)
+__global__ void __launch_bounds__(kApplyMax<float>, kApplyCtasPerSm<float>)
 k_eng_fused(OpView v, EngFusedArgs a) {
   const int k = *a.k, mode = *a.mode;
   float sc, shift = 0.f, beta = 0.f;
@@ -502,7 +526,7 @@ __global__ void k_eng_fused_place(EngFusedArgs a, int nblocks) {
 static size_t apply_smem(const OpView& v, int precision, bool staged) {
   const int up_words = (v.max_up_list + 3) & ~3;
   size_t s = sizeof(uint32_t) * (size_t)up_words;
-  if (staged) s += elem_bytes(precision) * (size_t)(v.Dd + kSlicedPads);
+  if (staged) s += (elem_bytes(precision) * (size_t)(v.Dd + kSlicedPads) + 15) & ~size_t(15);
   return s;
 }
 
@@ -511,23 +535,26 @@ static bool apply_staged(const OpView& v, int precision) {
 }
 
 // Threads of an apply's CTAs and how many of them an SM holds: together
-// kApplyThreads (twice that for complex64, see kApplyCtasPerSm).  Several small
+// kApplyResident, or fewer where the rows' shared memory ends it.  Several small
 // CTAs, where their rows fit in shared memory side by side, hide each other's
 // staging and barriers, and leave fewer warps without a column group in a row's
 // last round: complex128 4x4 4+4 (1,820 columns) 219 -> 197 us, 3x4 5+4 (495)
-// 41 -> 29 us with 256 threads against 1024; complex64 4x4 5+5 (4,368) 417 ->
-// 391 us with 512, rows of up to 32 groups best with 256 (3x4 6+6: 26 -> 23 us),
-// longer ones with 512 (4x4 4+4: 64 against 68 us).  128 threads were slower
-// everywhere but on 1,001 columns.
+// 41 -> 29 us with 256 threads against 1024; complex64 4x4 5+5 (4,368) 333 -> 314
+// us with 512, rows of up to 32 groups best with 256 (3x4 6+6: 22.6 -> 20.6 us),
+// longer ones with 512 (4x4 4+4: 55.6 against 59 with 256).  128 threads were
+// slower everywhere but on 1,001 columns.
 struct ApplyCtas {
   int threads, per_sm;
 };
 static ApplyCtas apply_ctas(const OpView& v, int precision) {
-  const int total = kApplyThreads * (precision == MB_PREC_F32 ? kApplyCtasPerSm<float> : 1);
+  const bool f32 = precision == MB_PREC_F32;
+  const int most = f32 ? kApplyMax<float> : kApplyMax<double>;
+  const int total = f32 ? kApplyResident<float> : kApplyResident<double>;
   const size_t row = apply_smem(v, precision, apply_staged(v, precision)) + 3072;
   const size_t sm = (size_t)max_smem_optin() + 1024;
-  int threads = precision == MB_PREC_F32 && v.Dd > 32 * 32 ? 512 : 256;
-  while (threads < kApplyThreads && (size_t)(total / threads) * row > sm) threads *= 2;
+  int threads = f32 && v.Dd > 32 * 32 ? 512 : 256;
+  while (threads < most && (size_t)(total / threads) * row > sm)
+    threads = std::min(2 * threads, most);
   return {threads, total / threads};
 }
 

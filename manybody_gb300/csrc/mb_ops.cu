@@ -151,7 +151,7 @@ static void build_op(mb_op_s* op, const mb_basis_s* b, const mb_model_s* m) {
   }
   v.max_up_degree = tu.max_degree;
   v.max_dn_degree = td.max_degree;
-  fill_fused_tables(v, tu, td, op->Du, op->Dd, [op](const void* h, size_t bytes) -> const void* {
+  fill_fused_tables(v, tu, td, op->Du, op->Dd, op->precision == MB_PREC_F32 ? 16 : 8, [op](const void* h, size_t bytes) -> const void* {
     void* p = nullptr;
     MB_CUDA(dev_malloc((void**)&p, std::max<size_t>(bytes, 16)));
     op->allocations.push_back(p);
