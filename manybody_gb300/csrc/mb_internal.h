@@ -349,6 +349,10 @@ struct KrylovStep {
 // Cuthill-McKee order L2 wrote them back half filled: 4x4 6+6 complex128 4.82
 // against 4.71 ms, 1D L=16 8+8 10.6 against 9.5, complex64 6.6 against 5.1).
 constexpr int kRefOut = 8;
+// With kRefOut, x and z are in the reference order too (floating-point lattice
+// applies): element i is x[out_perm[i]], and the whole call is one launch.  The
+// kernel must not read what it has written: y apart from x (see one_launch).
+constexpr int kRefIn = 16;
 
 // Device-side view of an operator (POD; passed to kernels by value).
 struct OpView {
@@ -686,6 +690,17 @@ constexpr int64_t kTileBytes = 100000000;
 inline bool writes_reference(int precision, int64_t dim) {
   return precision == MB_PREC_F64 ||
          (precision == MB_PREC_F32 ? 8 : 16) * dim < 2 * kTileBytes;
+}
+// Whether a reference-order call of a floating-point lattice operator is one
+// launch (kRefIn).  Every read of x then goes through the permutation, two loads
+// one after the other, so it pays where the launches and the moves are most of
+// the time: apply and affine calls, us, against moves around the apply:
+// complex128 1D L=8 4+4 9.0, 10.1 / 10.5, 16.4; 12 sites 4+4 18.8, 19.8 / 20.5,
+// 24.6; 4x4 3+3 (313600) 28.3, 28.7 / 28.9, 35.5; 3x4 5+4 (392040) 38.9, 39.0 /
+// 34.9, 41.2; complex64 14 sites 3+3 (132496) 10.2, 10.3 / 12.3, 16.4; 12 sites
+// 4+4 (245025) 14.4, 14.4 / 12.9, 18.4.
+inline bool one_launch(int precision, int64_t dim) {
+  return dim <= (precision == MB_PREC_F64 ? 300000 : 180000);
 }
 // dst = src in tensor order / in reference order, a lattice operator's vectors
 void launch_to_tensor(int precision, const RowOrder& o, const void* src, void* dst,

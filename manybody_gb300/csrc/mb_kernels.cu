@@ -276,7 +276,11 @@ __device__ __forceinline__ void apply_rows(
 
   for (int64_t ri = blockIdx.x; ri < v.Du; ri += gridDim.x, parity ^= 1) {
     const int64_t r = v.row_sched ? (int64_t)v.row_sched[ri] : ri;
-    const V2* xrow = x + r * Dd;
+    const int64_t row0 = r * Dd;
+    // tensor element i of x
+    auto x_at = [&](int64_t i) -> V2 {
+      return __ldg(x + (DOTS & kRefIn ? (int64_t)__ldg(v.out_perm + i) : i));
+    };
     __syncthreads();
     const int u0 = __ldg(&v.up_loff[r]), nu = __ldg(&v.up_loff[r + 1]) - u0;
     const int npos = __ldg(&v.up_lpos[r]);
@@ -286,7 +290,7 @@ __device__ __forceinline__ void apply_rows(
       if constexpr (kInt) {
         bool wide = false;
         for (int64_t c = threadIdx.x; c < Dd; c += blockDim.x) {
-          const V2 val = xrow[c];
+          const V2 val = x_at(row0 + c);
           reinterpret_cast<longlong2*>(smem)[c] =
               make_longlong2(isum_pack(val.x, &wide), isum_pack(val.y, &wide));
         }
@@ -294,7 +298,7 @@ __device__ __forceinline__ void apply_rows(
         if (threadIdx.x == 0) s_wide[parity ^ 1] = 0;  // read before the last barrier
       } else {
         for (int64_t c = threadIdx.x; c < Dd; c += blockDim.x)
-          reinterpret_cast<V2*>(smem)[c] = xrow[c];
+          reinterpret_cast<V2*>(smem)[c] = x_at(row0 + c);
       }
     }
     __syncthreads();
@@ -314,14 +318,14 @@ __device__ __forceinline__ void apply_rows(
       // an up neighbour by its list entry
       auto up = [&](uint32_t e) -> V2 {
         if (kInt) e &= 0x7FFFFFFFu;
+        if (DOTS & kRefIn) return x_at((int64_t)e * Dd + cl);
         return __ldg(reinterpret_cast<const V2*>(xc + (uint64_t)e * row_bytes));
       };
       // a down neighbour by table entry, in place or from global memory (the
       // sign bit shifts out)
       auto dn_far = [&](uint32_t e) -> V2 {
-        const uint32_t off = e << kShift;
-        if (off < row_bytes)
-          return __ldg(reinterpret_cast<const V2*>(reinterpret_cast<const char*>(xrow) + off));
+        const uint32_t i = e & 0x7FFFFFFFu;
+        if (i < (uint32_t)Dd) return x_at(row0 + i);
         V2 zero;
         zero.x = T(0);
         zero.y = T(0);
@@ -437,7 +441,7 @@ __device__ __forceinline__ void apply_rows(
         fp_hops();
       }
       if (!live) continue;
-      const V2 xv = STAGED && !kInt ? reinterpret_cast<const V2*>(smem)[c] : xrow[c];
+      const V2 xv = STAGED && !kInt ? reinterpret_cast<const V2*>(smem)[c] : x_at(row0 + c);
       T dv = ufold[__popc(um & v.dn_mask[c])] + su;
       if (self_dn) dv += self_dn[c];
       // (coefficients from shared memory, where given, only now: registers)
@@ -447,14 +451,15 @@ __device__ __forceinline__ void apply_rows(
       V2 out;
       out.x = fma(hc, ar, ds * xv.x);
       out.y = fma(hc, ai, ds * xv.y);
-      const int64_t idx = r * Dd + c;
+      const int64_t idx = row0 + c;
+      const int64_t out_idx = DOTS & kRefOut ? (int64_t)__ldcs(v.out_perm + idx) : idx;
       if (z) {
-        const V2 zv = z[idx];
+        const V2 zv = z[DOTS & kRefIn ? out_idx : idx];
         const T be = given ? s_coef[2] : beta;
         out.x = fma(be, zv.x, out.x);
         out.y = fma(be, zv.y, out.y);
       }
-      y[DOTS & kRefOut ? (int64_t)__ldcs(v.out_perm + idx) : idx] = out;
+      y[out_idx] = out;
       if (DOTS & 1) { a_xy.add_prod(xv.x, out.x); a_xy.add_prod(xv.y, out.y); }
       if (DOTS & 2) { a_yy.add_prod(out.x, out.x); a_yy.add_prod(out.y, out.y); }
       if (DOTS & 4) { a_xx.add_prod(xv.x, xv.x); a_xx.add_prod(xv.y, xv.y); }
@@ -599,6 +604,9 @@ static void apply_dots(const OpView& v, const void* x, void* y, double scale, do
     case 3: apply_t<T, STAGED, 3>(v, x, y, scale, shift, beta, z, partials, st); break;
     case 5: apply_t<T, STAGED, 5>(v, x, y, scale, shift, beta, z, partials, st); break;
     case kRefOut: apply_t<T, STAGED, kRefOut>(v, x, y, scale, shift, beta, z, partials, st); break;
+    case kRefOut | kRefIn:
+      apply_t<T, STAGED, kRefOut | kRefIn>(v, x, y, scale, shift, beta, z, partials, st);
+      break;
     default: apply_t<T, STAGED, 7>(v, x, y, scale, shift, beta, z, partials, st); break;
   }
 }

@@ -720,6 +720,11 @@ static void check_order(int order) {
              "order must be MB_ORDER_REFERENCE or MB_ORDER_TENSOR");
 }
 
+// Whether vectors a and b of n bytes share none of them.
+static bool apart(const void* a, const void* b, size_t n) {
+  return (const char*)a + n <= (const char*)b || (const char*)b + n <= (const char*)a;
+}
+
 // y = scale*(H - shift) x + beta z in `order`.
 static void apply_affine(mb_op_s* op, const void* x, void* y, double scale, double shift,
                          double beta, const void* z, int order, cudaStream_t st) {
@@ -738,6 +743,16 @@ static void apply_affine(mb_op_s* op, const void* x, void* y, double scale, doub
   }
   const bool lattice = !op->natural_order && !op->view.n_blocks && !op->view.csr_row;
   const bool fused = lattice && writes_reference(op->precision, op->dim);
+  const size_t bytes = elem_bytes(op->precision) * (size_t)op->dim;
+  // z may be y: each of its elements is read before the same one of y is written
+  if (lattice && one_launch(op->precision, op->dim) && apart(x, y, bytes) &&
+      (beta == 0.0 || z == y || apart(z, y, bytes))) {
+    OpView v = op->view;
+    v.out_perm = op_perm(op);
+    launch_apply(v, op->precision, x, y, scale, shift, beta, beta != 0.0 ? z : nullptr, nullptr,
+                 kRefOut | kRefIn, st);
+    return;
+  }
   auto& s = scratch_for(op, st, fused && beta == 0.0 ? 1 : 2);
   to_tensor(op, x, s.a, order, st);
   const void* zt = nullptr;
