@@ -85,6 +85,48 @@ constexpr int kModeLanczos = kEngLanczos;
 constexpr int kModeReplay = kEngReplay;
 constexpr int kModeCheb = kEngCheb;   // T_{k+1} = 2 Ht T_k - T_{k-1} (T_1 = Ht T_0)
 
+// A warp's sum of compensated float pairs, in lane 0, the tree in pairs too (the
+// error of a step is past the pairs' last bit, 2^-48): an FP64 add takes 17
+// cycles of the SM's one slow pipe for every warp, and a row's sums in FP64 (16
+// instructions in each of its 8 warps) were half of a step's apply.
+__device__ __forceinline__ float2 eng_warp_sum(float hi, float lo) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const float h = __shfl_down_sync(0xffffffffu, hi, o);
+    const float l = __shfl_down_sync(0xffffffffu, lo, o);
+    const float s = hi + h, b = s - hi;
+    lo += ((hi - (s - b)) + (h - b)) + l;
+    hi = s;
+  }
+  return make_float2(hi, lo);
+}
+__device__ __forceinline__ double eng_pair(float2 a) { return (double)a.x + (double)a.y; }
+
+// The block's sums of its warps' pairs into part and (TWO) part2, in a fixed tree.
+constexpr int kEngRowWarps = 8;
+template <bool TWO>
+__device__ __forceinline__ void eng_row_sums(float2 xy, float2 yy, float2 (*red)[2], double* part,
+                                             double* part2) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (lane == 0) {
+    red[warp][0] = xy;
+    if (TWO) red[warp][1] = yy;
+  }
+  __syncthreads();
+  if (warp != 0) return;
+  double a = lane < kEngRowWarps ? eng_pair(red[lane][0]) : 0.0, b = 0.0;
+  if (TWO && lane < kEngRowWarps) b = eng_pair(red[lane][1]);
+#pragma unroll
+  for (int o = kEngRowWarps / 2; o > 0; o >>= 1) {
+    a += __shfl_down_sync(0xffffffffu, a, o);
+    if (TWO) b += __shfl_down_sync(0xffffffffu, b, o);
+  }
+  if (lane == 0) {
+    *part = a;
+    *part2 = b;
+  }
+}
+
 // ---------------------------------------------------------------------------
 // Kernels.  One warp per (slot, row) item; lanes stride over the row.
 // ---------------------------------------------------------------------------
@@ -175,13 +217,8 @@ k_eng_apply(const SlotDesc* __restrict__ slots, const int2* __restrict__ items, 
           hi2 = s1;
         }
       }
-      dxy = (double)hi + (double)lo;
-      dyy = (double)hi2 + (double)lo2;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        dxy += __shfl_down_sync(0xffffffffu, dxy, o);
-        dyy += __shfl_down_sync(0xffffffffu, dyy, o);
-      }
+      dxy = eng_pair(eng_warp_sum(hi, lo));
+      if (cheb) dyy = eng_pair(eng_warp_sum(hi2, lo2));
     }
     if (lane == 0 && part) {
       part[s.item0 + item.y] = dxy;
@@ -197,7 +234,6 @@ k_eng_apply(const SlotDesc* __restrict__ slots, const int2* __restrict__ items, 
 // slots per 16-byte load), up hops are coalesced loads of the listed rows,
 // added then subtracted; the step arithmetic and compensated partials of
 // k_eng_apply.
-constexpr int kEngRowWarps = 8;
 constexpr int64_t kEngRowMinCols = 256;  // rows this wide and wider
 
 __global__ void __launch_bounds__(kEngRowWarps * 32)
@@ -206,7 +242,7 @@ k_eng_apply_rows(const SlotDesc* __restrict__ slots, const int2* __restrict__ it
   extern __shared__ __align__(16) unsigned char smem[];
   float2* srow = reinterpret_cast<float2*>(smem);
   uint32_t* s_up = reinterpret_cast<uint32_t*>(smem + sizeof(float2) * (max_cols + kSlicedPads));
-  __shared__ double red[kEngRowWarps][2];
+  __shared__ float2 red[kEngRowWarps][2];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (int it = blockIdx.x; it < n_items; it += gridDim.x) {
     const int2 item = items[it];
@@ -322,26 +358,9 @@ k_eng_apply_rows(const SlotDesc* __restrict__ slots, const int2* __restrict__ it
         hi2 = s1;
       }
     }
-    double dxy = (double)hi + (double)lo, dyy = (double)hi2 + (double)lo2;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      dxy += __shfl_down_sync(0xffffffffu, dxy, o);
-      dyy += __shfl_down_sync(0xffffffffu, dyy, o);
-    }
-    if (lane == 0) {
-      red[warp][0] = dxy;
-      red[warp][1] = dyy;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {  // fixed order over the warps
-      double a = 0.0, b = 0.0;
-      for (int q = 0; q < kEngRowWarps; ++q) {
-        a += red[q][0];
-        b += red[q][1];
-      }
-      part[pidx] = a;
-      part2[pidx] = b;
-    }
+    const float2 xy = eng_warp_sum(hi, lo);
+    if (cheb) eng_row_sums<true>(xy, eng_warp_sum(hi2, lo2), red, part + pidx, part2 + pidx);
+    else eng_row_sums<false>(xy, xy, red, part + pidx, part2 + pidx);
   }
 }
 
@@ -416,9 +435,7 @@ k_eng_update(const SlotDesc* __restrict__ slots, const int2* __restrict__ items,
         lo += ((hi - (s1 - bp)) + (p - bp)) + pe;
         hi = s1;
       }
-      nn = (double)hi + (double)lo;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) nn += __shfl_down_sync(0xffffffffu, nn, o);
+      nn = eng_pair(eng_warp_sum(hi, lo));
     }
     if (lane == 0) part[it] = nn;
   }
@@ -710,7 +727,7 @@ struct EngPersistArgs {
   long long budget;        // clock64 cycles one barrier wait may take
 };
 
-constexpr int kEngPWarps = 8;             // 256 threads: the reductions' width
+constexpr int kEngPWarps = kEngRowWarps;  // 256 threads: the reductions' width
 constexpr int kEngWarpRowCols = 256;      // widest row of the warp-per-row items
 
 __device__ __forceinline__ unsigned eng_ld_acquire(const unsigned* p) {
@@ -806,15 +823,16 @@ __device__ __forceinline__ float2 lz(float2 a, float f) {
 }
 
 // Phase A, one staged row (block-level): the arithmetic of k_eng_apply_rows.
+template <bool CHEB>
 __device__ void p_apply_row(const SlotDesc& s, const SlotNow& n, int64_t r, int64_t pidx,
                             double* part, double* part2, float2* srow, uint32_t* s_up,
-                            double (*red)[2], int step) {
+                            float2 (*red)[2], int step) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int k = n.k;
   const bool lanczos = n.mode == kModeLanczos && k < n.kmax;
   const bool replay = n.mode == kModeReplay && k + 1 < n.steps;
-  const bool cheb = n.mode == kModeCheb && k < n.kmax;
-  if (!(lanczos || replay || cheb)) {  // uniform over the block
+  constexpr bool cheb = CHEB;
+  if (!(lanczos || replay || (CHEB && k < n.kmax))) {  // uniform over the block
     if (threadIdx.x == 0) {
       part[pidx] = 0.0;
       part2[pidx] = 0.0;
@@ -822,7 +840,7 @@ __device__ void p_apply_row(const SlotDesc& s, const SlotNow& n, int64_t r, int6
     return;
   }
   const int64_t Dd = s.Dd;
-  const uint64_t row_bytes = sizeof(float2) * (uint64_t)Dd;
+  const uint32_t row_bytes = (uint32_t)sizeof(float2) * (uint32_t)Dd;  // staged: small
   const float2* x = s.buf[(k + 1) % 3];
   const float2* v = x + r * Dd;
   const float2* z = s.buf[k % 3] + r * Dd;
@@ -870,20 +888,46 @@ __device__ void p_apply_row(const SlotDesc& s, const SlotNow& n, int64_t r, int6
       dn(e.w);
     }
     const char* xc = reinterpret_cast<const char*>(x + cl);
-    auto up = [&](int q) {
-      return lz(*reinterpret_cast<const float2*>(xc + (uint64_t)s_up[q] * row_bytes), ls.v);
+    auto up = [&](uint32_t e) {
+      return lz(*reinterpret_cast<const float2*>(xc + (uint64_t)e * row_bytes), ls.v);
     };
     float pr = 0.f, pi = 0.f, nr = 0.f, ni = 0.f;
+    const uint4* up4 = reinterpret_cast<const uint4*>(s_up);
     int j = 0;
-#pragma unroll 4
-    for (; j < npos; ++j) {
-      const float2 val = up(j);
-      pr += val.x;
-      pi += val.y;
+#pragma unroll 1
+    for (; j + 4 <= npos; j += 4) {
+      const uint4 e = up4[j >> 2];
+      const float2 v0 = up(e.x), v1 = up(e.y), v2 = up(e.z), v3 = up(e.w);
+      pr = ((pr + v0.x) + v1.x) + v2.x + v3.x;
+      pi = ((pi + v0.y) + v1.y) + v2.y + v3.y;
     }
-#pragma unroll 4
+    if (j < nu && j < npos) {  // both signs
+      const uint4 e = up4[j >> 2];
+      const float2 zero = make_float2(0.f, 0.f);
+      const float2 v0 = up(e.x), v1 = j + 1 < nu ? up(e.y) : zero,
+                   v2 = j + 2 < nu ? up(e.z) : zero, v3 = j + 3 < nu ? up(e.w) : zero;
+      const float2 all[4] = {v0, v1, v2, v3};
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        if (j + q < npos) {
+          pr += all[q].x;
+          pi += all[q].y;
+        } else {
+          nr += all[q].x;
+          ni += all[q].y;
+        }
+      }
+      j += 4;
+    }
+#pragma unroll 1
+    for (; j + 4 <= nu; j += 4) {
+      const uint4 e = up4[j >> 2];
+      const float2 v0 = up(e.x), v1 = up(e.y), v2 = up(e.z), v3 = up(e.w);
+      nr = ((nr + v0.x) + v1.x) + v2.x + v3.x;
+      ni = ((ni + v0.y) + v1.y) + v2.y + v3.y;
+    }
     for (; j < nu; ++j) {
-      const float2 val = up(j);
+      const float2 val = up(s_up[j]);
       nr += val.x;
       ni += val.y;
     }
@@ -911,26 +955,9 @@ __device__ void p_apply_row(const SlotDesc& s, const SlotNow& n, int64_t r, int6
       eng_acc(hi2, lo2, o.y, o.y);
     }
   }
-  double dxy = (double)hi + (double)lo, dyy = (double)hi2 + (double)lo2;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    dxy += __shfl_down_sync(0xffffffffu, dxy, o);
-    dyy += __shfl_down_sync(0xffffffffu, dyy, o);
-  }
-  if (lane == 0) {
-    red[warp][0] = dxy;
-    red[warp][1] = dyy;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {  // fixed order over the warps
-    double a = 0.0, b = 0.0;
-    for (int q = 0; q < kEngPWarps; ++q) {
-      a += red[q][0];
-      b += red[q][1];
-    }
-    part[pidx] = a;
-    part2[pidx] = b;
-  }
+  const float2 xy = eng_warp_sum(hi, lo);
+  if constexpr (CHEB) eng_row_sums<true>(xy, eng_warp_sum(hi2, lo2), red, part + pidx, part2 + pidx);
+  else eng_row_sums<false>(xy, xy, red, part + pidx, part2 + pidx);
 }
 
 // Phase A, one small row (warp-level, the row staged in the warp's shared
@@ -1008,13 +1035,8 @@ __device__ void p_apply_warp_row(const SlotDesc& s, const SlotNow& n, int64_t r,
         eng_acc(hi2, lo2, o.y, o.y);
       }
     }
-    dxy = (double)hi + (double)lo;
-    dyy = (double)hi2 + (double)lo2;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      dxy += __shfl_down_sync(0xffffffffu, dxy, o);
-      dyy += __shfl_down_sync(0xffffffffu, dyy, o);
-    }
+    dxy = eng_pair(eng_warp_sum(hi, lo));
+    if (cheb) dyy = eng_pair(eng_warp_sum(hi2, lo2));
   }
   if (lane == 0) {
     part[pidx] = dxy;
@@ -1099,9 +1121,7 @@ __device__ void p_update_row(const SlotDesc& s, const SlotNow& n, int64_t r, int
       eng_acc(hi, lo, o.x, o.x);
       eng_acc(hi, lo, o.y, o.y);
     }
-    double nn = (double)hi + (double)lo;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) nn += __shfl_down_sync(0xffffffffu, nn, o);
+    double nn = eng_pair(eng_warp_sum(hi, lo));
     if (lane == 0) part[it] = nn;
     return;
   }
@@ -1186,16 +1206,20 @@ __device__ void p_advance(SlotDesc& s) {
   }
 }
 
-// four co-resident blocks an SM (64 registers a thread): the occupancy the
-// apply phase's gathers need
-__global__ void __launch_bounds__(kEngPWarps * 32, 4)
+// Co-resident blocks an SM (48 registers a thread): the apply's gathers and its
+// chains of loads a row want many warps, its row loop registers.  48 requests on
+// rings of 8, 10 and 12 sites, 100 steps, the apply phase with 4, 5 and 6 blocks:
+// 26.7, 24.6 and 25.3 ms (8: spills, 33).
+constexpr int kEngPCtas = 5;
+
+__global__ void __launch_bounds__(kEngPWarps * 32, kEngPCtas)
 k_eng_persistent(EngPersistArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ double red[kEngPWarps][2];
+  __shared__ float2 red[kEngRowWarps][2];
   __shared__ double sred[kEngPWarps * 32], sred2[kEngPWarps * 32];
   const int warp = threadIdx.x >> 5;
   float2* srow = reinterpret_cast<float2*>(smem);
-  uint32_t* s_up = reinterpret_cast<uint32_t*>(smem + sizeof(float2) * (a.row_cols + kSlicedPads));
+  uint32_t* s_up = reinterpret_cast<uint32_t*>(smem + sizeof(float2) * ((a.row_cols + kSlicedPads + 1) & ~1));
   float2* wrow = reinterpret_cast<float2*>(smem) + (size_t)warp * kEngWarpRowCols;
   const int gw = blockIdx.x * kEngPWarps + warp, nw = gridDim.x * kEngPWarps;
   for (int step = 0; step < a.steps; ++step) {
@@ -1204,8 +1228,11 @@ k_eng_persistent(EngPersistArgs a) {
     for (int it = blockIdx.x; it < a.n_rows; it += gridDim.x) {
       const int2 item = a.items_rows[it];
       const SlotDesc& s = a.slots[item.x];
-      p_apply_row(s, slot_now(s), item.y, s.item0 + item.y, a.part, a.part2, srow, s_up, red,
-                  step);
+      const SlotNow now = slot_now(s);
+      if (now.mode == kModeCheb)
+        p_apply_row<true>(s, now, item.y, s.item0 + item.y, a.part, a.part2, srow, s_up, red, step);
+      else
+        p_apply_row<false>(s, now, item.y, s.item0 + item.y, a.part, a.part2, srow, s_up, red, step);
     }
     __syncthreads();  // the row items' shared memory becomes the warps' rows
     for (int it = gw; it < a.n_warp; it += nw) {
@@ -1657,7 +1684,7 @@ void rebuild(mb_engine_s* e) {
                               sizeof(int2) * items_rows.size(), cudaMemcpyHostToDevice, e->st));
     // launch shape, set outside any capture: the staged row and its up list,
     // or the warps' rows, in dynamic shared memory; co-resident blocks
-    const size_t rows_smem = sizeof(float2) * (size_t)(e->row_cols + kSlicedPads) +
+    const size_t rows_smem = sizeof(float2) * (size_t)((e->row_cols + kSlicedPads + 1) & ~1) +
                              sizeof(uint32_t) * (size_t)((max_list + 3) & ~3);
     const size_t warps_smem = sizeof(float2) * (size_t)kEngPWarps * kEngWarpRowCols;
     e->p_smem = std::max(rows_smem, warps_smem);
