@@ -249,7 +249,8 @@ typedef struct {
   int table_bits;
   int prefetch;   /* 1: before its down hops, each warp asks L2 for the
                      up-hop lines of its column group, one 128-byte line a
-                     lane (any lattice operator) */
+                     lane (any lattice operator; a new one's shape
+                     has it where its vectors are much larger than L2) */
   int table_stage; /* 1: each warp copies its next column group's down-table
                       words into its own shared buffer (cp.async) while it
                       finishes the current one (MB_PREC_Q64, one pass, 32-bit

@@ -691,6 +691,7 @@ inline bool writes_reference(int precision, int64_t dim) {
   return precision == MB_PREC_F64 ||
          (precision == MB_PREC_F32 ? 8 : 16) * dim < 2 * kTileBytes;
 }
+bool apply_prefetches(const OpView& v, int precision);
 // Whether a reference-order call of a floating-point lattice operator is one
 // launch (kRefIn).  Every read of x then goes through the permutation, two loads
 // one after the other, so it pays where the launches and the moves are most of

@@ -539,6 +539,19 @@ static bool apply_staged(const OpView& v, int precision) {
   return apply_smem(v, precision, true) + 3072 <= (size_t)max_smem_optin();
 }
 
+// Whether an apply prefetches its up-hop lines unless told (OpView::up_prefetch):
+// vectors of more than ten times L2, whose up hops wait on HBM more often.  Off and
+// on, tensor order, ms: 4x4 8+8 (2.65 GB) complex128 12.3 and 11.2, Q64 10.6 and
+// 8.2, complex64 (1.33 GB) 5.86 and 4.56; 1D L=16 8+8 7.42, 7.25 / 5.69, 4.84 /
+// 3.03, 2.57; 4x4 7+6 (1.47 GB) 5.95, 5.99 / 3.84, 3.48; at 1.03 GB (4x4 6+6) 4.06,
+// 4.09 / 2.30, 2.31, smaller complex64 vectors 2-8 % slower with it.  Rows that are
+// not staged gain nothing but as Q64 (18 sites 5+7 13.1, 13.2 / 9.06, 8.61 / 4.80,
+// 5.05).
+bool apply_prefetches(const OpView& v, int precision) {
+  return (double)elem_bytes(precision) * (double)v.dim > 1.3e9 &&
+         (precision == MB_PREC_Q64 || apply_staged(v, precision));
+}
+
 // Threads of an apply's CTAs and how many of them an SM holds: together
 // kApplyResident, or fewer where the rows' shared memory ends it.  Several small
 // CTAs, where their rows fit in shared memory side by side, hide each other's

@@ -158,6 +158,7 @@ static void build_op(mb_op_s* op, const mb_basis_s* b, const mb_model_s* m) {
     if (bytes) MB_CUDA(cudaMemcpy(p, h, bytes, cudaMemcpyHostToDevice));
     return p;
   });
+  v.up_prefetch = apply_prefetches(v, op->precision) ? 1 : 0;
   const std::vector<double> uf = u_fold_table(m->u, m->has_u, op->L);
   v.u_fold = upload(op, uf);
   v.u_fold_f = upload(op, std::vector<float>(uf.begin(), uf.end()));
