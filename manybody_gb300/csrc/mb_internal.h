@@ -664,11 +664,15 @@ int multi_dot_grid(int64_t n);
 void launch_multi_dot(int vprec, int wprec, int64_t n, const void* V, int64_t ld, int m,
                       const void* w, double* partials, unsigned* ticket, double* out,
                       cudaStream_t st);
+// the same of complex128 vectors with the real parts alone (Im = 0)
+void launch_multi_dot_real(int64_t n, const void* V, int64_t ld, int m, const void* w,
+                           double* partials, unsigned* ticket, double* out, cudaStream_t st);
 // w -= sum_j c[j] V_j ; c on device (interleaved complex), then <w,w> partials,
 // summed to step.dots where it has a ticket
+// (real: the imaginary parts of c are 0, of complex128 vectors half the products)
 void launch_multi_axpy(int vprec, int wprec, int64_t n, const void* V, int64_t ld, int m,
                        const double* c, void* w, double* partials, const KrylovStep& step,
-                       cudaStream_t st);
+                       cudaStream_t st, bool real = false);
 void launch_convert(int from_prec, int to_prec, int64_t n, const void* x, void* y,
                     cudaStream_t st);
 void launch_gather(int precision, int64_t n, const int32_t* perm, const void* src, void* dst,

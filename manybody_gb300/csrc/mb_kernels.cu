@@ -1054,9 +1054,36 @@ constexpr int kMdChunk = 1024;
 constexpr int kMdThreads = 256;
 constexpr int kMdBatch = 8;  // loads in flight per lane in the multi-vector kernels
 constexpr int kMaxBasis = 1024;
+constexpr int kMdFew = 8;
+
+// The last block of a multi_dot to finish sums every block's partials in block
+// order: warp w the sums w, w + nwarps, ..., four chains a lane.
+__device__ void multi_dot_sums(const double* partials, int m, unsigned* ticket, double* out) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(ticket, 1u) + 1u == gridDim.x;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  const int nb = (int)gridDim.x, nc = 2 * m;
+  for (int k = warp; k < nc; k += nwarps) {
+    double a[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int b = lane; b < nb; b += 128)
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (b + 32 * q < nb) a[q] += __ldcg(partials + (size_t)(b + 32 * q) * nc + k);
+    double t = (a[0] + a[1]) + (a[2] + a[3]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+    if (lane == 0) out[k] = t;
+  }
+  if (threadIdx.x == 0) *ticket = 0;
+}
 
 template <typename TV, typename TW>
-__global__ void __launch_bounds__(kMdThreads)
+__global__ void __launch_bounds__(kMdThreads, 4)
 k_multi_dot(int64_t n, const typename C2<TV>::type* __restrict__ V, int64_t ld, int m,
             const typename C2<TW>::type* __restrict__ w, double* partials, unsigned* ticket,
             double* __restrict__ out) {
@@ -1141,28 +1168,7 @@ k_multi_dot(int64_t n, const typename C2<TV>::type* __restrict__ V, int64_t ld, 
   __syncthreads();
   for (int j = threadIdx.x; j < 2 * m; j += blockDim.x)
     partials[(size_t)blockIdx.x * 2 * m + j] = acc[j];
-  // the last block to finish sums every block's partials in block order: warp w
-  // the sums w, w + 8, ..., four chains a lane
-  __shared__ bool last;
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) last = atomicAdd(ticket, 1u) + 1u == gridDim.x;
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  const int nb = (int)gridDim.x, nc = 2 * m;
-  for (int k = warp; k < nc; k += nwarps) {
-    double a[4] = {0.0, 0.0, 0.0, 0.0};
-    for (int b = lane; b < nb; b += 128)
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-        if (b + 32 * q < nb) a[q] += __ldcg(partials + (size_t)(b + 32 * q) * nc + k);
-    double t = (a[0] + a[1]) + (a[2] + a[3]);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
-    if (lane == 0) out[k] = t;
-  }
-  if (threadIdx.x == 0) *ticket = 0;
+  multi_dot_sums(partials, m, ticket, out);
 }
 
 static int md_grid(int64_t n) {
@@ -1184,6 +1190,60 @@ static void multi_dot_t(int64_t n, const void* V, int64_t ld, int m, const void*
   MB_CUDA(cudaGetLastError());
 }
 
+// Re<V_j, w> of up to kMdFew complex128 columns (the imaginary parts of out 0), each
+// thread all columns of its elements: every warp has work and its sums stay in
+// registers, where multi_dot gives a warp a column and leaves the others idle.  Two
+// of the slow FP64 multiply-adds a column and element bound it.  1 to 8 columns of
+// 4x4 5+5 (305 MB each), mean: 0.86 -> 0.30 ms (and 0.78 -> 0.38 in
+// the multi_axpy after it, with real coefficients).
+__global__ void __launch_bounds__(kMdThreads, 4)
+k_multi_dot_real(int64_t n, const double2* __restrict__ V, int64_t ld, int m,
+                 const double2* __restrict__ w, double* partials, unsigned* ticket,
+                 double* __restrict__ out) {
+  double c[kMdFew];
+#pragma unroll
+  for (int j = 0; j < kMdFew; ++j) c[j] = 0.0;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    double2 a[kMdFew];
+#pragma unroll
+    for (int j = 0; j < kMdFew; ++j)
+      if (j < m) a[j] = V[(int64_t)j * ld + i];
+    const double2 b = w[i];
+#pragma unroll
+    for (int j = 0; j < kMdFew; ++j) {
+      if (j >= m) break;
+      c[j] = fma(a[j].x, b.x, c[j]);
+      c[j] = fma(a[j].y, b.y, c[j]);
+    }
+  }
+  __shared__ double red[kMdThreads / 32][kMdFew];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int j = 0; j < kMdFew; ++j) {
+    if (j >= m) break;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) c[j] += __shfl_down_sync(0xffffffffu, c[j], o);
+    if (lane == 0) red[warp][j] = c[j];
+  }
+  __syncthreads();
+  if ((int)threadIdx.x < 2 * m) {
+    double a = 0.0;
+    if (!(threadIdx.x & 1))
+      for (int q = 0; q < kMdThreads / 32; ++q) a += red[q][threadIdx.x >> 1];
+    partials[(size_t)blockIdx.x * 2 * m + threadIdx.x] = a;
+  }
+  multi_dot_sums(partials, m, ticket, out);
+}
+
+void launch_multi_dot_real(int64_t n, const void* V, int64_t ld, int m, const void* w,
+                           double* partials, unsigned* ticket, double* out, cudaStream_t st) {
+  MB_REQUIRE(m <= kMdFew, MB_ERR_CAPACITY, "more columns than a projection takes");
+  k_multi_dot_real<<<md_grid(n), kMdThreads, 0, st>>>(n, (const double2*)V, ld, m,
+                                                      (const double2*)w, partials, ticket, out);
+  MB_CUDA(cudaGetLastError());
+}
+
 void launch_multi_dot(int vprec, int wprec, int64_t n, const void* V, int64_t ld, int m,
                       const void* w, double* partials, unsigned* ticket, double* out,
                       cudaStream_t st) {
@@ -1195,8 +1255,9 @@ void launch_multi_dot(int vprec, int wprec, int64_t n, const void* V, int64_t ld
   else multi_dot_t<double, double>(n, V, ld, m, w, partials, ticket, out, st);
 }
 
-// w -= sum_j c_j V_j (c complex, on device), then <w,w> partials.
-template <typename TV, typename TW>
+// w -= sum_j c_j V_j (c complex, on device; REAL: its real parts), then <w,w>
+// partials.
+template <typename TV, typename TW, bool REAL>
 __global__ void __launch_bounds__(kBlasThreads)
 k_multi_axpy(int64_t n, const typename C2<TV>::type* __restrict__ V, int64_t ld, int m,
              const double* __restrict__ c, typename C2<TW>::type* __restrict__ w,
@@ -1248,10 +1309,11 @@ k_multi_axpy(int64_t n, const typename C2<TV>::type* __restrict__ V, int64_t ld,
         for (int u = 0; u < kMdBatch; ++u) {
           if (j0 + u >= m) break;
           // four multiply-adds (a difference of products would take six)
-          const double cr = sc[2 * (j0 + u)], ci = sc[2 * (j0 + u) + 1];
+          const double cr = sc[2 * (j0 + u)];
           sr = fma(-cr, (double)a[u].x, sr);
           si = fma(-cr, (double)a[u].y, si);
-          if (ci != 0.0) {
+          if constexpr (!REAL) {
+            const double ci = sc[2 * (j0 + u) + 1];
             sr = fma(ci, (double)a[u].y, sr);
             si = fma(-ci, (double)a[u].x, si);
           }
@@ -1272,17 +1334,19 @@ k_multi_axpy(int64_t n, const typename C2<TV>::type* __restrict__ V, int64_t ld,
 
 void launch_multi_axpy(int vprec, int wprec, int64_t n, const void* V, int64_t ld, int m,
                        const double* c, void* w, double* partials, const KrylovStep& step,
-                       cudaStream_t st) {
+                       cudaStream_t st, bool real) {
   MB_REQUIRE(m <= kMaxBasis, MB_ERR_CAPACITY, "re-orthogonalisation basis larger than 1024");
   const int g = blas_grid(n);
   if (vprec == MB_PREC_F32 && wprec == MB_PREC_F32)
-    k_multi_axpy<float, float><<<g, kBlasThreads, 0, st>>>(n, (const float2*)V, ld, m, c, (float2*)w, partials, step);
+    k_multi_axpy<float, float, false><<<g, kBlasThreads, 0, st>>>(n, (const float2*)V, ld, m, c, (float2*)w, partials, step);
   else if (vprec == MB_PREC_F32)
-    k_multi_axpy<float, double><<<g, kBlasThreads, 0, st>>>(n, (const float2*)V, ld, m, c, (double2*)w, partials, step);
+    k_multi_axpy<float, double, false><<<g, kBlasThreads, 0, st>>>(n, (const float2*)V, ld, m, c, (double2*)w, partials, step);
   else if (wprec == MB_PREC_F32)
-    k_multi_axpy<double, float><<<g, kBlasThreads, 0, st>>>(n, (const double2*)V, ld, m, c, (float2*)w, partials, step);
+    k_multi_axpy<double, float, false><<<g, kBlasThreads, 0, st>>>(n, (const double2*)V, ld, m, c, (float2*)w, partials, step);
+  else if (real)
+    k_multi_axpy<double, double, true><<<g, kBlasThreads, 0, st>>>(n, (const double2*)V, ld, m, c, (double2*)w, partials, step);
   else
-    k_multi_axpy<double, double><<<g, kBlasThreads, 0, st>>>(n, (const double2*)V, ld, m, c, (double2*)w, partials, step);
+    k_multi_axpy<double, double, false><<<g, kBlasThreads, 0, st>>>(n, (const double2*)V, ld, m, c, (double2*)w, partials, step);
   MB_CUDA(cudaGetLastError());
 }
 

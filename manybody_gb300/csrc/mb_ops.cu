@@ -906,6 +906,7 @@ struct Krylov {
   void combine_kept(int64_t m, const std::vector<double>& betas,
                     const std::vector<std::complex<double>>& y, void* x) {
     std::vector<double> c(2 * (size_t)m);
+    const bool real = std::all_of(y.begin(), y.begin() + m, [](auto v) { return v.imag() == 0.0; });
     for (int64_t j = 0; j < m; ++j) {
       const double sj = j > 0 ? betas[(size_t)j - 1] : 1.0;
       c[2 * (size_t)j] = -y[(size_t)j].real() / sj;  // multi_axpy subtracts
@@ -918,7 +919,7 @@ struct Krylov {
     for (int64_t j0 = 0; j0 < m; j0 += kKeepChunk) {
       const int cnt = (int)std::min<int64_t>(kKeepChunk, m - j0);
       launch_multi_axpy(prec, prec, n, keep_col(j0), n, cnt, (const double*)keep_coef.p + 2 * j0,
-                        x, red.p(), KrylovStep{}, st);
+                        x, red.p(), KrylovStep{}, st, real);
     }
   }
 
@@ -1268,15 +1269,17 @@ static void refine_chunk(std::vector<RefineRun>& runs, RefineBufs& bufs, cudaStr
     MB_REQUIRE(nx > 0.0, MB_ERR_ZERO_NORM, "refinement start vector has zero norm");
     launch_axpby(MB_PREC_F64, r.n, 1.0 / nx, 0.0, r.col(0), 0.0, 0.0, r.col(0), nullptr, 0, ls(i));
   }
-  // w -= Q Q^H w against q_0..q_j: the coefficients at dc[0..), the norm of
-  // the rest in the second dots
+  // w -= Q Re(Q^H w) against q_0..q_j: the coefficients at dc[0..), the norm of
+  // the rest in the second dots.  On pairs of real numbers H is a symmetric
+  // operator of twice the size, with the same eigenvalues and the inner product
+  // Re<.,.>: its Lanczos vectors, and T, are these, with the real parts alone.
   auto project = [&](size_t i, int j) {
     RefineRun& r = runs[i];
     void* w = r.col(j + 1);
-    launch_multi_dot(MB_PREC_F64, MB_PREC_F64, r.n, r.q, r.n, j + 1, w, pp(i),
-                     (unsigned*)bufs.tickets.p + i % kRefineLanes, r.dc, ls(i));
+    launch_multi_dot_real(r.n, r.q, r.n, j + 1, w, pp(i),
+                          (unsigned*)bufs.tickets.p + i % kRefineLanes, r.dc, ls(i));
     launch_multi_axpy(MB_PREC_F64, MB_PREC_F64, r.n, r.q, r.n, j + 1, r.dc, w, pp(i),
-                      step(i, blas_grid(r.n), 3), ls(i));
+                      step(i, blas_grid(r.n), 3), ls(i), true);
   };
   for (int j = 0;; ++j) {
     bool any = false;
