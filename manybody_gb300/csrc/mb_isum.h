@@ -91,12 +91,26 @@ struct ISum {
     asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(a) : "r"(lo), "r"(f.by0));
   }
   __device__ __forceinline__ bool odd() const { return e <= kISumLeast || e >= 0x7FF; }
+  // a and the exponent of its unit, for scaled_by
+  __device__ __forceinline__ double count() const { return __ll2double_rn(a); }
+  __device__ __forceinline__ int exponent(const ISumForm& f) const { return e + f.unit; }
   // a * 2^(e + unit): the conversion rounds, the product is exact.  e > 512 and
   // base < 64 keep the factor a normal number.
   __device__ __forceinline__ double value(const ISumForm& f) const {
     return __ll2double_rn(a) * __hiloint2double((e + f.unit + 1023) << 20, 0);
   }
 };
+
+// a * c = (a * 2^k) * c0 exactly, with the power of two in c where that stays a
+// normal number (no FP64 instruction), else in a; k of ISum::exponent, or 0.
+__device__ __forceinline__ void scaled_by(int k, double c0, double& a, double& c) {
+  const int h = __double2hiint(c0), ex = (h >> 20) & 0x7FF;
+  c = c0;
+  if (ex != 0 && (unsigned)(ex + k - 1) < 2046u && ex != 0x7FF)
+    c = __hiloint2double(h + k * (1 << 20), __double2loint(c0));
+  else
+    a *= __hiloint2double((k + 1023) << 20, 0);
+}
 
 // hi += sign * (r >> 32), lo += sign * (bits 3..31 of r)
 __device__ __forceinline__ void isum_parts(unsigned long long r, int sign, int& hi, int& lo) {

@@ -262,6 +262,13 @@ __device__ __forceinline__ void apply_rows(
   // value that does not fit there
   __shared__ int s_wide[2];
   if (threadIdx.x < 2) s_wide[threadIdx.x] = 0;
+  // The diagonal's factor of x by the number of doubly occupied sites, where there
+  // are no self energies: with the sums' powers of two in the coefficients
+  // (scaled_by) five of an element's 13 FP64 instructions less.  4x4 5+5 1149 ->
+  // 1121 us, 6+6 4.03 -> 3.95 ms, 14 sites 4+4 48.2 -> 45.2 us.
+  __shared__ T s_diag[33];
+  const bool given = (DOTS & 1) && s_coef;
+  const bool tabled = kInt && !self_up && !self_dn;
   if (STAGED && threadIdx.x < kSlicedPads) {
     V2 zero;
     zero.x = T(0);
@@ -282,6 +289,8 @@ __device__ __forceinline__ void apply_rows(
       return __ldg(x + (DOTS & kRefIn ? (int64_t)__ldg(v.out_perm + i) : i));
     };
     __syncthreads();
+    if (tabled && ri == blockIdx.x && (int)threadIdx.x <= v.L)
+      s_diag[threadIdx.x] = (given ? s_coef[1] : dscale) * (ufold[threadIdx.x] - shift);
     const int u0 = __ldg(&v.up_loff[r]), nu = __ldg(&v.up_loff[r + 1]) - u0;
     const int npos = __ldg(&v.up_lpos[r]);
     for (int j = threadIdx.x; j < nu; j += blockDim.x)  // complex128: the sign in bit 31
@@ -311,6 +320,7 @@ __device__ __forceinline__ void apply_rows(
       const int64_t cl = live ? c : Dd - 1;
       if (v.up_prefetch) prefetch_up_group<(int)sizeof(V2)>(x, s_up, nu, g, lane, row_bytes);
       T ar = T(0), ai = T(0);
+      int er = 0, ei = 0;  // the sums are ar * 2^er, ai * 2^ei
       const int2 gi = __ldg(reinterpret_cast<const int2*>(v.dn_sgrp) + g);
       // four slots per 16-byte load; the last word's unused slots are padding
       const uint4* ep = reinterpret_cast<const uint4*>(v.dn_sell + gi.x) + lane;
@@ -429,12 +439,14 @@ __device__ __forceinline__ void apply_rows(
             else if (j + 2 == nu) up_add(integral_constant<int, 2>{}, e);
             else up_add(integral_constant<int, 3>{}, e);
           }
-          const double2 hops = sum.value(form);
-          ar = hops.x;
-          ai = hops.y;
+          ar = sum.re.count();
+          ai = sum.im.count();
+          er = sum.re.exponent(form);
+          ei = sum.im.exponent(form);
         }
         if (wide || sum.odd()) {
           ar = ai = T(0);
+          er = ei = 0;
           fp_hops();
         }
       } else {
@@ -442,15 +454,28 @@ __device__ __forceinline__ void apply_rows(
       }
       if (!live) continue;
       const V2 xv = STAGED && !kInt ? reinterpret_cast<const V2*>(smem)[c] : x_at(row0 + c);
-      T dv = ufold[__popc(um & v.dn_mask[c])] + su;
-      if (self_dn) dv += self_dn[c];
+      const int both = __popc(um & v.dn_mask[c]);
+      T ds;
+      if (tabled) {
+        ds = s_diag[both];
+      } else {
+        T dv = ufold[both] + su;
+        if (self_dn) dv += self_dn[c];
+        ds = (given ? s_coef[1] : dscale) * (dv - shift);
+      }
       // (coefficients from shared memory, where given, only now: registers)
-      const bool given = (DOTS & 1) && s_coef;
       const T hc = given ? s_coef[0] : hop_coef;
-      const T ds = (given ? s_coef[1] : dscale) * (dv - shift);
       V2 out;
-      out.x = fma(hc, ar, ds * xv.x);
-      out.y = fma(hc, ai, ds * xv.y);
+      if constexpr (kInt) {
+        double hr, hi;
+        scaled_by(er, hc, ar, hr);
+        scaled_by(ei, hc, ai, hi);
+        out.x = fma(hr, ar, ds * xv.x);
+        out.y = fma(hi, ai, ds * xv.y);
+      } else {
+        out.x = fma(hc, ar, ds * xv.x);
+        out.y = fma(hc, ai, ds * xv.y);
+      }
       const int64_t idx = row0 + c;
       const int64_t out_idx = DOTS & kRefOut ? (int64_t)__ldcs(v.out_perm + idx) : idx;
       if (z) {

@@ -110,3 +110,21 @@ def test_integer_row_sums_of_a_momentum_sector(mb, cuda, dims, n, k, lanes, kind
         want, size = exact(m, part)
         off = np.abs(got.astype(np.longdouble) - want)
         assert np.all(off <= eps * size + 16 * 2.0 ** -1074), float(np.max(off / np.maximum(size, 1e-300)))
+
+
+# (results stay normal numbers: x is 2^-20 and larger)
+@pytest.mark.parametrize("k,xk", [(-975, 0), (-960, 0), (-500, -40), (300, -40), (950, 0), (950, -40)])
+def test_powers_of_two_in_the_coefficients(mb, cuda, k, xk):
+    """The scale of H and x powers of two: the result's exactly, also where the
+    sums' own power does not fit beside the hopping's; and no hopping at all."""
+    torch = cuda
+    basis = mb.FermionBasis.with_fixed_particle_number_and_spin(9, 9, 1)
+    one = mb.GpuHubbardOperator(basis, mb._Hubbard(1.0, 8.0, (9,)), 0)
+    flat = mb.GpuHubbardOperator(basis, mb._Hubbard(0.0, 8.0, (9,)), 0)
+    x = one.seed_vector(2)
+    want = torch.view_as_real(one.apply(x))
+    got = torch.view_as_real(one.apply_affine(x * 2.0 ** xk, scale=2.0 ** k))
+    assert torch.equal(got * 2.0 ** (-k // 2) * 2.0 ** (-k - -k // 2) * 2.0 ** -xk, want)
+    y = flat.apply(x)
+    d = (y / x).real.round()
+    assert torch.equal(y, d * x) and not (d % 8).any()
