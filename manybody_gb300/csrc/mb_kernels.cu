@@ -201,7 +201,7 @@ static int max_smem_optin() {
 // The matrix-free apply:  y = scale * (H - shift) x + beta * z
 // with optional fused dot products (dot_mode bit0: Re<x,y>, bit1: <y,y>,
 // bit2: <x,x>).  The CTAs walk the rows r_up in the row schedule's order; one
-// stages the row X[r_up, :] (and eight zero elements) in shared memory when it
+// stages the row X[r_up, :] (and sixteen zero elements) in shared memory when it
 // fits, so the down hops, which stay inside the row, gather from shared memory
 // through the sliced table (one coalesced 16-byte load per lane for four
 // slots: neighbour index | sign << 31, padding = one of the zero elements past
@@ -222,8 +222,8 @@ static int max_smem_optin() {
 // converts them and does the diagonal, the affine part and the dots.  A staged
 // row is decoded once (each element is a down neighbour about 16 times), up
 // neighbours as they arrive; a row or a sum outside the integer sums' range
-// takes the FP64 adds.  4x4 6+6 (64.1M states) 10.08 -> 4.06 ms, 5+5 2.81 ->
-// 1.15, 1D L=16 8+8 15.98 -> 7.41, 3x4 6+6 137 -> 58 us.  By the counters (4x4
+// takes the FP64 adds.  4x4 6+6 (64.1M states) 10.08 -> 3.95 ms, 5+5 2.81 ->
+// 1.12, 1D L=16 8+8 15.98 -> 6.83, 3x4 6+6 137 -> 57 us.  By the counters (4x4
 // 5+5) the ALU pipe is now 65 % busy, the FP64 pipe 38 %, issue 64 %, and the
 // largest stall is waiting for L2 (3.8 of 10.7 warps a scheduler).
 // ---------------------------------------------------------------------------

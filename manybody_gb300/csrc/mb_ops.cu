@@ -1120,7 +1120,8 @@ struct Krylov {
 // times the rounding, worse by that factor every step (1D L=14 13+13 at U=9.2,
 // beta_0 ~ 1e-5, |E0| ~ 100: the lowest Ritz value fell 7 % below E0 within six
 // steps).  Two passes in every step held it too, at twice the FP64 work: 27 of
-// the 65 ms of a 40-step 4x4 5+5 solve were these projections, now 14 of 52.
+// the 65 ms of a 40-step 4x4 5+5 solve were these projections; with one pass, on
+// real parts, they are 6 of 41.
 // After each step the lowest eigenvalue of T_(j+1) is the estimate; steps
 // continue until it settles to kRefineSettle relative (at least
 // kRefineMinSteps), the space breaks down, or the problem's step budget

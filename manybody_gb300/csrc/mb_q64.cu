@@ -239,7 +239,7 @@ void launch_q_reduce128(const void* part, int nblocks, double* out, cudaStream_t
 //
 // One CTA of 1024 threads per SM walks the rows r_up in the row schedule's
 // order (reverse Cuthill-McKee: rows in flight together share neighbour rows
-// in L2).  Per row: the row x[r,:] and eight zero elements go to shared
+// in L2).  Per row: the row x[r,:] and sixteen zero elements go to shared
 // memory, then warp w takes the 32-column groups g = w, w + 32, ...:
 //   down hops: sliced table, one coalesced 16-byte load per lane for four
 //     slots; entry = neighbour index in the staged row | sign << 31, in an
@@ -369,7 +369,7 @@ __device__ __forceinline__ void sliced_sum_t(const uint32_t* sell, const uint16_
 
 // ---------------------------------------------------------------------------
 // Column pass of the two-pass Q64 apply.  For every column c (down state) the
-// column x[:, c] (Du elements, 16 bytes apart by the row length) and eight zero
+// column x[:, c] (Du elements, 16 bytes apart by the row length) and sixteen zero
 // elements are staged in shared memory; warp w then takes the 32-row groups
 // g = w, w + 32, ... and gathers each row's up hops from the staged column
 // through the up sector's sliced table, exactly as the row pass gathers down
@@ -613,8 +613,8 @@ static int smem_optin() {
 // adds x ^ -1 = -x - 1, its count added back once) and dq = round(2^G scale
 // (diag - shift)) the row's fixed-point diagonal, formed here in FP64 once a
 // row.  kQCsrLanes lanes a row, 256 threads a block, the fused exact dots as
-// in k_apply_q.  The integer hop sums run on the integer pipe, where the
-// complex128 kernel's adds wait on this GPU's FP64 pipe.
+// in k_apply_q.  The hop sums are plain int64 adds, where the
+// complex128 kernel aligns every term (mb_isum.h).
 // ---------------------------------------------------------------------------
 constexpr int kQCsrThreads = 256;
 constexpr int kQCsrLanes = 8;  // lanes a row unless the operator's shape says otherwise
