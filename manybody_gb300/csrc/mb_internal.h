@@ -354,6 +354,9 @@ constexpr int kRefOut = 8;
 // kernel must not read what it has written: y apart from x (see one_launch).
 constexpr int kRefIn = 16;
 
+// of a kernel form for OpView::up_prefetch (kAheadForm; not a caller's flag)
+constexpr int kAhead = 64;
+
 // Device-side view of an operator (POD; passed to kernels by value).
 struct OpView {
   int64_t Du, Dd, dim;

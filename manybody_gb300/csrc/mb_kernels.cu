@@ -235,6 +235,14 @@ template <typename T> constexpr int kApplyMax = 1024;
 template <typename T> constexpr int kApplyResident = sizeof(T) == 4 ? 2048 : 1024;
 template <typename T> constexpr int kApplyCtasPerSm = kApplyResident<T> / kApplyMax<T>;
 
+// Whether the launches with up_prefetch have a kernel of their own (kAhead): the
+// complex64 forms with dots or in reference order, which have no registers for the
+// test.  Without it, reference order 1D L=14 7+7 249 -> 238 us, 4x4 6+6 1.72 -> 1.66
+// ms, a 40-step ground state of 4x4 5+5 with its refinement 40.3 -> 39.0 ms.  The
+// plain form keeps it: L=14 146 against 152 us, 5+5 318 / 328, 6+6 1.17 / 1.13 ms.
+template <typename T, int DOTS>
+constexpr bool kAheadForm = sizeof(T) == 4 && (DOTS & ~kAhead) != 0;
+
 // +-1 from the sign bit of a table entry
 __device__ __forceinline__ double unit_sign(uint32_t e, double) {
   return __hiloint2double((int)(0x3ff00000u | (e & 0x80000000u)), 0);
@@ -318,7 +326,8 @@ __device__ __forceinline__ void apply_rows(
       const int64_t c = (g << 5) + lane;
       const bool live = c < Dd;
       const int64_t cl = live ? c : Dd - 1;
-      if (v.up_prefetch) prefetch_up_group<(int)sizeof(V2)>(x, s_up, nu, g, lane, row_bytes);
+      if (kAheadForm<T, DOTS> ? (DOTS & kAhead) != 0 : v.up_prefetch != 0)
+        prefetch_up_group<(int)sizeof(V2)>(x, s_up, nu, g, lane, row_bytes);
       T ar = T(0), ai = T(0);
       int er = 0, ei = 0;  // the sums are ar * 2^er, ai * 2^ei
       const int2 gi = __ldg(reinterpret_cast<const int2*>(v.dn_sgrp) + g);
@@ -621,6 +630,8 @@ static void apply_t(const OpView& v, const void* x, void* y, double scale, doubl
   using V2 = typename C2<T>::type;
   const size_t smem = apply_smem(v, sizeof(T) == 8 ? MB_PREC_F64 : MB_PREC_F32, STAGED);
   auto kern = k_apply<T, STAGED, DOTS>;
+  if constexpr (kAheadForm<T, DOTS>)
+    if (v.up_prefetch) kern = k_apply<T, STAGED, DOTS | kAhead>;
   MB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const T* uf = sizeof(T) == 8 ? (const T*)v.u_fold : (const T*)v.u_fold_f;
   const T* su = sizeof(T) == 8 ? (const T*)v.self_up : (const T*)v.self_up_f;
