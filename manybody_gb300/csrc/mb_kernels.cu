@@ -215,8 +215,8 @@ static int max_smem_optin() {
 // above half.  Its sliced table is ordered for 8-byte elements now (2
 // wavefronts a slot instead of ~3.5), the up list is read four entries at a
 // time, whose neighbours are loaded together and added or subtracted without a
-// sign each: 123 wavefronts; 5+5 417 -> 314 us, 6+6 1.44 -> 1.18 ms, 3x4 6+6 26 ->
-// 20.6 us, 1D L=14 7+7 165 -> 149.  Issue (68 %) and waits for L2 are next.
+// sign each: 123 wavefronts; 5+5 417 -> 313 us, 6+6 1.44 -> 1.16 ms, 3x4 6+6 26 ->
+// 20.5 us, 1D L=14 7+7 165 -> 146.  Issue (68 %) and waits for L2 are next.
 //
 // complex128: the hop sums run on the integer pipes (mb_isum.h), the FP64 pipe
 // converts them and does the diagonal, the affine part and the dots.  A staged
@@ -224,7 +224,7 @@ static int max_smem_optin() {
 // neighbours as they arrive; a row or a sum outside the integer sums' range
 // takes the FP64 adds.  4x4 6+6 (64.1M states) 10.08 -> 3.95 ms, 5+5 2.81 ->
 // 1.12, 1D L=16 8+8 15.98 -> 6.83, 3x4 6+6 137 -> 57 us.  By the counters (4x4
-// 5+5) the ALU pipe is now 65 % busy, the FP64 pipe 38 %, issue 64 %, and the
+// 5+5) the ALU pipe is now 67 % busy, the FP64 pipe 29 %, issue 66 %, and the
 // largest stall is waiting for L2 (3.8 of 10.7 warps a scheduler).
 // ---------------------------------------------------------------------------
 // Most threads of a CTA, and the threads an SM holds: 64 registers a thread for
