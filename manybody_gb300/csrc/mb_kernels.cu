@@ -1091,6 +1091,7 @@ constexpr int kMdThreads = 256;
 constexpr int kMdBatch = 8;  // loads in flight per lane in the multi-vector kernels
 constexpr int kMaxBasis = 1024;
 constexpr int kMdFew = 8;
+static_assert(kRefineMaxSteps <= kMdFew, "a refinement projects against as many columns");
 
 // The last block of a multi_dot to finish sums every block's partials in block
 // order: warp w the sums w, w + nwarps, ..., four chains a lane.
