@@ -75,7 +75,14 @@ void ws_free(void* p, cudaStream_t st) {
 
 size_t ws_idle() {
   uint64_t reserved = 0, used = 0;
-  cudaMemPool_t pool = device_pool();
+  int dev = 0;
+  MB_CUDA(cudaGetDevice(&dev));
+  cudaMemPool_t pool = nullptr;
+  {
+    std::lock_guard<std::mutex> lk(g_mu);
+    if (dev >= 0 && dev < kPoolDevices) pool = g_pool[dev];
+  }
+  if (!pool) return 0;  // not made for the question
   if (cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess ||
       cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess) {
     cudaGetLastError();
