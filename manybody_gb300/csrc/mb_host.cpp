@@ -493,7 +493,7 @@ void fill_fused_tables(OpView& v, const HopTable& tu, const HopTable& td, int64_
   v.table_stage = 0;
   v.dn_max_words = 0;
   for (size_t g = 1; g < sd.grp.size(); g += 2) v.dn_max_words = std::max(v.dn_max_words, (sd.grp[g] + 3) / 4);
-  v.isum_base = isum_base((int64_t)v.max_up_list + 4 * (int64_t)v.dn_max_words);
+  v.isum_base = isum_base((int64_t)v.max_up_list + 4 * (int64_t)v.dn_max_words, kISumDecoded);
 }
 
 std::vector<double> u_fold_table(double u, bool has_u, int L) {

@@ -298,13 +298,18 @@ struct SlicedTable {
   std::vector<uint8_t> nneg;  // [D] negative entries per state
 };
 SlicedTable sliced_table(const HopTable& t, int64_t D, int lanes = 8);
-// 1 + ceil(log2(terms)), at least 6: the bits an integer sum (mb_isum.h) of that
-// many terms keeps free above its largest term, sign included.
+// 1 + ceil(log2(terms)), at least `least`: the bits an integer sum (mb_isum.h) of
+// that many terms keeps free above its largest term, sign included.  Four terms'
+// high parts, 35 - base bits each, meet in 32 bits: 6 where every term is a
+// magnitude with its sign multiplied in; 7 where decoded terms are among them,
+// which are shifted with their sign (floored), so that a negative one reaches
+// -2^(35 - base) itself and four of them with a negative hop 2^(37 - base).
 // Up to kISumBaseMax a sum keeps its largest term's whole significand (512
 // terms, one bit to spare).
+constexpr int kISumRaw = 6, kISumDecoded = 7;
 constexpr int kISumBaseMax = 10;
-inline int isum_base(int64_t terms) {
-  int b = 6;
+inline int isum_base(int64_t terms, int least) {
+  int b = least;
   while ((int64_t(1) << (b - 1)) < terms) ++b;
   return b;
 }

@@ -8,14 +8,19 @@
 // A sum keeps a 64-bit integer in units of the largest term so far: a term of
 // biased exponent e contributes its 53-bit significand, placed so that the
 // largest possible term is below 2^(64 - base), shifted right by E - e with E
-// the largest exponent met (when E grows the sum so far is shifted too).  base
-// = 1 + ceil(log2(terms)) leaves room for every term's carry; at 64 terms (4x4)
-// it is 7, and 3 or 4 bits stay below a double's last place of the largest
-// term.  What is cut off is below one such unit a term (each is rounded towards
-// zero), against half a last place of the partial sum for every FP64 add: the
-// sums are more exact than FP64's, element by element and not only against the
-// vector's norm.  A sum whose terms are all below 2^-511, or that holds an
-// infinity or NaN, is reported (odd) and left to FP64 by the caller.
+// the largest exponent met (when E grows the sum so far is shifted too, by a
+// spare bit more, which also keeps 2^(base - 1) floored terms of either sign in
+// 64 bits: the first ones are below half).  base = 1 + ceil(log2(terms)), at
+// least 7 with decoded terms and 6 without (isum_base), leaves room for every
+// term's carry; at 64 terms (4x4) it is 7, and 3 or 4 bits stay below a double's
+// last place of the largest term (at 512 terms one or none).  What is cut off is
+// below one such unit a term, towards zero, or of a decoded term downwards: a
+// sum is off by less than 2^-55 (base 7) of its largest term for every term,
+// where FP64 adds round by up to 2^-53 of the partial sum.  The bound is
+// against the largest term: where large terms cancel, a term below the unit is
+// lost that FP64 adds could have kept (1 - 1 + 2^-70 gives 0).  A sum whose terms
+// are all below 2^-511, or that holds an infinity or NaN, is reported (odd) and
+// left to FP64 by the caller.
 //
 // Signs are multiplied in: four terms' high and low parts (29 bits each) times
 // +-1 meet in two 32-bit integers, on the FMA pipe, and go to the 64-bit sum

@@ -332,7 +332,7 @@ static void build_momentum(mb_op_s* op, const mb_basis_s* b, const mb_model_s* m
   int64_t longest = 0;
   for (int64_t i = 0; i < out.n; ++i)
     longest = std::max(longest, out.row_ptr[(size_t)i + 1] - out.row_ptr[(size_t)i]);
-  v.isum_base = isum_base((longest + 3) / 4);  // at least 4 lanes a row
+  v.isum_base = isum_base((longest + 3) / 4, kISumRaw);  // at least 4 lanes a row
   if (v.isum_base > kISumBaseMax) v.isum_base = 0;
 }
 
