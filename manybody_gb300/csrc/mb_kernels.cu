@@ -222,8 +222,9 @@ static int max_smem_optin() {
 // converts them and does the diagonal, the affine part and the dots.  A staged
 // row is decoded once (each element is a down neighbour about 16 times), up
 // neighbours as they arrive; a row or a sum outside the integer sums' range
-// takes the FP64 adds.  4x4 6+6 (64.1M states) 10.08 -> 3.95 ms, 5+5 2.81 ->
-// 1.12, 1D L=16 8+8 15.98 -> 6.83, 3x4 6+6 137 -> 57 us.  By the counters (4x4
+// takes the FP64 adds.  4x4 6+6 (64.1M states) 10.08 -> 3.99 ms, 5+5 2.81 ->
+// 1.14, 1D L=16 8+8 15.98 -> 6.83, 3x4 6+6 137 -> 57 us; a real vector 4.08, one of
+// 99 % zeros 4.29 ms.  By the counters (4x4
 // 5+5) the ALU pipe is now 67 % busy, the FP64 pipe 29 %, issue 66 %, and the
 // largest stall is waiting for L2 (3.8 of 10.7 warps a scheduler).
 // ---------------------------------------------------------------------------
