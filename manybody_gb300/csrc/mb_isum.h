@@ -34,6 +34,9 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <cstddef>
+#include <type_traits>
+
 namespace mb {
 
 // PTX shifts: an amount above 63 gives 0 (or the sign), unlike C++'s
@@ -144,11 +147,7 @@ struct ISum2 {
       sr[k] = exponent((uint32_t)__double2hiint(v[k].x));
       si[k] = exponent((uint32_t)__double2hiint(v[k].y));
     }
-    shifts<N>(sr, si);
-    // Only zeros so far?  Rare, but for real or sparse vectors, whose sums went to
-    // FP64 without this look (4x4 6+6, real 11.0 ms, now 4.08; complex 3.94, now
-    // 3.99).  A loop of its own for warps that need it spilled: 4.07 and 4.42.
-    if (min(re.e, im.e) <= kISumLeast) {
+    auto look = [&] {
       uint32_t br = 0, bi = 0;
 #pragma unroll
       for (int k = 0; k < N; ++k) {
@@ -157,7 +156,8 @@ struct ISum2 {
       }
       re.see(br);
       im.see(bi);
-    }
+    };
+    shifts<N>(sr, si, look);
     int rh = 0, rl = 0, ih = 0, il = 0;
 #pragma unroll
     for (int k = 0; k < N; ++k) {
@@ -179,7 +179,7 @@ struct ISum2 {
       sr[k] = (int)((uint32_t)v[k].x & 1023u) + kISumLeast;
       si[k] = (int)((uint32_t)v[k].y & 1023u) + kISumLeast;
     }
-    shifts<N>(sr, si);
+    shifts<N>(sr, si, nullptr);
     int rh = 0, rl = 0, ih = 0, il = 0;
 #pragma unroll
     for (int k = 0; k < N; ++k) {
@@ -207,9 +207,15 @@ struct ISum2 {
     return (h + h) | (uint32_t)__double2loint(v);
   }
 
-  // exponents -> right shifts, the sums brought to larger exponents first
-  template <int N>
-  __device__ __forceinline__ void shifts(int (&sr)[N], int (&si)[N]) {
+  // Exponents -> right shifts, the sums brought to larger exponents first.  look
+  // (undecoded terms) runs while a sum holds only zeros: rare, but for real or
+  // sparse vectors, whose sums went to FP64 without it (4x4 6+6 real 11.0 ms, now
+  // 4.14, 99 % zeros 4.38).  It shares the branch that grows the sums: one of its
+  // own cost every vector 1.2 % (3.96 -> 4.01 ms, now 3.94), a loop of its own for
+  // the warps that need it spilled (4.07).
+  template <int N, typename Look>
+  __device__ __forceinline__ void shifts(int (&sr)[N], int (&si)[N], Look look) {
+    constexpr bool kLook = !std::is_same<Look, std::nullptr_t>::value;
     int any = 0;
 #pragma unroll
     for (int k = 0; k < N; ++k) {
@@ -217,20 +223,25 @@ struct ISum2 {
       si[k] = im.e - si[k];
       any |= sr[k] | si[k];
     }
-    if (any < 0) {  // rare after the first terms
-      const int er = re.e, ei = im.e;
-      int lr = sr[0], li = si[0];
+    if ((kLook ? any | (min(re.e, im.e) - (kISumLeast + 1)) : any) < 0) {  // rare after the first terms
+      if (!kLook || any < 0) {
+        const int er = re.e, ei = im.e;
+        int lr = sr[0], li = si[0];
 #pragma unroll
-      for (int k = 1; k < N; ++k) {
-        lr = min(lr, sr[k]);
-        li = min(li, si[k]);
+        for (int k = 1; k < N; ++k) {
+          lr = min(lr, sr[k]);
+          li = min(li, si[k]);
+        }
+        re.grow(lr);
+        im.grow(li);
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+          sr[k] += re.e - er;
+          si[k] += im.e - ei;
+        }
       }
-      re.grow(lr);
-      im.grow(li);
-#pragma unroll
-      for (int k = 0; k < N; ++k) {
-        sr[k] += re.e - er;
-        si[k] += im.e - ei;
+      if constexpr (kLook) {
+        if (min(re.e, im.e) <= kISumLeast) look();
       }
     }
   }

@@ -222,9 +222,9 @@ static int max_smem_optin() {
 // converts them and does the diagonal, the affine part and the dots.  A staged
 // row is decoded once (each element is a down neighbour about 16 times), up
 // neighbours as they arrive; a row or a sum outside the integer sums' range
-// takes the FP64 adds.  4x4 6+6 (64.1M states) 10.08 -> 3.99 ms, 5+5 2.81 ->
-// 1.14, 1D L=16 8+8 15.98 -> 6.83, 3x4 6+6 137 -> 57 us; a real vector 4.08, one of
-// 99 % zeros 4.29 ms.  By the counters (4x4
+// takes the FP64 adds.  4x4 6+6 (64.1M states) 10.08 -> 3.94 ms, 5+5 2.81 ->
+// 1.12, 1D L=16 8+8 15.98 -> 6.83, 3x4 6+6 137 -> 57 us; a real vector 4.14, one of
+// 99 % zeros 4.38 ms.  By the counters (4x4
 // 5+5) the ALU pipe is now 67 % busy, the FP64 pipe 29 %, issue 66 %, and the
 // largest stall is waiting for L2 (3.8 of 10.7 warps a scheduler).
 // ---------------------------------------------------------------------------
@@ -689,8 +689,10 @@ __device__ __forceinline__ float flip_sign(float v, uint32_t e) {
   return __int_as_float(__float_as_int(v) ^ (int)(e & 0x80000000u));
 }
 
+// (complex128 recurrences: 64 registers, four blocks an SM; with 72, 14.9 -> 16.9 ms
+// for 20 Lanczos steps of 4x4 5+5, K = (0,0))
 template <typename T, int DOTS, int LPR>
-__global__ void __launch_bounds__(kCsrThreads)
+__global__ void __launch_bounds__(kCsrThreads, sizeof(T) == 8 && (DOTS == 1 || DOTS == 2) ? 4 : 0)
 k_csr_apply(int64_t n, const int64_t* __restrict__ rp, const int32_t* __restrict__ ci,
             const typename C2<T>::type* __restrict__ val, const double* __restrict__ diag, T off,
             const typename C2<T>::type* __restrict__ x, typename C2<T>::type* y, T scale, T shift,

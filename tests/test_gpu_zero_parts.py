@@ -33,7 +33,9 @@ def time_us(torch, f):
 @pytest.mark.parametrize("space", ["lattice", "momentum"])
 def test_zero_parts_cost_no_more(mb, cuda, space, kind):
     """Beside a full complex vector (2.5 and 1.9 times as long where zeros went to
-    FP64): a tenth more for the look at the zeros and the clock."""
+    FP64): the look at a word of zeros is some 30 instructions beside its 150, in
+    half of the words, and a sparse sum grows at any word: an eighth, and as much
+    for the clock."""
     torch = cuda
     basis, model = lattice(mb, (4, 4), 4, 4) if space == "lattice" else momentum(mb, 8, (0, 0))
     op = mb.GpuHubbardOperator(basis, model, mb.PREC_F64)
@@ -50,7 +52,7 @@ def test_zero_parts_cost_no_more(mb, cuda, space, kind):
         x[x.numel() // 3] = 1
     y = op.empty()
     t = [time_us(torch, lambda v=v: op.apply(v, order=mb.ORDER_TENSOR, out=y)) for v in (full, x, full)]
-    assert t[1] <= 1.1 * max(t[0], t[2]), t
+    assert t[1] <= 1.25 * max(t[0], t[2]), t
 
 
 @pytest.mark.parametrize("case", [((6,), 3, 3), ((3, 3), 4, 5), ((17,), 1, 8), "momentum"])
