@@ -89,11 +89,24 @@ __device__ __forceinline__ double krylov_scale(const KrylovStep& s, int j) {
   return j > 0 ? __ldcg(s.beta + j - 1) : 1.0;
 }
 
-// (scale, factor of z) of a Lanczos step's apply
-__device__ __forceinline__ void step_coefs(const KrylovStep& s, double (&c)[2]) {
+// Whether a step with s_j is past the recurrence's end, ||u_j|| <= kTol: the host,
+// which looks at several steps at once, has queued it already.  Such a step does
+// nothing (its rows would be infinities and NaN, through the FP64 sums); its
+// apply hands the end on to the next one (end_step).  A replay (no ticket) has
+// no such steps.
+__device__ __forceinline__ bool krylov_over(const KrylovStep& s, double sj) {
+  return s.ticket && s.j > 0 && sj <= kTol;
+}
+__device__ __forceinline__ void end_step(const KrylovStep& s) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) s.beta[s.j] = 0.0;
+}
+
+// (scale, factor of z) of a Lanczos step's apply; true: it is past the end
+__device__ __forceinline__ bool step_coefs(const KrylovStep& s, double (&c)[2]) {
   const double sj = krylov_scale(s, s.j);
   c[0] = s.scale / sj;
   c[1] = s.j > 0 ? -sj / krylov_scale(s, s.j - 1) : 0.0;
+  return krylov_over(s, sj);
 }
 
 // The last block of a launch to get here sums every block's partials (thread 0
@@ -276,7 +289,7 @@ __device__ __forceinline__ void apply_rows(
   // (scaled_by) five of an element's 13 FP64 instructions less.  4x4 5+5 1149 ->
   // 1121 us, 6+6 4.03 -> 3.95 ms, 14 sites 4+4 48.2 -> 45.2 us.
   __shared__ T s_diag[33];
-  const bool given = (DOTS & 1) && s_coef;
+  const bool given = (DOTS & 1) && s_coef;  // [3]: nothing to do (krylov_over)
   const bool tabled = kInt && !self_up && !self_dn;
   if (STAGED && threadIdx.x < kSlicedPads) {
     V2 zero;
@@ -298,6 +311,7 @@ __device__ __forceinline__ void apply_rows(
       return __ldg(x + (DOTS & kRefIn ? (int64_t)__ldg(v.out_perm + i) : i));
     };
     __syncthreads();
+    if (given && ri == blockIdx.x && s_coef[3] != T(0)) return;
     if (tabled && ri == blockIdx.x && (int)threadIdx.x <= v.L)
       s_diag[threadIdx.x] = (given ? s_coef[1] : dscale) * (ufold[threadIdx.x] - shift);
     const int u0 = __ldg(&v.up_loff[r]), nu = __ldg(&v.up_loff[r + 1]) - u0;
@@ -512,17 +526,18 @@ k_apply(OpView v, const typename C2<T>::type* __restrict__ x, typename C2<T>::ty
         T hop_coef, T dscale, T shift, T beta, const typename C2<T>::type* z,
         const T* __restrict__ ufold, const T* __restrict__ self_up, const T* __restrict__ self_dn,
         double* __restrict__ partials) {
-  __shared__ T s_coef[3];  // hop_coef, dscale, beta: read past apply_rows' barriers
+  __shared__ T s_coef[4];  // hop_coef, dscale, beta, over: read past apply_rows' barriers
   if ((DOTS & 1) && threadIdx.x == 0) {
     double c[2] = {0.0, 0.0};
-    if (v.step.alpha) step_coefs(v.step, c);
+    s_coef[3] = v.step.alpha && step_coefs(v.step, c) ? T(1) : T(0);
     s_coef[0] = v.step.alpha ? (T)(-v.t * c[0]) : hop_coef;
     s_coef[1] = v.step.alpha ? (T)c[0] : dscale;
     s_coef[2] = v.step.alpha ? (T)c[1] : beta;
   }
   apply_rows<T, STAGED, DOTS>(v, x, y, hop_coef, dscale, shift, beta, z, ufold, self_up, self_dn,
                               partials, DOTS & 1 ? s_coef : nullptr);
-  if ((DOTS & 7) && v.step.ticket) finish_step<false, DOTS & 7>(v.step);
+  if ((DOTS & 1) && s_coef[3] != T(0)) end_step(v.step);
+  else if ((DOTS & 7) && v.step.ticket) finish_step<false, DOTS & 7>(v.step);
 }
 
 // One engine step of a large slot through the fused complex64 apply: the
@@ -702,8 +717,13 @@ k_csr_apply(int64_t n, const int64_t* __restrict__ rp, const int32_t* __restrict
   const ISumForm form(base);
   if ((DOTS & 1) && step.alpha) {
     __shared__ double c[2];
-    if (threadIdx.x == 0) step_coefs(step, c);
+    __shared__ bool over;
+    if (threadIdx.x == 0) over = step_coefs(step, c);
     __syncthreads();
+    if (over) {  // no rows
+      n = 0;
+      end_step(step);
+    }
     scale = (T)c[0];
     beta = (T)c[1];
   }
@@ -997,8 +1017,14 @@ k_update(int64_t n, T c, const typename C2<T>::type* __restrict__ u,
   using V2 = typename C2<T>::type;
   if (!NORM && step.alpha) {
     __shared__ double s_c;
-    if (threadIdx.x == 0) s_c = -__ldcg(step.alpha + step.j) / krylov_scale(step, step.j);
+    __shared__ bool over;
+    if (threadIdx.x == 0) {
+      const double sj = krylov_scale(step, step.j);
+      s_c = -__ldcg(step.alpha + step.j) / sj;
+      over = krylov_over(step, sj);
+    }
     __syncthreads();
+    if (over) return;
     c = (T)s_c;
   }
   DotAcc<T> acc;

@@ -977,7 +977,8 @@ struct Krylov {
   }
 
   // The recurrence (lanczos.h:25-36,113-121) without re-orthogonalisation: the
-  // steps between two looks at the scalars are queued at once.
+  // steps between two looks at the scalars are queued at once; those past a
+  // breakdown do nothing (krylov_over).
   static constexpr int64_t kPlainLook = 64;
   int64_t plain_steps(const void* b, int64_t k, double scale, std::vector<double>& alphas,
                       std::vector<double>& betas, double b_norm, double conv_tol, int check_every,
