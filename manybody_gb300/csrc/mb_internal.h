@@ -704,6 +704,16 @@ inline bool writes_reference(int precision, int64_t dim) {
          (precision == MB_PREC_F32 ? 8 : 16) * dim < 2 * kTileBytes;
 }
 bool apply_prefetches(const OpView& v, int precision);
+// Threads of an apply's CTAs, `threads` where there are rows enough for `total`
+// threads an SM.  Fewer rows, one CTA each, would leave SMs half empty: the CTAs
+// grow (to `most`, or a column a thread) while all rows still run at once.  Apply,
+// us, with 256 threads and so: 4x4 2+4 (120 rows) complex128 31.6, 19.2, Q64 26.7,
+// 15.3; ring of 14, 1+7 (14 rows) 37.7, 22.6 and 19.7, 17.3.
+inline int threads_for_rows(int threads, int most, int total, int64_t rows, int64_t cols, int sms) {
+  while (threads < most && threads < cols && rows <= (int64_t)sms * (total / (2 * threads)))
+    threads *= 2;
+  return threads;
+}
 // Whether a reference-order call of a floating-point lattice operator is one
 // launch (kRefIn).  Every read of x then goes through the permutation, two loads
 // one after the other, so it pays where the launches and the moves are most of

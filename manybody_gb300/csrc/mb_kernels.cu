@@ -611,6 +611,9 @@ bool apply_prefetches(const OpView& v, int precision) {
 // us with 512, rows of up to 32 groups best with 256 (3x4 6+6: 22.6 -> 20.6 us),
 // longer ones with 512 (4x4 4+4: 55.6 against 59 with 256).  128 threads were
 // slower everywhere but on 1,001 columns.
+// Rows that are not staged take the most: their down hops come through L1, which
+// holds no second row (complex128 17 sites 4+8 2.40 ms, 2.65 with 256; 18 sites 5+7
+// 12.1, 12.9; complex64 18 sites 5+7 4.62, 4.83).
 struct ApplyCtas {
   int threads, per_sm;
 };
@@ -618,11 +621,13 @@ static ApplyCtas apply_ctas(const OpView& v, int precision) {
   const bool f32 = precision == MB_PREC_F32;
   const int most = f32 ? kApplyMax<float> : kApplyMax<double>;
   const int total = f32 ? kApplyResident<float> : kApplyResident<double>;
-  const size_t row = apply_smem(v, precision, apply_staged(v, precision)) + 3072;
+  if (!apply_staged(v, precision)) return {most, total / most};
+  const size_t row = apply_smem(v, precision, true) + 3072;
   const size_t sm = (size_t)max_smem_optin() + 1024;
   int threads = f32 && v.Dd > 32 * 32 ? 512 : 256;
   while (threads < most && (size_t)(total / threads) * row > sm)
     threads = std::min(2 * threads, most);
+  threads = threads_for_rows(threads, most, total, v.Du, v.Dd, num_sms());
   return {threads, total / threads};
 }
 

@@ -748,17 +748,20 @@ static size_t q_apply_smem(const OpView& v, bool staged, bool ups, bool ts) {
 // each other's staging and barriers and leave fewer warps without a column group
 // in a row's last round (4x4 4+4, 1,820 columns:
 // 113 -> 101 us with 256; 3x4 5+4, 495: 26.7 -> 20.6; 4x4 5+5, 4,368: 677 -> 647
-// with 512).
+// with 512).  Rows that are not staged, and few rows, as in apply_ctas and
+// threads_for_rows (17 sites 4+8 1.64 ms, 1.89 with 256; 2+8 89 and 265 us).
 struct QCtas {
   int threads, per_sm;
 };
 static QCtas q_ctas(const OpView& v) {
   if (v.table_stage) return {kQThreads, 1};  // the warps' buffers take the rest
-  const bool staged = q_apply_smem(v, true, false, false) + 2048 <= (size_t)smem_optin();
-  const size_t row = q_apply_smem(v, staged, false, false) + 5120;
+  if (q_apply_smem(v, true, false, false) + 2048 > (size_t)smem_optin()) return {kQThreads, 1};
+  const size_t row = q_apply_smem(v, true, false, false) + 5120;
   int threads = 256;
   while (threads < kQThreads && (size_t)(kQThreads / threads) * row > (size_t)smem_optin() + 1024)
     threads *= 2;
+  const int64_t rows = v.Du * std::max(v.row_split, 1);
+  threads = threads_for_rows(threads, kQThreads, kQThreads, rows, v.Dd, sm_count());
   return {threads, kQThreads / threads};
 }
 
