@@ -220,6 +220,19 @@ OrderTiles order_tiles(int L, const SpinSector& up, const SpinSector& dn, int sl
   return out;
 }
 
+int64_t order_tile_count(int L, int n_up, int n_dn, int slots) {
+  const Binom& B = binom_table();
+  const int h = std::min(kTileHigh, (L + 1) / 2), m = L - h;
+  int64_t count = 0;
+  for (int u = std::max(0, n_up - h); u <= std::min(m, n_up); ++u)
+    for (int d = std::max(0, n_dn - h); d <= std::min(m, n_dn); ++d) {
+      const int64_t pairs = (int64_t)B.c[h][n_up - u] * B.c[h][n_dn - d];
+      const int64_t step = kTileWarps * std::max<int64_t>(1, slots / (pairs | 1));
+      count += B.c[m][u] * ((B.c[m][d] + step - 1) / step);
+    }
+  return count;
+}
+
 SignedLists signed_lists(const HopTable& t, int64_t D) {
   SignedLists s;
   s.off.resize((size_t)D + 1);

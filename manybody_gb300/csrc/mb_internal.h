@@ -542,6 +542,8 @@ struct OrderTiles {
 };
 // slots: a warp's shared-memory elements (at least kTilePairs + 1, below 1024)
 OrderTiles order_tiles(int L, const SpinSector& up, const SpinSector& dn, int slots);
+// how many tiles that makes
+int64_t order_tile_count(int L, int n_up, int n_dn, int slots);
 }  // namespace mb
 
 struct mb_op_s {
@@ -693,6 +695,14 @@ void launch_scatter(int precision, int64_t n, const int32_t* perm, const void* s
 // complex128, 53 MB: 26 against 38 us; 1D L=14 7+7, 188 MB: 135 against 100 us;
 // 4x4 6+6, 1.03 GB: 1.2 ms against 0.52; complex64 0.85 ms against 0.27).
 constexpr int64_t kTileBytes = 100000000;
+// and whose tiles are full enough for their blocks' 128 threads.  Tiles run along
+// the low Down occupations of one Up one: with few Down particles there are many
+// tiles of a few elements (and a table of them as large).  One move to tensor order
+// and one back, Q64, us, by tiles and by the gather: 22 sites 11+1 (39 elements a
+// tile) 1511, 1269 and 322, 141; 32 sites 4+2 (245) 556, 422 and 315, 181; 20 sites
+// 10+2 (226) 994, 786 and 731, 475; 18 sites 9+3 (654) 696, 492 and 810, 588; 20
+// sites 7+3 (716) 1458, 989 and 1974, 1692.
+constexpr int64_t kTileFill = 450;
 // Whether an apply of a reference-order call writes its result itself (kRefOut).
 // complex128 always: its apply hides the scattered stores (reference-order call,
 // ms, against a tile move after it: 4x4 5+5 1.38 / 1.48, 6+6 4.71 / 5.05, 1D L=16

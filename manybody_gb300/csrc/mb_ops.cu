@@ -505,14 +505,14 @@ constexpr int kTileSlots32 = 1016, kTileSlots64 = 512;
 RowOrder op_row_order(mb_op_s* op) {
   RowOrder none;
   none.perm = op_perm(op);
-  if (op->natural_order || op->view.n_blocks ||
-      (int64_t)elem_bytes(op->precision) * op->dim < kTileBytes)
-    return none;
+  const size_t es = elem_bytes(op->precision);
+  if (op->natural_order || op->view.n_blocks || (int64_t)es * op->dim < kTileBytes) return none;
+  const int slots = es == 8 ? kTileSlots32 : kTileSlots64;
+  if (op->dim < kTileFill * order_tile_count(op->L, op->n_up, op->n_down, slots)) return none;
   std::lock_guard<std::mutex> lk(op->mu);
   if (!op->order.tiles) {
-    const size_t es = elem_bytes(op->precision);
     RowOrder o;
-    o.warp_slots = es == 8 ? kTileSlots32 : kTileSlots64;
+    o.warp_slots = slots;
     o.warp_bytes = (int)((es + sizeof(int32_t)) * (size_t)o.warp_slots);
     const OrderTiles t = order_tiles(op->L, make_spin_sector(op->L, op->n_up),
                                      make_spin_sector(op->L, op->n_down), o.warp_slots);
