@@ -488,7 +488,7 @@ void fill_fused_tables(OpView& v, const HopTable& tu, const HopTable& td, int64_
 
 namespace mb {
 // Workspaces kept between calls (mb_pool.cu).  Device memory by stream order
-// (bytes = 0: nullptr), what the device's pool holds idle, and giving that back;
+// (bytes = 0: nullptr; what is too large to be kept by cudaMalloc), what the device's pool holds idle, and giving that back;
 // cudaMalloc that gives it back where it would not fit otherwise; page-locked
 // host memory (given back with the size it was taken with).  Operators and
 // engines hold the pools while they live.

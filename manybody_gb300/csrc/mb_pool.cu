@@ -10,9 +10,16 @@
 // operator and engine of the process are destroyed, and what is idle whenever
 // an allocation does not fit otherwise.  A block is freed in the order of the
 // stream it was used on; CUDA's pools serve any thread and stream.
+//
+// A block that would take the pool past twice what it keeps is cudaMalloc's: it
+// could not be kept, and the pool maps and unmaps memory more slowly than
+// cudaMalloc and cudaFree do.  A complex64 ground state of 1D L=16 8+8 (U = 2, 100
+// steps, 132 GB of kept Lanczos vectors) from the second call on: 0.71 ->
+// 0.54 s (0.545 the first; 0.65 with all of it cudaMalloc's and a slower apply).
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <unordered_set>
 #include <vector>
 
 #include "mb_internal.h"
@@ -31,10 +38,12 @@ struct Pinned {
 
 std::mutex g_mu;
 cudaMemPool_t g_pool[kPoolDevices] = {};
+uint64_t g_keep[kPoolDevices] = {};        // bytes kept mapped
+std::unordered_set<void*> g_apart;         // blocks of cudaMalloc
 std::vector<Pinned> g_pinned;  // idle
 int64_t g_holders = 0;
 
-cudaMemPool_t device_pool() {
+cudaMemPool_t device_pool(uint64_t* keep_out = nullptr) {
   int dev = 0;
   MB_CUDA(cudaGetDevice(&dev));
   MB_REQUIRE(dev >= 0 && dev < kPoolDevices, MB_ERR_CAPACITY, "device ordinal above 63");
@@ -51,8 +60,20 @@ cudaMemPool_t device_pool() {
     uint64_t keep = total_b / 32;
     MB_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
     g_pool[dev] = pool;
+    g_keep[dev] = keep;
   }
+  if (keep_out) *keep_out = g_keep[dev];
   return g_pool[dev];
+}
+
+constexpr size_t kLargeBlock = size_t(64) << 20;  // smaller ones are the pool's without a look
+
+// Whether a block would take the pool past twice what it keeps.
+bool too_large(cudaMemPool_t pool, size_t bytes, uint64_t keep) {
+  uint64_t used = 0;
+  if (bytes < kLargeBlock) return false;
+  MB_CUDA(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used));
+  return used + bytes > 2 * keep;
 }
 
 }  // namespace
@@ -60,7 +81,14 @@ cudaMemPool_t device_pool() {
 void* ws_alloc(size_t bytes, cudaStream_t st) {
   if (!bytes) return nullptr;
   void* p = nullptr;
-  cudaMemPool_t pool = device_pool();
+  uint64_t keep = 0;
+  cudaMemPool_t pool = device_pool(&keep);
+  if (too_large(pool, bytes, keep)) {
+    MB_CUDA(dev_malloc(&p, bytes));
+    std::lock_guard<std::mutex> lk(g_mu);
+    g_apart.insert(p);
+    return p;
+  }
   if (cudaMallocFromPoolAsync(&p, bytes, pool, st) != cudaSuccess) {
     cudaGetLastError();
     ws_trim();
@@ -70,7 +98,14 @@ void* ws_alloc(size_t bytes, cudaStream_t st) {
 }
 
 void ws_free(void* p, cudaStream_t st) {
-  if (p) cudaFreeAsync(p, st);
+  if (!p) return;
+  bool apart;
+  {
+    std::lock_guard<std::mutex> lk(g_mu);
+    apart = g_apart.erase(p) > 0;
+  }
+  if (apart) cudaFree(p);
+  else cudaFreeAsync(p, st);
 }
 
 size_t ws_idle() {

@@ -1,0 +1,44 @@
+"""Solver workspaces: what a call takes beyond what is kept between calls."""
+import time
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def test_large_workspaces_cost_no_more_the_second_time(mb, cuda):
+    """166 million states, 100 kept complex64 vectors (132 GB): the second call maps its
+    memory anew as the first does (a third longer where the pool gave back what it
+    could not keep at the next call's start): within an eighth."""
+    torch = cuda
+    torch.cuda.empty_cache()
+    basis = mb.FermionBasis.with_fixed_particle_number_and_spin(16, 16, 0)
+    op = mb.GpuHubbardOperator(basis, mb._Hubbard(1.0, 2.0, (16,)), mb.PREC_F32)
+    x = op.seed_vector(1, order=mb.ORDER_TENSOR)
+    t, e = [], []
+    for _ in range(3):
+        torch.cuda.synchronize()
+        t0 = time.perf_counter()
+        e.append(mb.find_min_eigenpair(op, 100, x, order=mb.ORDER_TENSOR, want_vector=False,
+                                       refine=True).value)
+        t.append(time.perf_counter() - t0)
+    assert e[0] == e[1] == e[2]
+    assert min(t[1:]) <= 1.125 * t[0], t
+
+
+@pytest.mark.parametrize("order", ["tensor", "reference"])
+def test_blocks_beside_the_pool(mb, cuda, order):
+    """Calls whose blocks are partly the pool's and partly not give the results of
+    small ones, in any sequence."""
+    basis = mb.FermionBasis.with_fixed_particle_number_and_spin(16, 12, 0)
+    big = mb.GpuHubbardOperator(basis, mb._Hubbard(1.0, 4.0, (4, 4)), mb.PREC_F64)
+    small = mb.GpuHubbardOperator(mb.FermionBasis.with_fixed_particle_number_and_spin(8, 8, 0),
+                                  mb._Hubbard(1.0, 4.0, (8,)), mb.PREC_F64)
+    o = mb.ORDER_TENSOR if order == "tensor" else mb.ORDER_REFERENCE
+    sx, bx = small.seed_vector(1, order=o), big.seed_vector(1, order=o)
+    want = mb.time_evolve_state(small, sx, 0.2, order=o)
+    big_want = mb.time_evolve_state(big, bx, 0.05, 18, order=o)
+    for _ in range(2):
+        assert cuda.equal(mb.time_evolve_state(big, bx, 0.05, 18, order=o), big_want)
+        assert cuda.equal(mb.time_evolve_state(small, sx, 0.2, order=o), want)
