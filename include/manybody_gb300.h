@@ -73,6 +73,14 @@ int mb_alloc(void** dev_ptr, size_t bytes);
 int mb_free(void* dev_ptr);
 int mb_memcpy(void* dst, const void* src, size_t bytes, int kind);
 int mb_synchronize(void);
+/* Gives the library's idle workspaces back to the device.  Solver calls keep up to
+ * 1/32 of a device's memory mapped for the next call (workspaces of one call beyond
+ * that are given back when it ends) while an operator or engine lives; the library's
+ * own allocations take it back where they need it, those of other allocators (and
+ * other processes) find it in use until this call, or until the last operator and
+ * engine are destroyed.  Waits for the device; the next solver call maps its
+ * workspaces anew. */
+int mb_trim(void);
 
 /* ---- basis: FermionBasis (src/algebra/fermion/basis.h, src/algebra/basis.h:12-76)
  * mb_basis_create_fixed_spin replaces

@@ -95,6 +95,7 @@ SIGNATURES = {
     "mb_free": (C.c_int, [_vp]),
     "mb_memcpy": (C.c_int, [_vp, _vp, C.c_size_t, C.c_int]),
     "mb_synchronize": (C.c_int, []),
+    "mb_trim": (C.c_int, []),
     "mb_basis_create_fixed_spin": (C.c_int, [_i64, _i64, C.c_int, C.POINTER(_vp)]),
     "mb_basis_destroy": (C.c_int, [_vp]),
     "mb_basis_size": (C.c_int, [_vp, _i64p]),
@@ -206,6 +207,12 @@ def device_count() -> int:
     n = C.c_int(0)
     lib().mb_device_count(C.byref(n))
     return n.value
+
+
+def trim() -> None:
+    """Gives the idle workspaces that solver calls keep back to the device (for other
+    allocators near the memory's limit); the next solver call takes them anew."""
+    _check(lib().mb_trim())
 
 
 def _ptr(t) -> int:

@@ -1543,6 +1543,13 @@ int mb_synchronize(void) {
   return guard([&] { MB_CUDA(cudaDeviceSynchronize()); });
 }
 
+int mb_trim(void) {
+  return guard([&] {
+    require_device();
+    ws_trim();
+  });
+}
+
 int mb_op_create(mb_basis_t basis, mb_model_t model, int precision, mb_op_t* out) {
   return guard([&] {
     MB_REQUIRE(basis && model && out, MB_ERR_INVALID_ARG, "NULL argument");

@@ -127,10 +127,19 @@ size_t ws_idle() {
 }
 
 void ws_trim() {
-  cudaDeviceSynchronize();
-  std::lock_guard<std::mutex> lk(g_mu);
-  for (cudaMemPool_t pool : g_pool)
-    if (pool) cudaMemPoolTrimTo(pool, 0);
+  cudaMemPool_t pools[kPoolDevices];
+  {
+    std::lock_guard<std::mutex> lk(g_mu);
+    std::copy(g_pool, g_pool + kPoolDevices, pools);
+  }
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return;
+  for (int d = 0; d < kPoolDevices; ++d)
+    if (pools[d] && cudaSetDevice(d) == cudaSuccess) {
+      cudaDeviceSynchronize();  // blocks freed in the order of a stream are back
+      cudaMemPoolTrimTo(pools[d], 0);
+    }
+  cudaSetDevice(dev);
 }
 
 cudaError_t dev_malloc(void** p, size_t bytes) {

@@ -42,3 +42,24 @@ def test_blocks_beside_the_pool(mb, cuda, order):
     for _ in range(2):
         assert cuda.equal(mb.time_evolve_state(big, bx, 0.05, 18, order=o), big_want)
         assert cuda.equal(mb.time_evolve_state(small, sx, 0.2, order=o), want)
+
+
+def test_trim_gives_kept_workspaces_back(mb, cuda):
+    """A solver call keeps its workspaces; after trim() another allocator has them,
+    and the next call gives the same result."""
+    torch = cuda
+    basis = mb.FermionBasis.with_fixed_particle_number_and_spin(16, 10, 0)
+    op = mb.GpuHubbardOperator(basis, mb._Hubbard(1.0, 4.0, (4, 4)), mb.PREC_F32)
+    x = op.seed_vector(1)
+    free = lambda: torch.cuda.mem_get_info()[0]
+    mb.find_min_eigenpair(op, 2, x, want_vector=False)  # the operator's own tables
+    mb.trim()
+    before = free()
+    a = mb.find_min_eigenpair(op, 30, x, want_vector=True)
+    torch.cuda.synchronize()
+    assert free() < before - (1 << 30)  # 30 kept vectors of 153 MB
+    mb.trim()
+    vectors = (a.vector.numel() * a.vector.element_size() + (64 << 20))  # torch's, in its own blocks
+    assert free() >= before - vectors
+    b = mb.find_min_eigenpair(op, 30, x, want_vector=True)
+    assert a.value == b.value and torch.equal(a.vector, b.vector)
