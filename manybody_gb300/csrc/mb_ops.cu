@@ -828,6 +828,20 @@ struct Krylov {
     return s;
   }
 
+  // The scalars of a run that goes on to step `to`, those of its first `at` steps
+  // kept: k may be a bound that no run reaches.
+  void more_scalars(KrylovStep& s, int64_t at, int64_t to) {
+    if (to <= scalar_cap) return;
+    const KrylovStep old = s;
+    DevBuf buf = std::move(scalars);
+    const int64_t cap = std::max(2 * scalar_cap, to);
+    scalar_cap = 0;
+    s = scalars_for(cap, old.scale);
+    const size_t len = sizeof(double) * (size_t)at;
+    MB_CUDA(cudaMemcpyAsync(s.alpha, old.alpha, len, cudaMemcpyDeviceToDevice, st));
+    MB_CUDA(cudaMemcpyAsync(s.beta, old.beta, len, cudaMemcpyDeviceToDevice, st));
+  }
+
   // u_j of the plain recurrence: a kept column, else a rotating vector.
   void* plain_vec(int64_t j, bool keep_vectors) {
     if (keep_vectors && kept == j && keep_room(j)) kept = j + 1;
@@ -980,36 +994,41 @@ struct Krylov {
   // steps between two looks at the scalars are queued at once; those past a
   // breakdown do nothing (krylov_over).
   static constexpr int64_t kPlainLook = 64;
+  static constexpr int64_t kScalarSteps = 1024;  // steps' scalars at first
   int64_t plain_steps(const void* b, int64_t k, double scale, std::vector<double>& alphas,
                       std::vector<double>& betas, double b_norm, double conv_tol, int check_every,
                       bool keep_vectors) {
     const bool check = conv_tol > 0.0 && check_every > 0;
-    const KrylovStep s = scalars_for(k, scale);
-    std::vector<double> host(2 * (size_t)k);
+    KrylovStep s = scalars_for(std::min(k, kScalarSteps), scale);
+    std::vector<double> host;
     void* prev = nullptr;
     void* cur = plain_vec(0, keep_vectors);
     launch_axpby(prec, n, 1.0 / b_norm, 0.0, b, 0.0, 0.0, cur, nullptr, 0, st);
     int64_t steps = 0;
     for (int64_t at = 0; at < k;) {
-      const int64_t to = std::min(k, at + (check ? check_every : kPlainLook));
+      int64_t to = std::min(k, at + kPlainLook);
+      if (check) to = std::min(to, (at / check_every + 1) * check_every);
+      more_scalars(s, at, to);
       for (int64_t j = at; j < to; ++j) {
         void* next = plain_vec(j + 1, keep_vectors && j + 1 < k);
         plain_step(s, j, prev, cur, next);
         prev = cur;
         cur = next;
       }
-      const size_t len = sizeof(double) * (size_t)(to - at);
-      MB_CUDA(cudaMemcpyAsync(host.data() + at, s.alpha + at, len, cudaMemcpyDeviceToHost, st));
-      MB_CUDA(cudaMemcpyAsync(host.data() + k + at, s.beta + at, len, cudaMemcpyDeviceToHost, st));
+      const size_t n_new = (size_t)(to - at), len = sizeof(double) * n_new;
+      host.resize(2 * n_new);
+      MB_CUDA(cudaMemcpyAsync(host.data(), s.alpha + at, len, cudaMemcpyDeviceToHost, st));
+      MB_CUDA(cudaMemcpyAsync(host.data() + n_new, s.beta + at, len, cudaMemcpyDeviceToHost, st));
       MB_CUDA(cudaStreamSynchronize(st));
-      for (; at < to; ++at) {
-        alphas.push_back(host[(size_t)at]);
+      for (size_t i = 0; at < to; ++at, ++i) {
+        alphas.push_back(host[i]);
         steps += 1;
-        const double beta = host[(size_t)(k + at)];
+        const double beta = host[n_new + i];
         if (beta <= kTol) return steps;
         if (at + 1 < k) betas.push_back(beta);
       }
-      if (check && steps < k && settled(alphas, betas, conv_tol)) return steps;
+      if (check && steps < k && steps % check_every == 0 && settled(alphas, betas, conv_tol))
+        return steps;
     }
     return steps;
   }
