@@ -754,7 +754,8 @@ static void apply_affine(mb_op_s* op, const void* x, void* y, double scale, doub
                  kRefOut | kRefIn, st);
     return;
   }
-  auto& s = scratch_for(op, st, fused && beta == 0.0 ? 1 : 2);
+  // (both from a stream's first call on: a later one, with z, may be in a capture)
+  auto& s = scratch_for(op, st, 2);
   to_tensor(op, x, s.a, order, st);
   const void* zt = nullptr;
   if (beta != 0.0) {
