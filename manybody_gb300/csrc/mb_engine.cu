@@ -85,28 +85,41 @@ constexpr int kModeLanczos = kEngLanczos;
 constexpr int kModeReplay = kEngReplay;
 constexpr int kModeCheb = kEngCheb;   // T_{k+1} = 2 Ht T_k - T_{k-1} (T_1 = Ht T_0)
 
-// A warp's sum of compensated float pairs, in lane 0, the tree in pairs too (the
-// error of a step is past the pairs' last bit, 2^-48): an FP64 add takes 17
-// cycles of the SM's one slow pipe for every warp, and a row's sums in FP64 (16
-// instructions in each of its 8 warps) were half of a step's apply.
-__device__ __forceinline__ float2 eng_warp_sum(float hi, float lo) {
+// A warp's sum of compensated float pairs, in lane 0: as integers in units of the
+// largest term (float_fixed), so that it is as exact as FP64 adds of the pairs and
+// costs one conversion: an FP64 add takes 17 cycles of the SM's one slow pipe for
+// every warp, and a row's sums in FP64 (16 instructions in each of its 8 warps)
+// were half of a step's apply.  48 requests on rings of 8, 10 and 12 sites, 100 steps:
+// 71.6 ms, 71.3 with the tree in float pairs (which lost bits below 2^-48).
+struct EngSum {
+  long long a;
+  int top;  // 255: a holds the bits of a double (infinities, NaN)
+};
+__device__ __forceinline__ EngSum eng_warp_sum(float hi, float lo) {
+  EngSum s;
+  s.top = (int)__reduce_max_sync(0xffffffffu, (unsigned)max(float_top(hi), float_top(lo)));
+  if (s.top == 255) {
+    double v = (double)hi + (double)lo;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const float h = __shfl_down_sync(0xffffffffu, hi, o);
-    const float l = __shfl_down_sync(0xffffffffu, lo, o);
-    const float s = hi + h, b = s - hi;
-    lo += ((hi - (s - b)) + (h - b)) + l;
-    hi = s;
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    s.a = __double_as_longlong(v);
+    return s;
   }
-  return make_float2(hi, lo);
+  s.a = float_fixed(hi, s.top) + float_fixed(lo, s.top);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s.a += __shfl_down_sync(0xffffffffu, s.a, o);
+  return s;
 }
-__device__ __forceinline__ double eng_pair(float2 a) { return (double)a.x + (double)a.y; }
+__device__ __forceinline__ double eng_value(const EngSum& s) {
+  return s.top == 255 ? __longlong_as_double(s.a)
+                      : __ll2double_rn(s.a) * __hiloint2double((s.top - 183 + 1023) << 20, 0);
+}
 
-// The block's sums of its warps' pairs into part and (TWO) part2, in a fixed tree.
+// The block's sums of its warps' sums into part and (TWO) part2, in a fixed tree.
 constexpr int kEngRowWarps = 8;
 template <bool TWO>
-__device__ __forceinline__ void eng_row_sums(float2 xy, float2 yy, float2 (*red)[2], double* part,
-                                             double* part2) {
+__device__ __forceinline__ void eng_row_sums(const EngSum& xy, const EngSum& yy, EngSum (*red)[2],
+                                             double* part, double* part2) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (lane == 0) {
     red[warp][0] = xy;
@@ -114,8 +127,8 @@ __device__ __forceinline__ void eng_row_sums(float2 xy, float2 yy, float2 (*red)
   }
   __syncthreads();
   if (warp != 0) return;
-  double a = lane < kEngRowWarps ? eng_pair(red[lane][0]) : 0.0, b = 0.0;
-  if (TWO && lane < kEngRowWarps) b = eng_pair(red[lane][1]);
+  double a = lane < kEngRowWarps ? eng_value(red[lane][0]) : 0.0, b = 0.0;
+  if (TWO && lane < kEngRowWarps) b = eng_value(red[lane][1]);
 #pragma unroll
   for (int o = kEngRowWarps / 2; o > 0; o >>= 1) {
     a += __shfl_down_sync(0xffffffffu, a, o);
@@ -217,8 +230,8 @@ k_eng_apply(const SlotDesc* __restrict__ slots, const int2* __restrict__ items, 
           hi2 = s1;
         }
       }
-      dxy = eng_pair(eng_warp_sum(hi, lo));
-      if (cheb) dyy = eng_pair(eng_warp_sum(hi2, lo2));
+      dxy = eng_value(eng_warp_sum(hi, lo));
+      if (cheb) dyy = eng_value(eng_warp_sum(hi2, lo2));
     }
     if (lane == 0 && part) {
       part[s.item0 + item.y] = dxy;
@@ -242,7 +255,7 @@ k_eng_apply_rows(const SlotDesc* __restrict__ slots, const int2* __restrict__ it
   extern __shared__ __align__(16) unsigned char smem[];
   float2* srow = reinterpret_cast<float2*>(smem);
   uint32_t* s_up = reinterpret_cast<uint32_t*>(smem + sizeof(float2) * (max_cols + kSlicedPads));
-  __shared__ float2 red[kEngRowWarps][2];
+  __shared__ EngSum red[kEngRowWarps][2];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (int it = blockIdx.x; it < n_items; it += gridDim.x) {
     const int2 item = items[it];
@@ -358,7 +371,7 @@ k_eng_apply_rows(const SlotDesc* __restrict__ slots, const int2* __restrict__ it
         hi2 = s1;
       }
     }
-    const float2 xy = eng_warp_sum(hi, lo);
+    const EngSum xy = eng_warp_sum(hi, lo);
     if (cheb) eng_row_sums<true>(xy, eng_warp_sum(hi2, lo2), red, part + pidx, part2 + pidx);
     else eng_row_sums<false>(xy, xy, red, part + pidx, part2 + pidx);
   }
@@ -435,7 +448,7 @@ k_eng_update(const SlotDesc* __restrict__ slots, const int2* __restrict__ items,
         lo += ((hi - (s1 - bp)) + (p - bp)) + pe;
         hi = s1;
       }
-      nn = eng_pair(eng_warp_sum(hi, lo));
+      nn = eng_value(eng_warp_sum(hi, lo));
     }
     if (lane == 0) part[it] = nn;
   }
@@ -826,7 +839,7 @@ __device__ __forceinline__ float2 lz(float2 a, float f) {
 template <bool CHEB>
 __device__ void p_apply_row(const SlotDesc& s, const SlotNow& n, int64_t r, int64_t pidx,
                             double* part, double* part2, float2* srow, uint32_t* s_up,
-                            float2 (*red)[2], int step) {
+                            EngSum (*red)[2], int step) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int k = n.k;
   const bool lanczos = n.mode == kModeLanczos && k < n.kmax;
@@ -955,7 +968,7 @@ __device__ void p_apply_row(const SlotDesc& s, const SlotNow& n, int64_t r, int6
       eng_acc(hi2, lo2, o.y, o.y);
     }
   }
-  const float2 xy = eng_warp_sum(hi, lo);
+  const EngSum xy = eng_warp_sum(hi, lo);
   if constexpr (CHEB) eng_row_sums<true>(xy, eng_warp_sum(hi2, lo2), red, part + pidx, part2 + pidx);
   else eng_row_sums<false>(xy, xy, red, part + pidx, part2 + pidx);
 }
@@ -1035,8 +1048,8 @@ __device__ void p_apply_warp_row(const SlotDesc& s, const SlotNow& n, int64_t r,
         eng_acc(hi2, lo2, o.y, o.y);
       }
     }
-    dxy = eng_pair(eng_warp_sum(hi, lo));
-    if (cheb) dyy = eng_pair(eng_warp_sum(hi2, lo2));
+    dxy = eng_value(eng_warp_sum(hi, lo));
+    if (cheb) dyy = eng_value(eng_warp_sum(hi2, lo2));
   }
   if (lane == 0) {
     part[pidx] = dxy;
@@ -1121,7 +1134,7 @@ __device__ void p_update_row(const SlotDesc& s, const SlotNow& n, int64_t r, int
       eng_acc(hi, lo, o.x, o.x);
       eng_acc(hi, lo, o.y, o.y);
     }
-    double nn = eng_pair(eng_warp_sum(hi, lo));
+    double nn = eng_value(eng_warp_sum(hi, lo));
     if (lane == 0) part[it] = nn;
     return;
   }
@@ -1215,7 +1228,7 @@ constexpr int kEngPCtas = 5;
 __global__ void __launch_bounds__(kEngPWarps * 32, kEngPCtas)
 k_eng_persistent(EngPersistArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ float2 red[kEngRowWarps][2];
+  __shared__ EngSum red[kEngRowWarps][2];
   __shared__ double sred[kEngPWarps * 32], sred2[kEngPWarps * 32];
   const int warp = threadIdx.x >> 5;
   float2* srow = reinterpret_cast<float2*>(smem);

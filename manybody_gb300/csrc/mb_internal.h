@@ -6,6 +6,7 @@
 
 #include <condition_variable>
 #include <cstdio>
+#include <cstring>
 #include <functional>
 #include <map>
 #include <memory>
@@ -313,6 +314,24 @@ inline int isum_base(int64_t terms, int least) {
   while ((int64_t(1) << (b - 1)) < terms) ++b;
   return b;
 }
+// Sums of floats over a warp as 64-bit integers.  With `top` the largest of the
+// terms' biased exponents (float_top, below 255), a term is a whole number of
+// units 2^(top - 183), cut towards zero below one (none of a term within 2^-32 of
+// the largest is): 57 bits, 64 terms in 62.
+__host__ __device__ inline int float_top(float v) {
+  uint32_t b;
+  memcpy(&b, &v, 4);
+  return (int)(b >> 23 & 255u);
+}
+__host__ __device__ inline long long float_fixed(float v, int top) {
+  uint32_t b;
+  memcpy(&b, &v, 4);
+  const int ex = (int)(b >> 23 & 255u), up = (ex ? ex : 1) - top + 33;
+  const unsigned long long m = (b & 0x7FFFFFu) | (ex ? 0x800000u : 0u);
+  const long long q = (long long)(up >= 0 ? m << up : up > -32 ? m >> -up : 0ull);
+  return (int32_t)b < 0 ? -q : q;
+}
+
 // The same table with 16-bit entries (index | negative << 15; D + kSlicedPads
 // must stay below 2^15), a lane's slots 8i..8i+7 in one 16-byte word.
 struct SlicedTable16 {
