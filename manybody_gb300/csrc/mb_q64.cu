@@ -237,10 +237,10 @@ void launch_q_reduce128(const void* part, int nblocks, double* out, cudaStream_t
 // per block as 128-bit integers (partials: 4 words a block; k_q_reduce128
 // sums them).
 //
-// One CTA of 1024 threads per SM walks the rows r_up in the row schedule's
-// order (reverse Cuthill-McKee: rows in flight together share neighbour rows
-// in L2).  Per row: the row x[r,:] and sixteen zero elements go to shared
-// memory, then warp w takes the 32-column groups g = w, w + 32, ...:
+// CTAs of 256 to 1024 threads, 1024 an SM (q_ctas), walk the rows r_up in the row
+// schedule's order (reverse Cuthill-McKee: rows in flight together share
+// neighbour rows in L2).  Per row: the row x[r,:] and sixteen zero elements go to
+// shared memory, then warp w of the CTA's n takes the 32-column groups g = w, w + n, ...:
 //   down hops: sliced table, one coalesced 16-byte load per lane for four
 //     slots; entry = neighbour index in the staged row | sign << 31, in an
 //     order that keeps each quarter warp on distinct bank groups; padding
