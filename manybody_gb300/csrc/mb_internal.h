@@ -676,9 +676,9 @@ void launch_apply(const OpView& v, int precision, const void* x, void* y, double
 int apply_grid(const OpView& v, int precision);
 void launch_reduce(const double* partials, int nblocks, int ncomp, double* out, cudaStream_t st);
 int blas_grid(int64_t n);
-// y = a*x + b*y (complex coefficients); dots of the result if dot_mode.
+// y = a*x + b*y (complex coefficients)
 void launch_axpby(int precision, int64_t n, double ar, double ai, const void* x, double br,
-                  double bi, void* y, double* partials, int dot_mode, cudaStream_t st);
+                  double bi, void* y, cudaStream_t st);
 // w += c u (c real; a Lanczos step takes its own), <w,w> of the result in comp 1
 void launch_update(int precision, int64_t n, double c, const void* u, void* w, double* partials,
                    const KrylovStep& step, cudaStream_t st);

@@ -960,12 +960,11 @@ int blas_grid(int64_t n) {
 }
 
 // y = a*x + b*y, complex a, b (REAL: ai = bi = 0, half the products, on the
-// slow FP64 pipe the longer part of a pass); dot_mode bit1: <y,y> of the result.
-template <typename T, int DOTS, bool REAL>
+// slow FP64 pipe the longer part of a pass).
+template <typename T, bool REAL>
 __global__ void k_axpby(int64_t n, T ar, T ai, const typename C2<T>::type* __restrict__ x, T br,
-                        T bi, typename C2<T>::type* __restrict__ y, double* __restrict__ partials) {
+                        T bi, typename C2<T>::type* __restrict__ y) {
   using V2 = typename C2<T>::type;
-  DotAcc<T> acc;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x) {
     const V2 xv = x ? x[i] : V2{T(0), T(0)};
@@ -979,37 +978,27 @@ __global__ void k_axpby(int64_t n, T ar, T ai, const typename C2<T>::type* __res
       o.y = ar * xv.y + ai * xv.x + br * yv.y + bi * yv.x;
     }
     y[i] = o;
-    if (DOTS & 2) { acc.add_prod(o.x, o.x); acc.add_prod(o.y, o.y); }
-  }
-  if (DOTS) {
-    double vals[3] = {0.0, acc.value(), 0.0};
-    block_reduce_store<2>(vals, partials);
   }
 }
 
 template <typename T, bool REAL>
 static void axpby_t(int64_t n, double ar, double ai, const void* x, double br, double bi, void* y,
-                    double* partials, int dot_mode, cudaStream_t st) {
+                    cudaStream_t st) {
   using V2 = typename C2<T>::type;
-  const int g = blas_grid(n);
-  if (dot_mode)
-    k_axpby<T, 2, REAL><<<g, kBlasThreads, 0, st>>>(n, (T)ar, (T)ai, (const V2*)x, (T)br, (T)bi,
-                                                    (V2*)y, partials);
-  else
-    k_axpby<T, 0, REAL><<<g, kBlasThreads, 0, st>>>(n, (T)ar, (T)ai, (const V2*)x, (T)br, (T)bi,
-                                                    (V2*)y, partials);
+  k_axpby<T, REAL><<<blas_grid(n), kBlasThreads, 0, st>>>(n, (T)ar, (T)ai, (const V2*)x, (T)br,
+                                                          (T)bi, (V2*)y);
   MB_CUDA(cudaGetLastError());
 }
 
 void launch_axpby(int precision, int64_t n, double ar, double ai, const void* x, double br,
-                  double bi, void* y, double* partials, int dot_mode, cudaStream_t st) {
+                  double bi, void* y, cudaStream_t st) {
   const bool real = ai == 0.0 && bi == 0.0;
   if (precision == MB_PREC_F32) {
-    if (real) axpby_t<float, true>(n, ar, ai, x, br, bi, y, partials, dot_mode, st);
-    else axpby_t<float, false>(n, ar, ai, x, br, bi, y, partials, dot_mode, st);
+    if (real) axpby_t<float, true>(n, ar, ai, x, br, bi, y, st);
+    else axpby_t<float, false>(n, ar, ai, x, br, bi, y, st);
   } else {
-    if (real) axpby_t<double, true>(n, ar, ai, x, br, bi, y, partials, dot_mode, st);
-    else axpby_t<double, false>(n, ar, ai, x, br, bi, y, partials, dot_mode, st);
+    if (real) axpby_t<double, true>(n, ar, ai, x, br, bi, y, st);
+    else axpby_t<double, false>(n, ar, ai, x, br, bi, y, st);
   }
 }
 

@@ -1004,7 +1004,7 @@ struct Krylov {
     std::vector<double> host;
     void* prev = nullptr;
     void* cur = plain_vec(0, keep_vectors);
-    launch_axpby(prec, n, 1.0 / b_norm, 0.0, b, 0.0, 0.0, cur, nullptr, 0, st);
+    launch_axpby(prec, n, 1.0 / b_norm, 0.0, b, 0.0, 0.0, cur, st);
     int64_t steps = 0;
     for (int64_t at = 0; at < k;) {
       int64_t to = std::min(k, at + kPlainLook);
@@ -1041,7 +1041,7 @@ struct Krylov {
     void* prev = rot_vec(0);
     void* cur = rot_vec(1);
     void* w = rot_vec(2);
-    launch_axpby(prec, n, 1.0 / b_norm, 0.0, b, 0.0, 0.0, cur, nullptr, 0, st);
+    launch_axpby(prec, n, 1.0 / b_norm, 0.0, b, 0.0, 0.0, cur, st);
     double beta_prev = 0.0;
     int64_t steps = 0;
     for (int64_t it = 0; it < k; ++it) {
@@ -1062,7 +1062,7 @@ struct Krylov {
       // v_prev <- v, v <- w / beta                               (lanczos.h:113-121)
       std::swap(prev, cur);
       std::swap(cur, w);
-      launch_axpby(prec, n, 0.0, 0.0, nullptr, 1.0 / beta, 0.0, cur, nullptr, 0, st);
+      launch_axpby(prec, n, 0.0, 0.0, nullptr, 1.0 / beta, 0.0, cur, st);
       beta_prev = beta;
       if (conv_tol > 0.0 && check_every > 0 && (steps % check_every) == 0 && it + 1 < k &&
           settled(alphas, betas, conv_tol))
@@ -1097,8 +1097,8 @@ struct Krylov {
     s.ticket = nullptr;  // the scalars are given
     void* prev = nullptr;
     void* cur = rot_vec(0);
-    launch_axpby(prec, n, 1.0 / b_norm, 0.0, b, 0.0, 0.0, cur, nullptr, 0, st);
-    launch_axpby(prec, n, y[0].real(), y[0].imag(), cur, 0.0, 0.0, x, nullptr, 0, st);
+    launch_axpby(prec, n, 1.0 / b_norm, 0.0, b, 0.0, 0.0, cur, st);
+    launch_axpby(prec, n, y[0].real(), y[0].imag(), cur, 0.0, 0.0, x, st);
     for (int64_t j = 0; j + 1 < steps; ++j) {
       void* next = rot_vec(j + 1);
       plain_step(s, j, prev, cur, next);
@@ -1107,7 +1107,7 @@ struct Krylov {
       // x += y_(j+1) v_(j+1), v_(j+1) = u_(j+1) / s_(j+1)
       const double sj = betas[(size_t)j];
       launch_axpby(prec, n, y[(size_t)j + 1].real() / sj, y[(size_t)j + 1].imag() / sj, cur, 1.0,
-                   0.0, x, nullptr, 0, st);
+                   0.0, x, st);
     }
   }
 
@@ -1289,7 +1289,7 @@ static void refine_chunk(std::vector<RefineRun>& runs, RefineBufs& bufs, cudaStr
     RefineRun& r = runs[i];
     const double nx = std::sqrt(r.hc[2 * (size_t)r.cap + 1]);
     MB_REQUIRE(nx > 0.0, MB_ERR_ZERO_NORM, "refinement start vector has zero norm");
-    launch_axpby(MB_PREC_F64, r.n, 1.0 / nx, 0.0, r.col(0), 0.0, 0.0, r.col(0), nullptr, 0, ls(i));
+    launch_axpby(MB_PREC_F64, r.n, 1.0 / nx, 0.0, r.col(0), 0.0, 0.0, r.col(0), ls(i));
   }
   // w -= Q Re(Q^H w) against q_0..q_j: the coefficients at dc[0..), the norm of
   // the rest in the second dots.  On pairs of real numbers H is a symmetric
@@ -1349,8 +1349,7 @@ static void refine_chunk(std::vector<RefineRun>& runs, RefineBufs& bufs, cudaStr
         continue;
       }
       r.beta.push_back(b);
-      launch_axpby(MB_PREC_F64, r.n, 1.0 / b, 0.0, r.col(j + 1), 0.0, 0.0, r.col(j + 1), nullptr,
-                   0, ls(i));
+      launch_axpby(MB_PREC_F64, r.n, 1.0 / b, 0.0, r.col(j + 1), 0.0, 0.0, r.col(j + 1), ls(i));
     }
   }
 }
@@ -2472,17 +2471,17 @@ int mb_kpm_projector_apply(mb_op_t op, int64_t expansion_order, double e_min, do
     const size_t vb = elem_bytes(op->precision) * (size_t)op->dim;
     DevBuf tp(vb), tc(vb), res(vb);
     to_tensor(op, v_dev, tp.p, order, st);
-    launch_axpby(op->precision, op->dim, g[0] * mu[0], 0.0, tp.p, 0.0, 0.0, res.p, nullptr, 0, st);
+    launch_axpby(op->precision, op->dim, g[0] * mu[0], 0.0, tp.p, 0.0, 0.0, res.p, st);
     if (M > 0) {
       launch_apply(op->view, op->precision, tp.p, tc.p, 1.0 / a, b, 0.0, nullptr, nullptr, 0, st);
-      launch_axpby(op->precision, op->dim, g[1] * mu[1], 0.0, tc.p, 1.0, 0.0, res.p, nullptr, 0, st);
+      launch_axpby(op->precision, op->dim, g[1] * mu[1], 0.0, tc.p, 1.0, 0.0, res.p, st);
       void* prev = tp.p;
       void* cur = tc.p;
       for (int64_t m = 2; m <= M; ++m) {
         launch_apply(op->view, op->precision, cur, prev, 2.0 / a, b, -1.0, prev, nullptr, 0, st);
         std::swap(prev, cur);
         launch_axpby(op->precision, op->dim, g[(size_t)m] * mu[(size_t)m], 0.0, cur, 1.0, 0.0,
-                     res.p, nullptr, 0, st);
+                     res.p, st);
       }
     }
     from_tensor(op, res.p, out_dev, order, st);
@@ -2506,7 +2505,7 @@ int mb_estimate_bounds(mb_op_t op, int64_t power_iterations, double spectral_pad
       launch_dot(op->precision, op->dim, s0.p, s0.p, red.p(), st);
       double nrm = std::sqrt(red.fetch(gb, 3, st)[2]);
       if (nrm == 0.0) return 0.0;
-      launch_axpby(op->precision, op->dim, 1.0 / nrm, 0.0, s0.p, 0.0, 0.0, v.p, nullptr, 0, st);
+      launch_axpby(op->precision, op->dim, 1.0 / nrm, 0.0, s0.p, 0.0, 0.0, v.p, st);
       double eig = 0.0;
       for (int64_t i = 0; i < power_iterations; ++i) {
         launch_apply(op->view, op->precision, v.p, w.p, scale, shift, 0.0, nullptr, red.p(), 7, st);
@@ -2515,7 +2514,7 @@ int mb_estimate_bounds(mb_op_t op, int64_t power_iterations, double spectral_pad
         if (den == 0.0) return 0.0;
         eig = num / den;
         if (wn == 0.0) return 0.0;
-        launch_axpby(op->precision, op->dim, 1.0 / wn, 0.0, w.p, 0.0, 0.0, v.p, nullptr, 0, st);
+        launch_axpby(op->precision, op->dim, 1.0 / wn, 0.0, w.p, 0.0, 0.0, v.p, st);
       }
       return eig;
     };

@@ -205,7 +205,7 @@ void q_apply_affine(mb_op_s* op, const void* x, void* y, double scale, double sh
   // temporary, then combine with the FP64 vector kernel.
   QBuf tmp(sizeof(double2) * (size_t)op->dim, st);
   q_to_order(op, s.yq, order, ey, tmp.p, st);
-  launch_axpby(MB_PREC_F64, op->dim, beta, 0.0, z, 1.0, 0.0, tmp.p, nullptr, 0, st);
+  launch_axpby(MB_PREC_F64, op->dim, beta, 0.0, z, 1.0, 0.0, tmp.p, st);
   MB_CUDA(cudaMemcpyAsync(y, tmp.p, sizeof(double2) * (size_t)op->dim, cudaMemcpyDeviceToDevice, st));
   MB_CUDA(cudaStreamSynchronize(st));
 }
