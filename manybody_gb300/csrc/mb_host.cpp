@@ -260,6 +260,17 @@ SignedLists signed_lists(const HopTable& t, int64_t D) {
 
 namespace {
 
+// A stable sort of a few elements (std::stable_sort allocates a buffer).
+template <typename Less>
+void insertion_sort(int* v, int n, const Less& less) {
+  for (int i = 1; i < n; ++i) {
+    const int x = v[i];
+    int j = i;
+    for (; j > 0 && less(x, v[j - 1]); --j) v[j] = v[j - 1];
+    v[j] = x;
+  }
+}
+
 // Orders the entries of N lanes (one wavefront of a gather) over k slots: in each
 // slot a maximum matching of lanes to bank groups (target mod N), lanes that must
 // take an entry now (as many left as slots) first, entries of the groups with
@@ -276,7 +287,7 @@ void order_lanes(std::vector<uint32_t>* lst, int k, uint32_t D, uint32_t* out) {
       for (uint32_t w : lst[l]) ++gdeg[(w & kIdx) % N];
     int order[N];
     for (int l = 0; l < N; ++l) order[l] = l;
-    std::stable_sort(order, order + N, [&](int a, int b) {
+    insertion_sort(order, N, [&](int a, int b) {
       const bool fa = (int)lst[a].size() >= left, fb = (int)lst[b].size() >= left;
       if (fa != fb) return fa;
       return lst[a].size() > lst[b].size();
@@ -284,18 +295,18 @@ void order_lanes(std::vector<uint32_t>* lst, int k, uint32_t D, uint32_t* out) {
     int match_g[N], pick[N];
     for (int i = 0; i < N; ++i) match_g[i] = pick[i] = -1;
     // Kuhn's augmenting paths; candidates by descending group degree
-    std::function<bool(int, unsigned&)> augment = [&](int l, unsigned& seen) -> bool {
+    auto augment = [&](auto& self, int l, unsigned& seen) -> bool {
       int cand[64];
       int nc = 0;
       for (int i = 0; i < (int)lst[l].size() && nc < 64; ++i) cand[nc++] = i;
-      std::stable_sort(cand, cand + nc, [&](int a, int b) {
+      insertion_sort(cand, nc, [&](int a, int b) {
         return gdeg[(lst[l][(size_t)a] & kIdx) % N] > gdeg[(lst[l][(size_t)b] & kIdx) % N];
       });
       for (int ci = 0; ci < nc; ++ci) {
         const int g = (int)((lst[l][(size_t)cand[ci]] & kIdx) % N);
         if (seen & (1u << g)) continue;
         seen |= 1u << g;
-        if (match_g[g] < 0 || augment(match_g[g], seen)) {
+        if (match_g[g] < 0 || self(self, match_g[g], seen)) {
           match_g[g] = l;
           pick[l] = cand[ci];
           return true;
@@ -307,7 +318,7 @@ void order_lanes(std::vector<uint32_t>* lst, int k, uint32_t D, uint32_t* out) {
       const int l = order[oi];
       if (lst[l].empty()) continue;
       unsigned seen = 0;
-      augment(l, seen);
+      augment(augment, l, seen);
     }
     unsigned used = 0;
     uint32_t slot[N];

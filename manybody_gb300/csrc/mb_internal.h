@@ -507,7 +507,8 @@ void fill_fused_tables(OpView& v, const HopTable& tu, const HopTable& td, int64_
 
 namespace mb {
 // Workspaces kept between calls (mb_pool.cu).  Device memory by stream order
-// (bytes = 0: nullptr; what is too large to be kept by cudaMalloc), what the device's pool holds idle, and giving that back;
+// (bytes = 0: nullptr; what is too large to be kept by cudaMalloc), what the
+// device's pool holds idle, and giving that back;
 // cudaMalloc that gives it back where it would not fit otherwise; page-locked
 // host memory (given back with the size it was taken with).  Operators and
 // engines hold the pools while they live.
@@ -581,7 +582,7 @@ struct mb_op_s {
   int32_t* perm = nullptr;         // tensor -> reference index (lazy)
   int32_t* iperm = nullptr;        // reference -> tensor index (lazy)
   mb::RowOrder order;              // of a lattice operator (with perm, lazy)
-  const int32_t* low_rows = nullptr;  // its rows by low_first_order
+  const int32_t* low_rows = nullptr;  // its rows by low_first_order (lazy)
   std::mutex mu;
   std::mutex host_mu;  // host-buffer calls: the lane pool and the row groups
   std::mutex host_link_mu;  // host-buffer calls on page-locked vectors take turns
@@ -770,6 +771,7 @@ void upload_binomials(cudaStream_t st);
 int32_t* op_perm(mb_op_s* op);
 // reference -> tensor index table (inverse of op_perm), built on first use
 int32_t* op_iperm(mb_op_s* op);
+const int32_t* op_low_rows(mb_op_s* op);
 // the operator's reference order (built on first use); perm and tiles are
 // nullptr where the operator's own index is the reference order, tiles alone
 // where it is no lattice operator of one sector

@@ -137,7 +137,6 @@ static void build_op(mb_op_s* op, const mb_basis_s* b, const mb_model_s* m) {
   v.L = op->L;
   v.t = m->t;
   v.up_mask = upload(op, b->up.masks);
-  op->low_rows = upload(op, low_first_order(b->up));
   v.up_off = upload(op, tu.off);
   v.up_ent = upload(op, tu.ent.empty() ? std::vector<uint32_t>{0u} : tu.ent);
   if (same) {
@@ -499,6 +498,13 @@ int32_t* op_iperm(mb_op_s* op) {
   return op->iperm;
 }
 
+// the rows by low_first_order, for the launches with kRefOut
+const int32_t* op_low_rows(mb_op_s* op) {
+  std::lock_guard<std::mutex> lk(op->mu);
+  if (!op->low_rows) op->low_rows = upload(op, low_first_order(make_spin_sector(op->L, op->n_up)));
+  return op->low_rows;
+}
+
 // a warp's slots of 8- and 16-byte elements: 12 and 10 KB of shared memory
 constexpr int kTileSlots32 = 1016, kTileSlots64 = 512;
 
@@ -766,7 +772,7 @@ static void apply_affine(mb_op_s* op, const void* x, void* y, double scale, doub
   if (fused) {
     OpView v = op->view;
     v.out_perm = op_perm(op);
-    v.row_sched = op->low_rows;
+    v.row_sched = op_low_rows(op);
     launch_apply(v, op->precision, s.a, y, scale, shift, beta, zt, nullptr, kRefOut, st);
     return;
   }

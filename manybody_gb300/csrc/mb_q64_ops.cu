@@ -188,7 +188,7 @@ void q_apply_affine(mb_op_s* op, const void* x, void* y, double scale, double sh
   if (!z && o.perm && !op->view.csr_row && writes_reference(MB_PREC_Q64, op->dim)) {
     OpView v = op->view;
     v.out_perm = o.perm;
-    v.row_sched = op->low_rows;
+    v.row_sched = op_low_rows(op);
     void* ups = q_ups_for(op, st);
     if (ups) launch_upcol_q(v, s.xq, ups, st);
     launch_apply_q(v, s.xq, y, nullptr, (const QParams*)s.prm, nullptr, nullptr, kRefOut, st, ups);
