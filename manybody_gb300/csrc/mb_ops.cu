@@ -88,19 +88,20 @@ void require_device() {
 
 // Reduction helper: partials -> device result -> host (pinned) values.
 struct Reducer {
-  DevBuf partials, out;
+  DevBuf partials;  // and the sums after them
+  double* out = nullptr;
   double* host = nullptr;
   int cap_blocks, cap_comp;
-  Reducer(int blocks, int comps) : partials(sizeof(double) * (size_t)blocks * comps),
-                                   out(sizeof(double) * (size_t)comps),
+  Reducer(int blocks, int comps) : partials(sizeof(double) * ((size_t)blocks + 1) * comps),
+                                   out((double*)partials.p + (size_t)blocks * comps),
                                    host((double*)pinned_take(sizeof(double) * (size_t)comps)),
                                    cap_blocks(blocks), cap_comp(comps) {}
   ~Reducer() { pinned_give(host, sizeof(double) * (size_t)cap_comp); }
   double* p() { return (double*)partials.p; }
   // Reduce `nblocks` x `ncomp` partials and copy to host; waits on st.
   const double* fetch(int nblocks, int ncomp, cudaStream_t st) {
-    launch_reduce(p(), nblocks, ncomp, (double*)out.p, st);
-    MB_CUDA(cudaMemcpyAsync(host, out.p, sizeof(double) * ncomp, cudaMemcpyDeviceToHost, st));
+    launch_reduce(p(), nblocks, ncomp, out, st);
+    MB_CUDA(cudaMemcpyAsync(host, out, sizeof(double) * ncomp, cudaMemcpyDeviceToHost, st));
     MB_CUDA(cudaStreamSynchronize(st));
     return host;
   }
