@@ -1014,7 +1014,8 @@ struct Krylov {
     launch_axpby(prec, n, 1.0 / b_norm, 0.0, b, 0.0, 0.0, cur, st);
     int64_t steps = 0;
     for (int64_t at = 0; at < k;) {
-      int64_t to = std::min(k, at + kPlainLook);
+      // (first after as many steps as there are states: most runs of a tiny sector end)
+      int64_t to = std::min(k, at ? at + kPlainLook : std::min(kPlainLook, n));
       if (check) to = std::min(to, (at / check_every + 1) * check_every);
       more_scalars(s, at, to);
       for (int64_t j = at; j < to; ++j) {
