@@ -159,6 +159,8 @@ static void build_op(mb_op_s* op, const mb_basis_s* b, const mb_model_s* m) {
     return p;
   });
   v.up_prefetch = apply_prefetches(v, op->precision) ? 1 : 0;
+  // (a small sector's is made when a call needs it: most of its calls are one launch)
+  if (!one_launch(op->precision, op->dim) && writes_reference(op->precision, op->dim)) op_low_rows(op);
   const std::vector<double> uf = u_fold_table(m->u, m->has_u, op->L);
   v.u_fold = upload(op, uf);
   v.u_fold_f = upload(op, std::vector<float>(uf.begin(), uf.end()));
