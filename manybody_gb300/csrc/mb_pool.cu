@@ -11,11 +11,12 @@
 // an allocation does not fit otherwise.  A block is freed in the order of the
 // stream it was used on; CUDA's pools serve any thread and stream.
 //
-// A block that would take the pool past twice what it keeps is cudaMalloc's: it
-// could not be kept, and the pool maps and unmaps memory more slowly than
-// cudaMalloc and cudaFree do.  A complex64 ground state of 1D L=16 8+8 (U = 2, 100
-// steps, 132 GB of kept Lanczos vectors) from the second call on: 0.71 ->
-// 0.54 s (0.545 the first; 0.65 with all of it cudaMalloc's and a slower apply).
+// A block that would take the pool past what it keeps is cudaMalloc's: it could
+// not be kept, and the pool maps and unmaps memory more slowly than cudaMalloc
+// and cudaFree do.  From the second call on: a complex64 ground state of 1D L=16
+// 8+8 (U = 2, 100 steps, 132 GB of kept Lanczos vectors) 0.71 -> 0.54 s, 4x4 6+6, 40
+// steps, 167 -> 143 ms (151 with a line at twice what is kept), Q64, 20 steps, 149
+// -> 106, complex64 4x4 5+5, 40 steps, 39.3 -> 38.1.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -68,12 +69,12 @@ cudaMemPool_t device_pool(uint64_t* keep_out = nullptr) {
 
 constexpr size_t kLargeBlock = size_t(64) << 20;  // smaller ones are the pool's without a look
 
-// Whether a block would take the pool past twice what it keeps.
+// Whether a block would take the pool past what it keeps.
 bool too_large(cudaMemPool_t pool, size_t bytes, uint64_t keep) {
   uint64_t used = 0;
   if (bytes < kLargeBlock) return false;
   MB_CUDA(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used));
-  return used + bytes > 2 * keep;
+  return used + bytes > keep;
 }
 
 }  // namespace
